@@ -41,7 +41,7 @@ __device__ __forceinline__ Sc ld_sc(const Sc* s) { return sc_make(__ldg(&s->re),
 __device__ __forceinline__ Fe ld_fe(const Fe* f) { return fe_make(__ldg(&f->m), __ldg(&f->e)); }
 
 __device__ float smooth_escape(int iteration, const Nrm& norm, double bias) {
-    if (norm.m == 0.0) return static_cast<float>(static_cast<double>(iteration) - bias);
+    if (is_zero(norm.m)) return static_cast<float>(static_cast<double>(iteration) - bias);
     const double log_mag = 0.5 * (log(norm.m) + static_cast<double>(norm.e) * kLogTwo);
     if (!(log_mag > 0.0) || !is_finite(log_mag)) return static_cast<float>(static_cast<double>(iteration) - bias);
     return static_cast<float>((static_cast<double>(iteration) - log(log_mag) / kLogTwo) - bias);
@@ -60,28 +60,29 @@ __device__ Jac jac_holomorphic(const Sc& d) {
     return Jac{re, fe_neg(im), im, re};
 }
 
+__device__ __forceinline__ bool negative(const Fe& a) { return hi_of(a.m) < 0 && !is_zero(a.m); }
+
 __device__ Jac jac_step(int formula, const Sc& total, const Jac& p, bool parameter_plane) {
     const Fe re = fe_from(total.re, total.e);
     const Fe im = fe_from(total.im, total.e);
     Fe m00, m01, m10, m11;
     if (formula == kFormulaTricorn) {
-        m00 = fe_mul(re, 2.0);
-        m01 = fe_mul(im, -2.0);
-        m10 = fe_mul(im, -2.0);
-        m11 = fe_mul(re, -2.0);
+        m00 = fe_twice(re, false);
+        m01 = fe_twice(im, true);
+        m10 = m01;
+        m11 = fe_twice(re, true);
     } else if (formula == kFormulaBurningShip) {
         const Fe ar = fe_abs(re), ai = fe_abs(im);
-        const double rs = re.m < 0.0 ? -1.0 : 1.0;
-        const double is = im.m < 0.0 ? -1.0 : 1.0;
-        m00 = fe_mul(ar, 2.0 * rs);
-        m01 = fe_mul(ai, -2.0 * is);
-        m10 = fe_mul(ai, 2.0 * rs);
-        m11 = fe_mul(ar, 2.0 * is);
+        const bool rneg = negative(re), ineg = negative(im);
+        m00 = fe_twice(ar, rneg);
+        m01 = fe_twice(ai, !ineg);
+        m10 = fe_twice(ai, rneg);
+        m11 = fe_twice(ar, ineg);
     } else {
-        m00 = fe_mul(re, 2.0);
-        m01 = fe_mul(im, -2.0);
-        m10 = fe_mul(im, 2.0);
-        m11 = fe_mul(re, 2.0);
+        m00 = fe_twice(re, false);
+        m01 = fe_twice(im, true);
+        m10 = fe_twice(im, false);
+        m11 = m00;
     }
     const Fe one = parameter_plane ? fe_from(1.0, 0) : fe_zero();
     return Jac{fe_add(fe_add(fe_mul(m00, p.xa), fe_mul(m01, p.ya)), one),
@@ -157,7 +158,7 @@ __device__ Fe alt_margin(const AltParams& p, int i, const Sc& d) {
     const Fe m0 = ld_fe(&r->margin);
     const Fe zr = fe_make(__ldg(&r->parts.re.m), __ldg(&r->parts.re.e));
     const Fe zi = fe_make(__ldg(&r->parts.im.m), __ldg(&r->parts.im.e));
-    const Fe cross = fe_mul(fe_add(fe_mul(zr, fe_from(d.re, d.e)), fe_mul(zi, fe_from(d.im, d.e))), 2.0);
+    const Fe cross = fe_twice(fe_add(fe_mul(zr, fe_from(d.re, d.e)), fe_mul(zi, fe_from(d.im, d.e))), false);
     const Nrm dn = sc_norm2(d);
     return fe_add(fe_add(m0, cross), fe_make(dn.m, dn.e));
 }
@@ -174,23 +175,22 @@ __device__ Sc alt_step(const AltParams& p, int i, const Sc& d, const Sc& pd) {
         const Fe dr = fe_from(d.re, d.e), di = fe_from(d.im, d.e);
         const Fe ar = fe_abs(rr), ai = fe_abs(ri);
         const Fe tr = fe_add(rr, dr), ti = fe_add(ri, di);
-        const bool cross_r = (fe_cmp(rr, fe_zero()) >= 0) != (fe_cmp(tr, fe_zero()) >= 0);
-        const bool cross_i = (fe_cmp(ri, fe_zero()) >= 0) != (fe_cmp(ti, fe_zero()) >= 0);
+        const bool cross_r = fe_at_least_zero(rr) != fe_at_least_zero(tr);
+        const bool cross_i = fe_at_least_zero(ri) != fe_at_least_zero(ti);
         if (cross_r || cross_i) {
             const Fe atr = fe_abs(tr), ati = fe_abs(ti);
             const Sc zn = ld_sc(&p.orbit[i + 1].z);
             const Fe por = fe_sub(fe_from(p.parameter.re, p.parameter.e), fe_from(zn.re, zn.e));
             const Fe poi = fe_sub(fe_from(p.parameter.im, p.parameter.e), fe_from(zn.im, zn.e));
             const Fe nr = fe_add(fe_sub(fe_sqr(atr), fe_sqr(ati)), fe_add(por, fe_from(pd.re, pd.e)));
-            const Fe ni = fe_add(fe_mul(fe_mul(atr, ati), 2.0), fe_add(poi, fe_from(pd.im, pd.e)));
+            const Fe ni = fe_add(fe_twice(fe_mul(atr, ati), false), fe_add(poi, fe_from(pd.im, pd.e)));
             return sc_from_fe(nr, ni);
         }
-        const double rs = rr.m < 0.0 ? -1.0 : 1.0;
-        const double is = ri.m < 0.0 ? -1.0 : 1.0;
-        const Fe lr = fe_sub(fe_mul(fe_mul(ar, dr), 2.0 * rs), fe_mul(fe_mul(ai, di), 2.0 * is));
-        const Fe li = fe_add(fe_mul(fe_mul(ar, di), 2.0 * is), fe_mul(fe_mul(ai, dr), 2.0 * rs));
+        const bool rneg = negative(rr), ineg = negative(ri);
+        const Fe lr = fe_sub(fe_twice(fe_mul(ar, dr), rneg), fe_twice(fe_mul(ai, di), ineg));
+        const Fe li = fe_add(fe_twice(fe_mul(ar, di), ineg), fe_twice(fe_mul(ai, dr), rneg));
         const Fe sr = fe_sub(fe_sqr(dr), fe_sqr(di));
-        const Fe si = fe_mul(fe_mul(dr, di), 2.0 * rs * is);
+        const Fe si = fe_twice(fe_mul(dr, di), rneg != ineg);
         return sc_from_fe(fe_add(fe_add(lr, sr), fe_from(pd.re, pd.e)), fe_add(fe_add(li, si), fe_from(pd.im, pd.e)));
     }
     return sc_add(sc_twice(sc_mul(z, d)), sc_add(sc_mul(d, d), pd));
@@ -372,7 +372,7 @@ __device__ __forceinline__ bool alt_advance(const AltParams& p, AltLane<WithPlan
         const Nrm cnorm = nrm_from_margin(cmargin, p.escape_mode);
         const Sc ctotal = sc_add(ld_sc(&p.orbit[end].z), cand);
         const bool bad = !sc_finite(cand) || !fe_finite(cmargin) || !sc_finite(ctotal)
-            || fe_cmp(cmargin, fe_zero()) > 0 || nrm_cmp(cnorm, nrm_make(0.75, 2)) >= 0;
+            || fe_positive(cmargin) || nrm_cmp(cnorm, nrm_make(0.75, 2)) >= 0;
         if (!bad) {
             s.delta = cand;
             if constexpr (WithPlanes) s.jac = jac_bla(step, s.jac, !julia);
@@ -400,7 +400,7 @@ __device__ __forceinline__ bool alt_advance(const AltParams& p, AltLane<WithPlan
             const Fe margin = alt_margin(p, s.ref, s.delta);
             s.total_norm = nrm_from_margin(margin, p.escape_mode);
             s.total = sc_add(ld_sc(&p.orbit[s.ref].z), s.delta);
-            if (fe_cmp(margin, fe_zero()) > 0 || nrm_outside(s.total_norm, p.escape_mode)) {
+            if (fe_positive(margin) || nrm_outside(s.total_norm, p.escape_mode)) {
                 if constexpr (WithPlanes) {
                     planes.escape(index, raw_iteration(s.it), s.total, prev_palette, s.jac, p.pixel_spacing);
                 }
@@ -428,7 +428,7 @@ __device__ __forceinline__ bool alt_advance(const AltParams& p, AltLane<WithPlan
     const Fe margin = alt_margin(p, s.ref, s.delta);
     s.total_norm = nrm_from_margin(margin, p.escape_mode);
     s.total = sc_add(ld_sc(&p.orbit[s.ref].z), s.delta);
-    if (fe_cmp(margin, fe_zero()) > 0 || nrm_outside(s.total_norm, p.escape_mode)) {
+    if (fe_positive(margin) || nrm_outside(s.total_norm, p.escape_mode)) {
         if constexpr (WithPlanes) planes.escape(index, raw_iteration(s.it), s.total, prev_palette, s.jac, p.pixel_spacing);
         alt_store(p, index, smooth_escape(s.it, s.total_norm, p.output_bias), static_cast<std::uint32_t>(s.it));
         return true;
@@ -445,7 +445,7 @@ __device__ __forceinline__ bool alt_advance(const AltParams& p, AltLane<WithPlan
         } else {
             const Nrm dist = sc_norm2(sc_sub(s.total, s.tortoise));
             const int scale_e = s.total_norm.e > 0 ? s.total_norm.e : 0;
-            if (dist.m == 0.0 || dist.e <= scale_e - 78) {
+            if (is_zero(dist.m) || dist.e <= scale_e - 78) {
                 if (++s.hits >= 3) {
                     if constexpr (WithPlanes) planes.clear(index, p.max_iter);
                     alt_store(p, index, static_cast<float>(static_cast<double>(p.max_iter) - p.output_bias),

@@ -180,7 +180,7 @@ __device__ __forceinline__ int kalles_raw(int iteration) { return iteration - 1 
 
 // smooth_escape_value (renderer.cpp:8170-8181), evaluated in double.
 __device__ float smooth_escape(int iteration, const Nrm& norm, double bias) {
-    if (norm.m == 0.0) return encode(static_cast<double>(iteration), bias);
+    if (is_zero(norm.m)) return encode(static_cast<double>(iteration), bias);
     const double log_mag = 0.5 * (log(norm.m) + static_cast<double>(norm.e) * kLogTwo);
     if (!(log_mag > 0.0) || !is_finite(log_mag)) return encode(static_cast<double>(iteration), bias);
     return encode(static_cast<double>(iteration) - log(log_mag) / kLogTwo, bias);
@@ -296,7 +296,7 @@ struct OrbitView {
         const Fe m0 = fe_make(__ldg(&r[i].margin.m), __ldg(&r[i].margin.e));
         const Fe dr = fe_from(d.re, d.e);
         const Fe di = fe_from(d.im, d.e);
-        const Fe cross = fe_mul(fe_add(fe_mul(pr, dr), fe_mul(pi, di)), 2.0);
+        const Fe cross = fe_twice(fe_add(fe_mul(pr, dr), fe_mul(pi, di)), false);
         return fe_add(fe_add(m0, cross), fe_add(fe_sqr(dr), fe_sqr(di)));
     }
 };
@@ -350,7 +350,7 @@ __device__ __noinline__ void exact_continuation(const PlainParams& p, const Orbi
                 } else {
                     const Nrm dist = sc_norm2(sc_sub(total, tortoise));
                     const int scale_e = total_norm.e > 0 ? total_norm.e : 0;
-                    if (dist.m == 0.0 || dist.e <= scale_e - cycle_margin) {
+                    if (is_zero(dist.m) || dist.e <= scale_e - cycle_margin) {
                         out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
                         out_count = static_cast<std::uint32_t>(p.max_iter);
                         escaped = true;
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
         have_total = false;
         // Glitch sentinel (renderer.cpp:12938-12988).
         const Fe glitch = orbit.glitch(ref);
-        if (glitch.m != 0.0 && fe_cmp(fe_make(total_norm.m, total_norm.e), glitch) < 0) {
+        if (!is_zero(glitch.m) && fe_cmp(fe_make(total_norm.m, total_norm.e), glitch) < 0) {
             st.add(kGlitchCount);
             if (p.exact_flags) {
                 // Strict point renders repair the pixel exactly (MPFR, on
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
             st.add(kUnresolvedPixels);
             break;
         }
-        if (nrm_outside(total_norm, p.escape_mode) || fe_cmp(margin, fe_zero()) > 0) {
+        if (nrm_outside(total_norm, p.escape_mode) || fe_positive(margin)) {
             out_value = smooth_escape(iteration, total_norm, p.output_bias);
             out_count = static_cast<std::uint32_t>(iteration);
             if constexpr (Planes) planes.escape(index, kalles_raw(iteration), total, total_norm, prev_total_norm,
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
                 } else {
                     const Nrm dist = sc_norm2(sc_sub(total, tortoise));
                     const int scale_e = total_norm.e > 0 ? total_norm.e : 0;
-                    if (dist.m == 0.0 || dist.e <= scale_e - cycle_margin) {
+                    if (is_zero(dist.m) || dist.e <= scale_e - cycle_margin) {
                         st.add(kCycleInside);
                         out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
                         out_count = static_cast<std::uint32_t>(p.max_iter);
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
                         retry = true;
                         break;
                     }
-                    if (nrm_outside(replay_norm, p.escape_mode) || fe_cmp(replay_margin, fe_zero()) > 0) {
+                    if (nrm_outside(replay_norm, p.escape_mode) || fe_positive(replay_margin)) {
                         out_value = smooth_escape(iteration, replay_norm, p.output_bias);
                         out_count = static_cast<std::uint32_t>(iteration);
                         if constexpr (Planes) planes.escape(index, kalles_raw(iteration), replay_total, replay_norm,

@@ -12,6 +12,19 @@
 // -ffp-contract=off.  The frexp/ldexp replacements below are exact
 // bit-level operations with one correctly rounded step for subnormal
 // results, i.e. the same values glibc's frexp/scalbn return.
+//
+// What bounds the kernels that use it is the FP64 pipe: one warp instruction
+// takes it 80 cycles of an SM sub-partition on GB300 (measured with
+// dependent-free chains of DADD, DMUL, DFMA and DSETP alike), against 1 to 2
+// for an integer instruction, and both run side by side.  So an FP64
+// instruction is spent only where a sum or product of two full mantissas is
+// rounded.  Zero and range tests, comparisons, sign changes and every
+// multiplication by a power of two work on the bit patterns, and the rare
+// operands those rules do not cover (subnormal, infinite, NaN) go to an
+// out-of-line general path.  A complex product with its normalisation then
+// takes 6 FP64 instructions where the comparisons and halvings made it 18.
+// Measured: a 640x360 plain field at 1e30 in 3.10 ms before and 0.98 ms now,
+// an 853x480 burning-ship field with planes at 1e40 in 106 and 39 ms.
 #pragma once
 
 #include <cstdint>
@@ -20,8 +33,10 @@
 
 #ifdef __CUDACC__
 #define FX_HD __host__ __device__ __forceinline__
+#define FX_HD_SLOW static __host__ __device__ __noinline__
 #else
 #define FX_HD inline
+#define FX_HD_SLOW inline
 #endif
 
 namespace fx {
@@ -46,9 +61,47 @@ FX_HD double from_bits(std::uint64_t b) {
 #endif
 }
 
-FX_HD bool is_finite(double v) { return (bits_of(v) & 0x7ff0000000000000ull) != 0x7ff0000000000000ull; }
-FX_HD bool is_nan(double v) { return v != v; }
-FX_HD double fabs_(double v) { return from_bits(bits_of(v) & 0x7fffffffffffffffull); }
+// The high word (sign, exponent, top of the mantissa) and the low word.
+// Register moves in PTX: the word intrinsics (__double2hiint and the like)
+// lose a product's low word here, as seen with CUDA 13.0 where fe_from takes
+// the product of a logarithm.
+FX_HD int hi_of(double v) {
+#ifdef __CUDA_ARCH__
+    int lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+    (void)lo;
+    return hi;
+#else
+    return static_cast<int>(bits_of(v) >> 32);
+#endif
+}
+
+FX_HD unsigned lo_of(double v) {
+#ifdef __CUDA_ARCH__
+    unsigned lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+    (void)hi;
+    return lo;
+#else
+    return static_cast<unsigned>(bits_of(v));
+#endif
+}
+
+FX_HD double from_hilo(int hi, unsigned lo) {
+#ifdef __CUDA_ARCH__
+    double v;
+    asm("mov.b64 %0, {%1, %2};" : "=d"(v) : "r"(lo), "r"(hi));
+    return v;
+#else
+    return from_bits((static_cast<std::uint64_t>(static_cast<std::uint32_t>(hi)) << 32) | lo);
+#endif
+}
+
+FX_HD bool is_finite(double v) { return (hi_of(v) & 0x7ff00000) != 0x7ff00000; }
+FX_HD bool is_nan(double v) { return (bits_of(v) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull; }
+FX_HD bool is_zero(double v) { return ((hi_of(v) & 0x7fffffff) | lo_of(v)) == 0; }
+FX_HD double fabs_(double v) { return from_hilo(hi_of(v) & 0x7fffffff, lo_of(v)); }
+FX_HD double neg_(double v) { return from_hilo(hi_of(v) ^ static_cast<int>(0x80000000u), lo_of(v)); }
 FX_HD double copysign_(double mag, double sign) {
     return from_bits((bits_of(mag) & 0x7fffffffffffffffull) | (bits_of(sign) & 0x8000000000000000ull));
 }
@@ -56,8 +109,34 @@ FX_HD int imax(int a, int b) { return a > b ? a : b; }
 FX_HD int imin(int a, int b) { return a < b ? a : b; }
 FX_HD double dmax(double a, double b) { return a < b ? b : a; }
 
+// Biased exponent; 0 marks zeros and subnormals, 0x7ff infinities and NaN.
+FX_HD int bexp(double v) { return (hi_of(v) >> 20) & 0x7ff; }
+FX_HD bool is_normal(int be) { return static_cast<unsigned>(be - 1) < 2046u; }
+// v * 2^k for a normal v whose result is normal: exact.
+FX_HD double add_exp(double v, int k) { return from_hilo(hi_of(v) + (k << 20), lo_of(v)); }
+
+// (a > b) - (a < b) for finite a and b that are not both zero: sign and
+// magnitude order of the bit patterns.
+FX_HD int order_of(double a, double b) {
+    const long long x = static_cast<long long>(bits_of(a)), y = static_cast<long long>(bits_of(b));
+    const long long r = (x & y) < 0 ? y - x : (x > y ? 1 : (x < y ? -1 : 0));
+    return r > 0 ? 1 : (r < 0 ? -1 : 0);
+}
+
+// Exponent sum, saturated to the int range.
+FX_HD int sat_add(int a, int b) {
+#ifdef __CUDA_ARCH__
+    int r;
+    asm("add.sat.s32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+#else
+    const long long v = static_cast<long long>(a) + b;
+    return v > INT_MAX ? INT_MAX : (v < INT_MIN ? INT_MIN : static_cast<int>(v));
+#endif
+}
+
 // x * 2^n with a single round-to-nearest-even step (glibc scalbn semantics).
-FX_HD double scale2(double x, int n) {
+FX_HD_SLOW double scale2_general(double x, int n) {
     std::uint64_t b = bits_of(x);
     int be = static_cast<int>((b >> 52) & 0x7ff);
     if (be == 0x7ff || (b << 1) == 0) return x;  // inf, nan, +-0
@@ -82,6 +161,14 @@ FX_HD double scale2(double x, int n) {
     const int r = ne - 1;  // <= -1
     if (r < -54) return copysign_(0.0, x);
     return y * from_bits(static_cast<std::uint64_t>(1023 + r) << 52);
+}
+
+FX_HD double scale2(double x, int n) {
+    n = imin(imax(n, -4096), 4096);
+    const int be = bexp(x);
+    if (is_normal(be) && is_normal(be + n)) return add_exp(x, n);
+    if (is_zero(x)) return x;
+    return scale2_general(x, n);
 }
 
 // frexp: mantissa in [0.5, 1) and exponent; zero/inf/nan returned unchanged
@@ -116,71 +203,86 @@ struct Fe {
 FX_HD Fe fe_make(double m, int e) { Fe r; r.m = m; r.e = e; return r; }
 FX_HD Fe fe_zero() { return fe_make(0.0, 0); }
 FX_HD bool fe_finite(const Fe& a) { return is_finite(a.m); }
-FX_HD bool fe_is_zero(const Fe& a) { return a.m == 0.0; }
+FX_HD bool fe_is_zero(const Fe& a) { return is_zero(a.m); }
 
 // FloatExp::from_parts (renderer.cpp:7551-7561).
-FX_HD Fe fe_from(double value, int exponent) {
-    if (value == 0.0 || is_nan(value)) return fe_make(value, 0);
+FX_HD_SLOW Fe fe_from_general(double value, int exponent) {
+    if (is_zero(value) || is_nan(value)) return fe_make(value, 0);
     int shift = 0;
     const double n = split2(value, &shift);
     return fe_make(n, sat_exp(static_cast<long long>(exponent) + shift));
 }
 
-FX_HD Fe fe_neg(const Fe& a) { return fe_make(-a.m, a.e); }
+FX_HD Fe fe_from(double value, int exponent) {
+    const int be = bexp(value);
+    if (is_normal(be)) return fe_make(add_exp(value, 1022 - be), sat_add(exponent, be - 1022));
+    if (is_zero(value)) return fe_make(value, 0);
+    return fe_from_general(value, exponent);
+}
+
+FX_HD Fe fe_neg(const Fe& a) { return fe_make(neg_(a.m), a.e); }
 FX_HD Fe fe_abs(const Fe& a) { return fe_make(fabs_(a.m), a.e); }
 
-// fe_add (renderer.cpp:8197-8235).
+// fe_add (renderer.cpp:8197-8235): a sum at or above 1 is halved once, one
+// below 0.5 normalised.
 FX_HD Fe fe_add(const Fe& a, const Fe& b) {
-    if (a.m == 0.0) return b;
-    if (b.m == 0.0) return a;
-    const Fe* hi = &a;
-    const Fe* lo = &b;
-    if (b.e > a.e) { hi = &b; lo = &a; }
-    const long long diff = static_cast<long long>(hi->e) - lo->e;
-    if (diff > 60) return *hi;
-    const double m = hi->m + scale2(lo->m, -static_cast<int>(diff));
-    if (m == 0.0 || !is_finite(m)) return fe_from(m, hi->e);
-    const double mag = fabs_(m);
-    if (mag >= 1.0) return fe_make(m * 0.5, sat_exp(static_cast<long long>(hi->e) + 1));
-    if (mag >= 0.5) return fe_make(m, hi->e);
-    int shift = 0;
-    const double n = split2(m, &shift);
-    return fe_make(n, sat_exp(static_cast<long long>(hi->e) + shift));
+    if (is_zero(a.m)) return b;
+    if (is_zero(b.m)) return a;
+    const bool swap = b.e > a.e;
+    const double hm = swap ? b.m : a.m, lm = swap ? a.m : b.m;
+    const int he = swap ? b.e : a.e, le = swap ? a.e : b.e;
+    const unsigned diff = static_cast<unsigned>(he) - static_cast<unsigned>(le);
+    if (diff > 60u) return fe_make(hm, he);
+    const double m = hm + scale2(lm, -static_cast<int>(diff));
+    const int be = bexp(m);
+    if (!is_normal(be)) return fe_from(m, he);
+    const int shift = be >= 1023 ? 1 : be - 1022;
+    return fe_make(add_exp(m, -shift), sat_add(he, shift));
 }
 
 FX_HD Fe fe_sub(const Fe& a, const Fe& b) { return fe_add(a, fe_neg(b)); }
 
-// fe_mul (renderer.cpp:8241-8266).
+// Result of a product or quotient: halved once at or above 1, doubled once
+// below 0.5 (fe_mul / fe_div, renderer.cpp:8241-8291).  `e` is the exponent
+// sum or difference; its saturation matters only for values that no orbit of
+// at most 131,072 bits reaches.
+FX_HD Fe fe_step(double m, int e) {
+    const int be = bexp(m);
+    if (be >= 1023) {
+        if (be == 0x7ff) return fe_from(m, 0);
+        return fe_make(add_exp(m, -1), sat_add(e, 1));
+    }
+    if (be >= 1022) return fe_make(m, e);
+    return fe_make(be > 0 ? add_exp(m, 1) : m * 2.0, sat_add(e, -1));
+}
+
 FX_HD Fe fe_mul(const Fe& a, const Fe& b) {
-    if (a.m == 0.0 || b.m == 0.0) return fe_zero();
-    const double m = a.m * b.m;
-    if (!is_finite(m)) return fe_from(m, 0);
-    const double mag = fabs_(m);
-    const long long es = static_cast<long long>(a.e) + b.e;
-    if (mag >= 1.0) return fe_make(m * 0.5, sat_exp(es + 1));
-    if (mag < 0.5) return fe_make(m * 2.0, sat_exp(es - 1));
-    return fe_make(m, sat_exp(es));
+    if (is_zero(a.m) || is_zero(b.m)) return fe_zero();
+    return fe_step(a.m * b.m, sat_add(a.e, b.e));
+}
+
+// fe_mul(a, fe_from(s, 0)) for s = +2 or -2 (`minus`), without the product.
+FX_HD Fe fe_twice(const Fe& a, bool minus) {
+    if (is_zero(a.m)) return fe_zero();
+    const double m = minus ? neg_(a.m) : a.m;
+    return is_finite(m) ? fe_make(m, sat_add(a.e, 1)) : fe_make(m, 0);
 }
 
 FX_HD Fe fe_mul(const Fe& a, double b) { return fe_mul(a, fe_from(b, 0)); }
 
 // fe_div (renderer.cpp:8272-8291).
 FX_HD Fe fe_div(const Fe& a, const Fe& b) {
-    if (a.m == 0.0) return fe_zero();
+    if (is_zero(a.m)) return fe_zero();
     const double m = a.m / b.m;
-    if (!is_finite(m)) return fe_from(m, 0);
-    const double mag = fabs_(m);
-    const long long ed = static_cast<long long>(a.e) - b.e;
-    if (mag >= 1.0) return fe_make(m * 0.5, sat_exp(ed + 1));
-    if (mag < 0.5) return fe_make(m * 2.0, sat_exp(ed - 1));
-    return fe_make(m, sat_exp(ed));
+    const long long d = static_cast<long long>(a.e) - b.e;
+    return fe_step(m, sat_exp(d));
 }
 
 FX_HD Fe fe_sqr(const Fe& a) { return fe_mul(a, a); }
 
 // fe_sqrt (renderer.cpp:8297-8315).
 FX_HD Fe fe_sqrt(const Fe& a) {
-    if (a.m == 0.0) return a;
+    if (is_zero(a.m)) return a;
     long long e = a.e;
     double m = a.m;
     if (m < 0.0 || !is_finite(m)) return fe_from(sqrt(m), 0);
@@ -196,17 +298,17 @@ FX_HD Fe fe_sqrt(const Fe& a) {
 FX_HD int fe_cmp(const Fe& a, const Fe& b) {
     if (!fe_finite(a)) return fe_finite(b) ? 1 : 0;
     if (!fe_finite(b)) return -1;
-    if (a.m == 0.0) return b.m == 0.0 ? 0 : -1;
-    if (b.m == 0.0) return a.m > 0.0 ? 1 : -1;
-    if (a.m < 0.0 && b.m >= 0.0) return -1;
-    if (a.m >= 0.0 && b.m < 0.0) return 1;
-    const bool negative = a.m < 0.0;
-    if (a.e != b.e) {
-        const int r = a.e < b.e ? -1 : 1;
-        return negative ? -r : r;
-    }
-    return (a.m > b.m) - (a.m < b.m);
+    const bool an = hi_of(a.m) < 0, bn = hi_of(b.m) < 0;
+    if (is_zero(a.m)) return is_zero(b.m) ? 0 : -1;
+    if (is_zero(b.m)) return an ? -1 : 1;
+    if (an != bn) return an ? -1 : 1;
+    if (a.e != b.e) return (a.e < b.e) == an ? 1 : -1;
+    return order_of(a.m, b.m);
 }
+
+// fe_cmp(a, 0) as its callers use it: > 0 and >= 0.
+FX_HD bool fe_positive(const Fe& a) { return !fe_finite(a) || (hi_of(a.m) >= 0 && !is_zero(a.m)); }
+FX_HD bool fe_at_least_zero(const Fe& a) { return !fe_finite(a) || hi_of(a.m) >= 0 || is_zero(a.m); }
 
 FX_HD Fe fe_min(const Fe& a, const Fe& b) { return fe_cmp(a, b) <= 0 ? a : b; }
 
@@ -232,7 +334,7 @@ FX_HD double escape_r2_d(int mode) { return mode == 1 ? 1.0e8 : 4.0; }
 
 // |R + D|^2 - R_escape^2 in FloatExp (renderer.cpp:8374-8390).
 FX_HD Fe fec_escape_margin(const Fec& r, const Fec& d, int mode) {
-    const Fe cross = fe_mul(fe_add(fe_mul(r.re, d.re), fe_mul(r.im, d.im)), 2.0);
+    const Fe cross = fe_twice(fe_add(fe_mul(r.re, d.re), fe_mul(r.im, d.im)), false);
     const Fe ref_margin = fe_sub(fec_norm2(r), escape_r2_fe(mode));
     return fe_add(fe_add(ref_margin, cross), fec_norm2(d));
 }
@@ -252,86 +354,77 @@ struct Nrm {
 FX_HD Sc sc_make(double re, double im, int e) { Sc r; r.re = re; r.im = im; r.e = e; return r; }
 FX_HD Sc sc_zero() { return sc_make(0.0, 0.0, 0); }
 FX_HD Sc sc_one() { return sc_make(1.0, 0.0, 0); }
-FX_HD bool sc_is_zero(const Sc& a) { return a.re == 0.0 && a.im == 0.0; }
+FX_HD bool sc_is_zero(const Sc& a) {
+    return (((hi_of(a.re) | hi_of(a.im)) & 0x7fffffff) | lo_of(a.re) | lo_of(a.im)) == 0;
+}
 FX_HD bool sc_finite(const Sc& a) { return is_finite(a.re) && is_finite(a.im); }
 FX_HD Nrm nrm_make(double m, int e) { Nrm r; r.m = m; r.e = e; return r; }
 
 // ScaledComplex::normalize (renderer.cpp:7611-7656).
-FX_HD void sc_normalize(Sc& v) {
+FX_HD_SLOW void sc_normalize_general(Sc& v) {
     const double mag = dmax(fabs_(v.re), fabs_(v.im));
     if (mag == 0.0) { v.re = 0.0; v.im = 0.0; v.e = 0; return; }
-    if (mag >= 2.0) {
-        int shift = 0;
-        (void)split2(mag, &shift);
-        v.re = scale2(v.re, -shift);
-        v.im = scale2(v.im, -shift);
-        v.e = sat_exp(static_cast<long long>(v.e) + shift);
-        return;
-    }
-    if (mag >= 1.0) {
-        v.re *= 0.5;
-        v.im *= 0.5;
-        v.e = sat_exp(static_cast<long long>(v.e) + 1);
-        return;
-    }
-    if (mag >= 0.5) return;
-    if (mag >= 0.25) {
-        v.re *= 2.0;
-        v.im *= 2.0;
-        v.e = sat_exp(static_cast<long long>(v.e) - 1);
-        return;
-    }
     int shift = 0;
     (void)split2(mag, &shift);
+    if (shift == 0) return;
     v.re = scale2(v.re, -shift);
     v.im = scale2(v.im, -shift);
-    v.e = sat_exp(static_cast<long long>(v.e) + shift);
+    v.e = sat_add(v.e, shift);
+}
+
+FX_HD void sc_normalize(Sc& v) {
+    const int be = imax(bexp(v.re), bexp(v.im));
+    if (!is_normal(be)) { sc_normalize_general(v); return; }
+    const int shift = be - 1022;
+    if (shift == 0) return;
+    v.re = scale2(v.re, -shift);
+    v.im = scale2(v.im, -shift);
+    v.e = sat_add(v.e, shift);
 }
 
 // ScaledComplex::from_float_exp (renderer.cpp:7658-7675).
 FX_HD Sc sc_from_fe(const Fe& re, const Fe& im) {
-    if (re.m == 0.0 && im.m == 0.0) return sc_zero();
+    if (is_zero(re.m) && is_zero(im.m)) return sc_zero();
     const int common = imax(re.e, im.e);
-    const long long rd = static_cast<long long>(re.e) - common;
-    const long long id = static_cast<long long>(im.e) - common;
-    Sc r = sc_make(rd < -1074 ? 0.0 : scale2(re.m, static_cast<int>(rd)),
-                   id < -1074 ? 0.0 : scale2(im.m, static_cast<int>(id)), common);
+    const unsigned rd = static_cast<unsigned>(common) - static_cast<unsigned>(re.e);
+    const unsigned id = static_cast<unsigned>(common) - static_cast<unsigned>(im.e);
+    Sc r = sc_make(rd > 1074u ? 0.0 : scale2(re.m, -static_cast<int>(rd)),
+                   id > 1074u ? 0.0 : scale2(im.m, -static_cast<int>(id)), common);
     sc_normalize(r);
     return r;
 }
 
 // sc_add (renderer.cpp:7678-7698).
 FX_HD Sc sc_add(const Sc& a, const Sc& b) {
-    if (a.re == 0.0 && a.im == 0.0) return b;
-    if (b.re == 0.0 && b.im == 0.0) return a;
-    const Sc* hi = &a;
-    const Sc* lo = &b;
-    if (b.e > a.e) { hi = &b; lo = &a; }
-    const long long diff = static_cast<long long>(hi->e) - lo->e;
-    if (diff > 60) return *hi;
+    if (sc_is_zero(a)) return b;
+    if (sc_is_zero(b)) return a;
+    const bool swap = b.e > a.e;
+    const Sc hi = sc_make(swap ? b.re : a.re, swap ? b.im : a.im, swap ? b.e : a.e);
+    const Sc lo = sc_make(swap ? a.re : b.re, swap ? a.im : b.im, swap ? a.e : b.e);
+    const unsigned diff = static_cast<unsigned>(hi.e) - static_cast<unsigned>(lo.e);
+    if (diff > 60u) return hi;
     const int d = static_cast<int>(diff);
-    Sc r = sc_make(hi->re + scale2(lo->re, -d), hi->im + scale2(lo->im, -d), hi->e);
+    Sc r = sc_make(hi.re + scale2(lo.re, -d), hi.im + scale2(lo.im, -d), hi.e);
     sc_normalize(r);
     return r;
 }
 
-FX_HD Sc sc_neg(const Sc& a) { return sc_make(-a.re, -a.im, a.e); }
-FX_HD Sc sc_conj(const Sc& a) { return sc_make(a.re, -a.im, a.e); }
+FX_HD Sc sc_neg(const Sc& a) { return sc_make(neg_(a.re), neg_(a.im), a.e); }
+FX_HD Sc sc_conj(const Sc& a) { return sc_make(a.re, neg_(a.im), a.e); }
 FX_HD Sc sc_sub(const Sc& a, const Sc& b) { return sc_add(a, sc_neg(b)); }
 
 // sc_mul (renderer.cpp:7712-7722).
 FX_HD Sc sc_mul(const Sc& a, const Sc& b) {
-    if ((a.re == 0.0 && a.im == 0.0) || (b.re == 0.0 && b.im == 0.0)) return sc_zero();
-    Sc r = sc_make(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re,
-                   sat_exp(static_cast<long long>(a.e) + b.e));
+    if (sc_is_zero(a) || sc_is_zero(b)) return sc_zero();
+    Sc r = sc_make(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re, sat_add(a.e, b.e));
     sc_normalize(r);
     return r;
 }
 
 // sc_double (renderer.cpp:7724-7733): exact doubling through the exponent.
 FX_HD Sc sc_twice(const Sc& a) {
-    if (a.re == 0.0 && a.im == 0.0) return sc_zero();
-    return sc_make(a.re, a.im, sat_exp(static_cast<long long>(a.e) + 1));
+    if (sc_is_zero(a)) return sc_zero();
+    return sc_make(a.re, a.im, sat_add(a.e, 1));
 }
 
 // sc_norm_squared (renderer.cpp:7740-7770).
@@ -339,33 +432,25 @@ FX_HD Nrm sc_norm2(const Sc& a) {
     const double inf = from_bits(0x7ff0000000000000ull);
     if (!sc_finite(a)) return nrm_make(inf, INT_MAX);
     const double n = a.re * a.re + a.im * a.im;
-    if (n == 0.0) return nrm_make(0.0, 0);
-    if (!is_finite(n)) return nrm_make(inf, INT_MAX);
-    const long long se = 2LL * a.e;
-    if (n >= 1.0) {
-        const long long e = se + 1;
-        if (e > INT_MAX) return nrm_make(inf, INT_MAX);
-        return nrm_make(n * 0.5, static_cast<int>(e));
-    }
-    if (n < 0.5) {
-        const long long e = se - 1;
-        if (e < INT_MIN) return nrm_make(0.0, 0);
-        return nrm_make(n * 2.0, static_cast<int>(e));
-    }
-    if (se > INT_MAX) return nrm_make(inf, INT_MAX);
-    if (se < INT_MIN) return nrm_make(0.0, 0);
-    return nrm_make(n, static_cast<int>(se));
+    if (is_zero(n)) return nrm_make(0.0, 0);
+    const int be = bexp(n);
+    if (be == 0x7ff) return nrm_make(inf, INT_MAX);
+    // One doubling or halving into [0.5, 1), as the reference.
+    const int shift = be >= 1023 ? 1 : (be < 1022 ? -1 : 0);
+    const long long e = 2LL * a.e + shift;
+    if (e > INT_MAX && shift >= 0) return nrm_make(inf, INT_MAX);
+    if (e < INT_MIN && shift <= 0) return nrm_make(0.0, 0);
+    return nrm_make(be > 0 ? add_exp(n, -shift) : n * 2.0, static_cast<int>(e));
 }
 
 // sc_compare_norm (renderer.cpp:7772-7781).
 FX_HD int nrm_cmp(const Nrm& a, const Nrm& b) {
     if (!is_finite(a.m)) return is_finite(b.m) ? 1 : 0;
     if (!is_finite(b.m)) return -1;
-    if (a.m == 0.0 && b.m == 0.0) return 0;
-    if (a.m == 0.0) return -1;
-    if (b.m == 0.0) return a.m > 0.0 ? 1 : -1;
+    if (is_zero(a.m)) return is_zero(b.m) ? 0 : -1;
+    if (is_zero(b.m)) return hi_of(a.m) >= 0 ? 1 : -1;
     if (a.e != b.e) return a.e < b.e ? -1 : 1;
-    return (a.m > b.m) - (a.m < b.m);
+    return order_of(a.m, b.m);
 }
 
 FX_HD bool nrm_outside(const Nrm& n, int mode) {
@@ -378,7 +463,7 @@ FX_HD double sc_im_d(const Sc& a) { return scale2(a.im, a.e); }
 
 // scaled_norm_to_double / scaled_norm_from_double (renderer.cpp:7801-7823).
 FX_HD double nrm_to_d(const Nrm& n) {
-    if (n.m == 0.0) return 0.0;
+    if (is_zero(n.m)) return 0.0;
     const double dbl_max = 1.7976931348623157e308;
     if (!is_finite(n.m)) return dbl_max;
     const double v = scale2(n.m, n.e);
