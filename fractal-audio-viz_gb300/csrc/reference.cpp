@@ -926,6 +926,10 @@ std::vector<OrbitRec> make_orbit_records(const ReferenceContext& ctx) {
         r.z = orbit.scaled[i];
         r.zd_re = orbit.re_d[i];
         r.zd_im = orbit.im_d[i];
+        r.zf_re = static_cast<float>(fx::sc_re_d(r.z));
+        r.zf_im = static_cast<float>(fx::sc_im_d(r.z));
+        r.raw = fx::raw_value(fx::sc_make(fx::sc_re_d(r.z), fx::sc_im_d(r.z), 0))
+            && r.zd_re == fx::sc_re_d(r.z) && r.zd_im == fx::sc_im_d(r.z);
         r.parts = fx::sc_to_fec(orbit.scaled[i]);
         // Mandelbrot rebuilds the escape margin from the compact orbit
         // (renderer.cpp:8374-8390); the other formulas use the MPFR margin

@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "raw_double.h"
 #include "scaled.h"
 
 namespace fgb {
@@ -56,13 +57,18 @@ struct AltStep {
 // Everything one perturbation step needs about reference index i, packed so
 // a lane touches a single 128-byte record.
 struct alignas(128) OrbitRec {
-    fx::Sc z;          // compact orbit value Z_i
-    double zd_re;      // Z_i as plain double (double-tail path)
+    double zd_re;      // Z_i as plain double
     double zd_im;
+    float zf_re;       // Z_i rounded to float: the estimates that settle a
+    float zf_im;       // test far from its bound without FP64
+    int raw;           // both parts of Z_i in the raw range (raw_double.h)
+    int pad;
+    fx::Sc z;          // compact orbit value Z_i
     fx::Fec parts;     // Z_i components as FloatExp (escape margin input)
     fx::Fe margin;     // |Z_i|^2 - R^2 (escape margin constant term)
     fx::Fe glitch;     // 1e-7 |Z_i|^2, zero when the glitch test is off
 };
+static_assert(sizeof(OrbitRec) == 128, "one record per cache line");
 
 struct OrbitData {
     std::vector<fx::Sc> scaled;

@@ -20,8 +20,8 @@
 // instruction is spent only where a sum or product of two full mantissas is
 // rounded.  Zero and range tests, comparisons, sign changes and every
 // multiplication by a power of two work on the bit patterns, and the rare
-// operands those rules do not cover (subnormal, infinite, NaN) go to an
-// out-of-line general path.  A complex product with its normalisation then
+// operands those rules do not cover (subnormal, infinite, NaN) go to
+// out-of-line general paths.  A complex product with its normalisation then
 // takes 6 FP64 instructions where the comparisons and halvings made it 18.
 // Measured: a 640x360 plain field at 1e30 in 3.10 ms before and 0.98 ms now,
 // an 853x480 burning-ship field with planes at 1e40 in 106 and 39 ms.
@@ -62,9 +62,8 @@ FX_HD double from_bits(std::uint64_t b) {
 }
 
 // The high word (sign, exponent, top of the mantissa) and the low word.
-// Register moves in PTX: the word intrinsics (__double2hiint and the like)
-// lose a product's low word here, as seen with CUDA 13.0 where fe_from takes
-// the product of a logarithm.
+// Register moves in PTX: with the word intrinsics (__double2hiint and the
+// like) CUDA 13.0 lost the low word where fe_from takes a product.
 FX_HD int hi_of(double v) {
 #ifdef __CUDA_ARCH__
     int lo, hi;
@@ -171,6 +170,9 @@ FX_HD double scale2(double x, int n) {
     return scale2_general(x, n);
 }
 
+// A subnormal moved into the normal range: v * 2^54, exact.
+FX_HD_SLOW double lift54(double v) { return v * 18014398509481984.0; }
+
 // frexp: mantissa in [0.5, 1) and exponent; zero/inf/nan returned unchanged
 // with exponent 0.
 FX_HD double split2(double x, int* e) {
@@ -206,18 +208,14 @@ FX_HD bool fe_finite(const Fe& a) { return is_finite(a.m); }
 FX_HD bool fe_is_zero(const Fe& a) { return is_zero(a.m); }
 
 // FloatExp::from_parts (renderer.cpp:7551-7561).
-FX_HD_SLOW Fe fe_from_general(double value, int exponent) {
-    if (is_zero(value) || is_nan(value)) return fe_make(value, 0);
-    int shift = 0;
-    const double n = split2(value, &shift);
-    return fe_make(n, sat_exp(static_cast<long long>(exponent) + shift));
-}
-
 FX_HD Fe fe_from(double value, int exponent) {
     const int be = bexp(value);
     if (is_normal(be)) return fe_make(add_exp(value, 1022 - be), sat_add(exponent, be - 1022));
-    if (is_zero(value)) return fe_make(value, 0);
-    return fe_from_general(value, exponent);
+    if (is_zero(value) || is_nan(value)) return fe_make(value, 0);
+    if (be != 0) return fe_make(value, exponent);  // infinite: frexp's exponent is 0
+    const double lifted = lift54(value);
+    const int shift = bexp(lifted) - 1022;
+    return fe_make(add_exp(lifted, -shift), sat_add(exponent, shift - 54));
 }
 
 FX_HD Fe fe_neg(const Fe& a) { return fe_make(neg_(a.m), a.e); }
@@ -361,21 +359,31 @@ FX_HD bool sc_finite(const Sc& a) { return is_finite(a.re) && is_finite(a.im); }
 FX_HD Nrm nrm_make(double m, int e) { Nrm r; r.m = m; r.e = e; return r; }
 
 // ScaledComplex::normalize (renderer.cpp:7611-7656).
-FX_HD_SLOW void sc_normalize_general(Sc& v) {
-    const double mag = dmax(fabs_(v.re), fabs_(v.im));
-    if (mag == 0.0) { v.re = 0.0; v.im = 0.0; v.e = 0; return; }
+// The exponent of max(|re|, |im|) as frexp gives it, for parts that are both
+// zero or subnormal, or not finite (0: zero, infinite or NaN).  Scalars only
+// in and out: passing the pair through memory, by reference or as a struct,
+// let the compiler (CUDA 13.0, sm_100 and up) mix up two such pairs.
+FX_HD_SLOW int sc_general_shift(double re, double im) {
+    const double mag = dmax(fabs_(re), fabs_(im));
     int shift = 0;
     (void)split2(mag, &shift);
-    if (shift == 0) return;
-    v.re = scale2(v.re, -shift);
-    v.im = scale2(v.im, -shift);
-    v.e = sat_add(v.e, shift);
+    return shift;
 }
 
 FX_HD void sc_normalize(Sc& v) {
     const int be = imax(bexp(v.re), bexp(v.im));
-    if (!is_normal(be)) { sc_normalize_general(v); return; }
-    const int shift = be - 1022;
+    int shift = be - 1022;
+    if (!is_normal(be)) {
+        // A NaN in the imaginary part beside a zero real part clears both, as
+        // the reference's magnitude comparison has it.
+        if (is_zero(v.re) && (is_zero(v.im) || is_nan(v.im))) {
+            v.re = 0.0;
+            v.im = 0.0;
+            v.e = 0;
+            return;
+        }
+        shift = sc_general_shift(v.re, v.im);
+    }
     if (shift == 0) return;
     v.re = scale2(v.re, -shift);
     v.im = scale2(v.im, -shift);
@@ -421,6 +429,16 @@ FX_HD Sc sc_mul(const Sc& a, const Sc& b) {
     return r;
 }
 
+// sc_mul(a, a): the two equal cross products are one product, doubled.
+FX_HD Sc sc_sqr(const Sc& a) {
+    if (sc_is_zero(a)) return sc_zero();
+    const double cross = a.re * a.im;
+    Sc r = sc_make(a.re * a.re - a.im * a.im, is_normal(bexp(cross)) ? add_exp(cross, 1) : cross + cross,
+                   sat_add(a.e, a.e));
+    sc_normalize(r);
+    return r;
+}
+
 // sc_double (renderer.cpp:7724-7733): exact doubling through the exponent.
 FX_HD Sc sc_twice(const Sc& a) {
     if (sc_is_zero(a)) return sc_zero();
@@ -456,6 +474,26 @@ FX_HD int nrm_cmp(const Nrm& a, const Nrm& b) {
 FX_HD bool nrm_outside(const Nrm& n, int mode) {
     const Fe t = escape_r2_fe(mode);
     return nrm_cmp(n, nrm_make(t.m, t.e)) > 0;
+}
+
+// m * 2^e truncated to a float without the FP64 pipe: relative error below
+// 2^-23, 0 below the float range, infinity above it (for |e| < 2^20).
+FX_HD float float_of(double m, int e) {
+    const int h = hi_of(m);
+    const int fe = ((h >> 20) & 0x7ff) - 896 + e;
+    std::uint32_t b = static_cast<std::uint32_t>(h) & 0x80000000u;
+    if (fe >= 255) {
+        b |= 0x7f800000u;
+    } else if (fe > 0) {
+        b |= (static_cast<std::uint32_t>(fe) << 23) | ((static_cast<std::uint32_t>(h) << 3) & 0x7fffffu) | (lo_of(m) >> 29);
+    }
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float v;
+    __builtin_memcpy(&v, &b, sizeof v);
+    return v;
+#endif
 }
 
 FX_HD double sc_re_d(const Sc& a) { return scale2(a.re, a.e); }

@@ -7,7 +7,8 @@ definition written with frexp, ldexp and floating-point comparisons
 (renderer.cpp:7532-7824, 8190-8475), on seeded operands: random, sparse and
 nearly equal mantissas, zeros of both signs, subnormals, infinities and NaN,
 exponents near and far apart.  Host build; the device build runs the same
-code and is compared with the reference's fields by test_gpu_parity.py.
+code and is compared with the reference's fields by test_gpu_parity.py.  The
+raw-double sums of csrc/raw_double.h are compared with the same definitions.
 """
 
 from __future__ import annotations
@@ -18,6 +19,7 @@ import subprocess
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fractal-audio-viz_gb300", "csrc")
 
 DRIVER = r"""
+#include "raw_double.h"
 #include "scaled.h"
 #include <cstdio>
 #include <cstdlib>
@@ -190,6 +192,21 @@ int main(int, char** argv) {
         sc_normalize(u);
         d_normalize(w);
         eq("sc_normalize", u, w);
+        // Raw doubles (raw_double.h): parts in range or zero.
+        const int top = (int)(g() % 380) - 375;
+        auto part = [&](int e) { return g() % 10 ? std::ldexp(mant(), e - (int)(g() % 20)) : 0.0; };
+        Sc x = sc_make(part(top), part(top), 0), y = sc_make(part(top), part(top), 0);
+        if (g() % 2) { const int e = -(int)(g() % 130); y.re = std::ldexp(y.re, e < -370 - top ? 0 : e); y.im = std::ldexp(y.im, e < -370 - top ? 0 : e); }
+        if (g() % 6 == 0) { y.re = -x.re; if (g() % 2) y.im = from_bits(bits_of(x.im) ^ (g() & 1) ^ (1ull << 63)); }
+        Sc xn = x, yn = y, sum = add_cut(x, y);
+        d_normalize(xn);
+        d_normalize(yn);
+        d_normalize(sum);
+        Sc want = d_scadd(xn, yn);
+        check("add_cut", sum.re == want.re && sum.im == want.im && sum.e == want.e);
+        eq("to_raw", normal_form(to_raw(xn)), xn);
+        check("to_raw in range", to_raw(xn).e == 0 || d_zero(xn));
+        if (is_finite(s.re) && is_finite(s.im)) { Sc n = s; d_normalize(n); eq("to_raw any", normal_form(to_raw(n)), n); }
     }
     std::printf("bad %ld\n", bad);
     return bad ? 1 : 0;
