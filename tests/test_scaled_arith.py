@@ -197,7 +197,7 @@ int main(int, char** argv) {
         auto part = [&](int e) { return g() % 10 ? std::ldexp(mant(), e - (int)(g() % 20)) : 0.0; };
         Sc x = sc_make(part(top), part(top), 0), y = sc_make(part(top), part(top), 0);
         if (g() % 2) { const int e = -(int)(g() % 130); y.re = std::ldexp(y.re, e < -370 - top ? 0 : e); y.im = std::ldexp(y.im, e < -370 - top ? 0 : e); }
-        if (g() % 6 == 0) { y.re = -x.re; if (g() % 2) y.im = from_bits(bits_of(x.im) ^ (g() & 1) ^ (1ull << 63)); }
+        if (g() % 6 == 0) { y.re = -x.re; if (g() % 2 && !is_zero(x.im)) y.im = from_bits(bits_of(x.im) ^ (g() & 1) ^ (1ull << 63)); }
         Sc xn = x, yn = y, sum = add_cut(x, y);
         d_normalize(xn);
         d_normalize(yn);
