@@ -333,22 +333,39 @@ void launch_deep_mandelbrot(ReferenceContext& ctx, DeviceTables& dev, const Outp
                "plain Mandelbrot kernel launch");
 }
 
-// Claim counters of the alternate-formula queue: one 256-byte slot per lane
-// stream of a batch, and one (the last) for single renders.
+// Counters and spill lists of the alternate-formula queue: one slot per lane
+// stream of a batch, and one (the last) for single renders.  A list holds up
+// to 65,536 pixels (the ones of a field that outlast a launch's budget;
+// beyond that they run on where they are).
 constexpr int kAltQueueSlots = ThreadRuntime::kPlainLanes + 1;
-constexpr std::size_t kAltQueueStride = 256 / sizeof(unsigned long long);
+constexpr std::size_t kAltQueueStride = 256;
+static_assert(kAltQueueCounters * sizeof(unsigned long long) <= kAltQueueStride, "one slot");
 
-unsigned long long* alt_queue_counters(ThreadRuntime& rt) {
-    return static_cast<unsigned long long*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * 256));
+struct AltQueues {
+    char* counters = nullptr;
+    char* spill = nullptr;
+    long long capacity = 0;
+};
+
+// Sized for fields of up to `pixels` pixels in `slots` slots at once.
+AltQueues alt_queues(ThreadRuntime& rt, long long pixels, int slots) {
+    AltQueues q;
+    q.counters = static_cast<char*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * kAltQueueStride));
+    q.capacity = std::min<long long>(pixels, 65536);
+    q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill,
+                                         static_cast<std::size_t>(slots) * 2 * q.capacity * alt_spill_entry_bytes()));
+    return q;
 }
 
-// `queue_counter`: the claim counter of the lane-refill queue (a batch
-// passes its lane's slot); NULL takes the single-render slot, and point
-// lists always run one thread per point.
+AltQueue alt_queue_slot(const AltQueues& q, int counters, int list) {
+    return AltQueue{reinterpret_cast<unsigned long long*>(q.counters + counters * kAltQueueStride),
+                    q.spill + static_cast<std::size_t>(list) * 2 * q.capacity * alt_spill_entry_bytes(), q.capacity};
+}
+
+// `queue`: the lane's slot of a batch; NULL takes the single-render slot.
 void launch_deep_alternate(ReferenceContext& ctx, DeviceTables& dev, const Outputs& out, int width, int height,
-                           const fx::Fe& zoom, int max_iter, const FractalRenderOptions& o, bool collect_stats,
-                           ThreadRuntime& rt, cudaStream_t stream, const PointInput* points = nullptr,
-                           unsigned long long* queue_counter = nullptr) {
+                           const fx::Fe& zoom, int max_iter, const FractalRenderOptions& o, ThreadRuntime& rt,
+                           cudaStream_t stream, const PointInput* points = nullptr, const AltQueue* queue = nullptr) {
     const DeepGeometry g = deep_geometry(zoom, width, height, o.coordinate_mode);
     AltParams p{};
     p.orbit = dev.orbit;
@@ -400,13 +417,9 @@ void launch_deep_alternate(ReferenceContext& ctx, DeviceTables& dev, const Outpu
         p.deadline_base = rt.stamp;
         p.budget_ns = static_cast<unsigned long long>(o.time_budget_ms) * 1000000ull;
     }
-    p.stats = collect_stats ? rt.stats : nullptr;
-    if (points == nullptr && queue_counter == nullptr) {
-        queue_counter = alt_queue_counters(rt) + (kAltQueueSlots - 1) * kAltQueueStride;
-    }
-    check_cuda(launch_plain_alternate(p, out.p_iter != nullptr, collect_stats, points ? nullptr : queue_counter,
-                                      stream),
-               "plain alternate-formula kernel launch");
+    const AltQueue slot = queue ? *queue
+        : alt_queue_slot(alt_queues(rt, static_cast<long long>(width) * height, 1), kAltQueueSlots - 1, 0);
+    check_cuda(launch_plain_alternate(p, out.p_iter != nullptr, slot, stream), "plain alternate-formula kernel launch");
 }
 
 // Spill-list entries for a direct batch of `pixels` pixels: enough for the
@@ -480,7 +493,7 @@ void render_from_reference(ReferenceContext& ctx, const Outputs& out, int width,
     if (zoom_log10 >= 6.0L) {
         std::shared_ptr<DeviceTables> dev = device_tables(ctx);
         if (ctx.formula != kFormulaMandelbrot) {
-            launch_deep_alternate(ctx, *dev, out, width, height, zoom, max_iter, o, collect_stats, rt, stream);
+            launch_deep_alternate(ctx, *dev, out, width, height, zoom, max_iter, o, rt, stream);
         } else {
             launch_deep_mandelbrot(ctx, *dev, out, width, height, zoom, max_iter, series_order, series_block, o,
                                    collect_stats, rt, stream);
@@ -1552,7 +1565,8 @@ struct BatchPlan {
     int feature_rows = 0;
     // Plain-form launches: (stream, the alternate queue's claim counter for
     // that stream).
-    std::vector<std::function<void(cudaStream_t, unsigned long long*)>> plain;
+    std::vector<std::function<void(cudaStream_t, const AltQueue&)>> plain;
+    long long alternate_pixels = 0;  // of the largest alternate-formula field among them
     // A time budget stamps its origin per launch in one per-thread word, so
     // budgeted plain launches stay one after another on one stream.
     bool serial_plain = false;
@@ -1598,8 +1612,15 @@ TileBuffers tile_buffers(char* base, int tiles, int rows) {
     return t;
 }
 
+// Lane streams a batch's plain-form launches are dealt over (0: one after
+// another on one stream).
+int plain_lanes(const BatchPlan& plan) {
+    return plan.plain.size() > 1 && !plan.serial_plain
+        ? static_cast<int>(std::min<std::size_t>(ThreadRuntime::kPlainLanes, plan.plain.size())) : 0;
+}
+
 void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRuntime& rt, cudaStream_t main,
-                   void* direct_scratch, unsigned long long* counter, unsigned long long* alt_counters) {
+                   void* direct_scratch, unsigned long long* counter, const AltQueues& alternates) {
     // The direct queue runs on the second stream beside the other launches;
     // with an FP32 queue in the batch a single plain-form (FP64) launch joins
     // it there, so the FP64 and FP32 pipes work at once.  Two or more
@@ -1607,8 +1628,7 @@ void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRunti
     // from and joined back to the caller's stream), so their tails overlap.
     // Fields that asked for derivative planes only share one discard region
     // for the planes nobody reads; concurrent lanes may write it in any order.
-    const int lanes = plan.plain.size() > 1 && !plan.serial_plain
-        ? static_cast<int>(std::min<std::size_t>(ThreadRuntime::kPlainLanes, plan.plain.size())) : 0;
+    const int lanes = plain_lanes(plan);
     const bool fork = (!plan.direct.empty() && (!plan.floatexp.empty() || !plan.plain.empty()))
         || (!plan.plain.empty() && !plan.floatexp.empty());
     cudaStream_t plain_stream = fork && !plan.floatexp.empty() ? rt.side : main;
@@ -1669,14 +1689,15 @@ void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRunti
     }
     if (lanes > 0) {
         for (std::size_t i = 0; i < plan.plain.size(); ++i) {
-            plan.plain[i](rt.lanes[i % lanes], alt_counters + (i % lanes) * kAltQueueStride);
+            const int lane = static_cast<int>(i % lanes);
+            plan.plain[i](rt.lanes[lane], alt_queue_slot(alternates, lane, lane));
         }
         for (int l = 0; l < lanes; ++l) {
             check_cuda(cudaEventRecord(rt.lane_join[l], rt.lanes[l]), "cudaEventRecord (lane join)");
             check_cuda(cudaStreamWaitEvent(main, rt.lane_join[l], 0), "cudaStreamWaitEvent (lane join)");
         }
     } else {
-        for (const auto& launch : plan.plain) launch(plain_stream, alt_counters);
+        for (const auto& launch : plan.plain) launch(plain_stream, alt_queue_slot(alternates, 0, 0));
     }
     if (fork) {
         check_cuda(cudaEventRecord(rt.join, rt.side), "cudaEventRecord (join)");
@@ -1688,16 +1709,19 @@ void launch_plan(const BatchPlan& plan, const BatchShapes& shapes, ThreadRuntime
                  bool graph) {
     void* direct_scratch = plan.direct.empty() ? nullptr : scratch(rt, kScratchDirect, plan.direct_bytes);
     auto* counter = static_cast<unsigned long long*>(scratch(rt, kScratchQueue, 256));
-    unsigned long long* alt_counters = plan.plain.empty() ? nullptr : alt_queue_counters(rt);
+    AltQueues alternates;
+    if (plan.alternate_pixels > 0) alternates = alt_queues(rt, plan.alternate_pixels, std::max(1, plain_lanes(plan)));
     if (!graph) {
-        enqueue_batch(plan, shapes, rt, stream, direct_scratch, counter, alt_counters);
+        enqueue_batch(plan, shapes, rt, stream, direct_scratch, counter, alternates);
         return;
     }
     std::string key = plan.key;
     append_bytes(key, shapes);
     append_bytes(key, direct_scratch);
     append_bytes(key, counter);
-    append_bytes(key, alt_counters);
+    append_bytes(key, alternates.counters);
+    append_bytes(key, alternates.spill);
+    append_bytes(key, alternates.capacity);
     auto found = rt.graphs.find(key);
     if (found == rt.graphs.end()) {
         if (rt.graphs.size() >= 16) {
@@ -1707,7 +1731,7 @@ void launch_plan(const BatchPlan& plan, const BatchShapes& shapes, ThreadRuntime
         }
         check_cuda(cudaStreamBeginCapture(rt.capture, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
         try {
-            enqueue_batch(plan, shapes, rt, rt.capture, direct_scratch, counter, alt_counters);
+            enqueue_batch(plan, shapes, rt, rt.capture, direct_scratch, counter, alternates);
         } catch (...) {
             cudaGraph_t broken = nullptr;
             cudaStreamEndCapture(rt.capture, &broken);
@@ -2017,15 +2041,17 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
         ReferenceContext* raw = ctx.get();
         const int max_iter = frame.max_iter;
         plan.plain.push_back([raw, dev, out, width, height, zoom, max_iter, series_order, series_block, o,
-                              &rt](cudaStream_t s, unsigned long long* queue_counter) {
+                              &rt](cudaStream_t s, const AltQueue& queue) {
             if (raw->formula != kFormulaMandelbrot) {
-                launch_deep_alternate(*raw, *dev, out, width, height, zoom, max_iter, o, false, rt, s, nullptr,
-                                      queue_counter);
+                launch_deep_alternate(*raw, *dev, out, width, height, zoom, max_iter, o, rt, s, nullptr, &queue);
             } else {
                 launch_deep_mandelbrot(*raw, *dev, out, width, height, zoom, max_iter, series_order,
                                        series_block, o, false, rt, s);
             }
         });
+        if (raw->formula != kFormulaMandelbrot) {
+            plan.alternate_pixels = std::max(plan.alternate_pixels, static_cast<long long>(width) * height);
+        }
         append_bytes(plan.key, raw);
         append_bytes(plan.key, raw->generation);
         append_bytes(plan.key, out);
@@ -2346,7 +2372,7 @@ int render_points(float* output, int count, const char* zoom_text, const double*
                 std::shared_ptr<DeviceTables> dev = device_tables(*ctx);
                 check_cuda(cudaEventRecord(rt.start, stream), "cudaEventRecord");
                 if (ctx->formula != kFormulaMandelbrot) {
-                    launch_deep_alternate(*ctx, *dev, out, n, 1, zoom, max_iter, o, collect, rt, stream, &input);
+                    launch_deep_alternate(*ctx, *dev, out, n, 1, zoom, max_iter, o, rt, stream, &input);
                 } else {
                     launch_deep_mandelbrot(*ctx, *dev, out, n, 1, zoom, max_iter, series_order, series_block, o,
                                            collect, rt, stream, &input);

@@ -451,12 +451,17 @@ void render_floatexp_from_reference(ReferenceContext& ctx, const Outputs& out, i
                                     cudaStream_t stream);
 
 cudaError_t launch_plain_mandelbrot(const PlainParams& params, bool planes, bool stats, cudaStream_t stream);
-// With `queue_counter` (8 bytes of device memory no other launch uses at
-// the same time) a Julia field renders through the persistent lane-refill
-// queue; other formulas, point lists and calls without a counter run one
-// thread per pixel.
-cudaError_t launch_plain_alternate(const AltParams& params, bool planes, bool stats,
-                                   unsigned long long* queue_counter, cudaStream_t stream);
+// Device memory of one alternate-formula render, which no other launch uses
+// at the same time: kAltQueueCounters words and two spill lists of `capacity`
+// entries each (alt_spill_entry_bytes; may be absent).
+constexpr int kAltQueueCounters = 16;
+struct AltQueue {
+    unsigned long long* counters;
+    void* spill;
+    long long capacity;
+};
+std::size_t alt_spill_entry_bytes();
+cudaError_t launch_plain_alternate(const AltParams& params, bool planes, const AltQueue& queue, cudaStream_t stream);
 // A batch of direct fields (one kernel over all of them); the batch struct
 // travels as a __grid_constant__ kernel parameter.
 constexpr int kMaxDirectFields = 64;

@@ -928,8 +928,9 @@ std::vector<OrbitRec> make_orbit_records(const ReferenceContext& ctx) {
         r.zd_im = orbit.im_d[i];
         r.zf_re = static_cast<float>(fx::sc_re_d(r.z));
         r.zf_im = static_cast<float>(fx::sc_im_d(r.z));
-        r.raw = fx::raw_value(fx::sc_make(fx::sc_re_d(r.z), fx::sc_im_d(r.z), 0))
+        const bool raw = fx::raw_value(fx::sc_make(fx::sc_re_d(r.z), fx::sc_im_d(r.z), 0))
             && r.zd_re == fx::sc_re_d(r.z) && r.zd_im == fx::sc_im_d(r.z);
+        r.raw = raw ? kRawOrbit : 0;
         r.parts = fx::sc_to_fec(orbit.scaled[i]);
         // Mandelbrot rebuilds the escape margin from the compact orbit
         // (renderer.cpp:8374-8390); the other formulas use the MPFR margin
@@ -937,6 +938,21 @@ std::vector<OrbitRec> make_orbit_records(const ReferenceContext& ctx) {
         r.margin = ctx.formula == kFormulaMandelbrot || i >= orbit.escape_margin.size()
             ? fx::fe_sub(fx::fec_norm2(r.parts), escape_r2)
             : orbit.escape_margin[i];
+        if (ctx.formula == kFormulaBurningShip) {
+            if (i + 1 < orbit.scaled.size()) {
+                const fx::Sc& c = ctx.parameter;
+                const fx::Sc& next = orbit.scaled[i + 1];
+                const fx::Fe part[2] = {fx::fe_sub(fx::fe_from(c.re, c.e), fx::fe_from(next.re, next.e)),
+                                        fx::fe_sub(fx::fe_from(c.im, c.e), fx::fe_from(next.im, next.e))};
+                bool fits = raw;
+                for (int k = 0; k < 2; ++k) {
+                    r.fold[k] = fx::scale2(part[k].m, part[k].e);
+                    fits = fits && (fx::fe_is_zero(part[k]) || fx::raw_part(r.fold[k]));
+                }
+                if (fits) r.raw |= kRawFold;
+            }
+            continue;
+        }
         const fx::Nrm n = fx::sc_norm2(orbit.scaled[i]);
         const fx::Fe norm = fx::fe_make(n.m, n.e);
         r.glitch = (norm.m != 0.0 && fx::fe_finite(norm)) ? fx::fe_mul(norm, 1.0e-7) : fx::fe_zero();

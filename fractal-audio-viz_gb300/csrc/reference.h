@@ -61,13 +61,18 @@ struct alignas(128) OrbitRec {
     double zd_im;
     float zf_re;       // Z_i rounded to float: the estimates that settle a
     float zf_im;       // test far from its bound without FP64
-    int raw;           // both parts of Z_i in the raw range (raw_double.h)
+    int raw;           // kRawOrbit, kRawFold (raw_double.h)
     int pad;
     fx::Sc z;          // compact orbit value Z_i
     fx::Fec parts;     // Z_i components as FloatExp (escape margin input)
     fx::Fe margin;     // |Z_i|^2 - R^2 (escape margin constant term)
-    fx::Fe glitch;     // 1e-7 |Z_i|^2, zero when the glitch test is off
+    union {
+        fx::Fe glitch;   // Mandelbrot: 1e-7 |Z_i|^2, zero when the glitch test is off
+        double fold[2];  // burning ship: parameter - Z_(i+1), the constant of a folded step
+    };
 };
+constexpr int kRawOrbit = 1;  // both parts of Z_i in the raw range
+constexpr int kRawFold = 2;   // and of the fold constant, or zero
 static_assert(sizeof(OrbitRec) == 128, "one record per cache line");
 
 struct OrbitData {

@@ -1,5 +1,6 @@
 // Plain form for julia / burning-ship / tricorn: FP64-mantissa perturbation
-// with the formula-aware real 2x2 linear BLA, one thread per pixel.
+// with the formula-aware real 2x2 linear BLA, in a persistent lane-refill
+// queue.
 //
 // Restates render_alternate_reference_impl and alternate_delta_step
 // (renderer.cpp:11933-12448): the image series for Julia, the signed escape
@@ -22,7 +23,7 @@ namespace {
 
 using namespace fx;
 
-constexpr int kAltPastTurns = 16;  // formula steps per turn past the orbit's end
+constexpr int kAltRound = 16;  // raw steps per round
 constexpr double kTwoPi = 6.283185307179586476925286766559005768;
 constexpr double kLogTwo = 0.693147180559945309417232121458176568;
 
@@ -268,83 +269,88 @@ __device__ __noinline__ Jac jac_step_general(int formula, Sc total, const Jac j,
     return jac_pack(jac_step(formula, total, jac_normal(j), parameter_plane));
 }
 
+// The Jacobian as a raw value: four doubles times 2^k.
+struct RawJac {
+    double xa, xb, ya, yb;
+    int k;
+};
+
 __device__ __forceinline__ bool jac_part(double v) {
     return static_cast<unsigned>(bexp(v) - kRawLow) <= kJacSpan || is_zero(v);
 }
+
+__device__ __forceinline__ double twice_raw(double v) { return is_zero(v) ? v : add_exp(v, 1); }
 
 // jac_step on the values themselves: total raw (a part may have cancelled to
 // zero), entries on one exponent k.  The parameter plane's +1 is 2^-k in the
 // entries' unit; below 2^-600 of it, it cannot move a sum that is above
 // 2^-463.  Returns false, with nothing changed, where the ranges do not fit.
 template <int Formula>
-__device__ __forceinline__ bool jac_step_raw(const Sc& total, Jac& j) {
+__device__ __forceinline__ bool jac_step_raw(const Sc& total, RawJac& j) {
     constexpr bool parameter_plane = Formula != kFormulaJulia;
-    const int k = j.xa.e;
-    const bool fits = k == j.xb.e && k == j.ya.e && k == j.yb.e && k >= -400 && jac_part(j.xa.m) && jac_part(j.xb.m)
-        && jac_part(j.ya.m) && jac_part(j.yb.m);
-    if (!fits) return false;
-    const double tr = is_zero(total.re) ? total.re : add_exp(total.re, 1);
-    const double ti = is_zero(total.im) ? total.im : add_exp(total.im, 1);
-    // Rows of M (jac_step): real part 2 (tr, -ti); imaginary part 2 (ti, tr)
-    // with each formula's signs.
-    bool s0 = false, s1 = false;  // signs of (ti, tr) in the second row
-    if constexpr (Formula == kFormulaTricorn) {
-        s0 = s1 = true;
-    } else if constexpr (Formula == kFormulaBurningShip) {
-        const bool rn = hi_of(tr) < 0 && !is_zero(tr), in = hi_of(ti) < 0 && !is_zero(ti);
-        s0 = s1 = rn != in;
+    if (!(j.k >= -400 && jac_part(j.xa) && jac_part(j.xb) && jac_part(j.ya) && jac_part(j.yb))) return false;
+    const double tr = twice_raw(total.re), ti = twice_raw(total.im);
+    // Rows of M (jac_step): real part 2 (tr, -ti); imaginary part 2 (ti, tr),
+    // negated for the tricorn and where the burning ship's signs differ.
+    bool negate = Formula == kFormulaTricorn;
+    if constexpr (Formula == kFormulaBurningShip) {
+        negate = (hi_of(tr) < 0 && !is_zero(tr)) != (hi_of(ti) < 0 && !is_zero(ti));
     }
-    const double m00 = tr, m01 = neg_(ti), m10 = flip(ti, s0), m11 = flip(tr, s1);
-    double xa = m00 * j.xa.m + m01 * j.ya.m, xb = m00 * j.xb.m + m01 * j.yb.m;
-    double ya = m10 * j.xa.m + m11 * j.ya.m, yb = m10 * j.xb.m + m11 * j.yb.m;
+    const double m01 = neg_(ti), m10 = flip(ti, negate), m11 = flip(tr, negate);
+    double xa = tr * j.xa + m01 * j.ya, yb = m10 * j.xb + m11 * j.yb;
+    const double xb = tr * j.xb + m01 * j.yb, ya = m10 * j.xa + m11 * j.ya;
     if constexpr (parameter_plane) {
-        if (k <= 600) {
-            const double one = from_hilo((1023 - k) << 20, 0);
+        if (j.k <= 600) {
+            const double one = from_hilo((1023 - j.k) << 20, 0);
             xa = xa + one;
             yb = yb + one;
         } else if (bexp(xa) < 560 || bexp(yb) < 560) {
             return false;
         }
     }
-    const int top = imax(imax(bexp(xa), bexp(xb)), imax(bexp(ya), bexp(yb)));
-    int shift = 0;
-    if (top > 1023 + 300) {
+    j.xa = xa;
+    j.xb = xb;
+    j.ya = ya;
+    j.yb = yb;
+    if (imax(imax(bexp(xa), bexp(xb)), imax(bexp(ya), bexp(yb))) > 1023 + 300) {
         const auto low = [](double v) { return is_zero(v) ? 2046 : bexp(v); };
-        const int least = imin(imin(low(xa), low(xb)), imin(low(ya), low(yb)));
-        if (least - 300 >= kRawLow) shift = 300;
+        if (imin(imin(low(xa), low(xb)), imin(low(ya), low(yb))) - 300 >= kRawLow) {
+            const auto down = [](double v) { return is_zero(v) ? v : add_exp(v, -300); };
+            j = RawJac{down(xa), down(xb), down(ya), down(yb), j.k + 300};
+        }
     }
-    const auto entry = [&](double v) { return fe_make(is_zero(v) ? v : add_exp(v, -shift), k + shift); };
-    j = Jac{entry(xa), entry(xb), entry(ya), entry(yb)};
     return true;
 }
 
+// alt_step on raw values: 7 products and 5 to 7 sums.  For the burning ship
+// the signs of |Z| cancel to one sign on the imaginary part, and a step
+// where a part of Z + d crosses zero (`fold`: 18 % of a 1e40 view's steps)
+// runs the same products and sums on Z + d and the record's constant, so
+// folding lanes do not leave the others.
 template <int Formula>
-__device__ __forceinline__ void jac_advance(const Sc& total, bool raw, Jac& j) {
-    if (raw && jac_step_raw<Formula>(total, j)) return;
-    j = jac_step_general(Formula, total, j, Formula != kFormulaJulia);
-}
-
-// alt_step on raw values.  For the burning ship, away from a fold (no part of
-// Z + d on the other side of zero from Z's) the signs of |Z| cancel to one
-// sign on the imaginary part: 7 products and 7 sums, as for the others.
-template <int Formula>
-__device__ __forceinline__ Sc alt_step_raw(double zr, double zi, const Sc& d, const Sc& pd) {
-    const double z2r = add_exp(zr, 1), z2i = add_exp(zi, 1);
-    const double lr = z2r * d.re - z2i * d.im;
-    const double li = z2r * d.im + z2i * d.re;
+__device__ __forceinline__ Sc alt_step_raw(const double2& z, const Sc& d, const Sc& pd, bool fold, const Sc& total,
+                                           const double2& constant) {
+    const double z2r = add_exp(z.x, 1), z2i = add_exp(z.y, 1);
+    double lr = z2r * d.re - z2i * d.im;
+    double li = z2r * d.im + z2i * d.re;
+    if constexpr (Formula == kFormulaBurningShip) {
+        const double u = choose(fold, total.re, d.re), v = choose(fold, total.im, d.im);
+        const double sr = u * u - v * v;
+        const double si = twice_raw(u * v);
+        const bool s = !fold && (hi_of(z.x) ^ hi_of(z.y)) < 0;
+        const double tr = choose(fold, constant.x, lr) + choose(fold, pd.re, sr);
+        const double ti = choose(fold, constant.y, li) + choose(fold, pd.im, si);
+        return sc_make(tr + choose(fold, sr, pd.re), flip(ti, s) + choose(fold, fabs_(si), pd.im), 0);
+    }
     const double sr = d.re * d.re - d.im * d.im;
     const double si = add_exp(d.re * d.im, 1);
-    if constexpr (Formula == kFormulaBurningShip) {
-        const bool s = (hi_of(zr) ^ hi_of(zi)) < 0;
-        return sc_make((lr + sr) + pd.re, flip(li + si, s) + pd.im, 0);
-    } else if constexpr (Formula == kFormulaTricorn) {
+    if constexpr (Formula == kFormulaTricorn) {
         return add_cut(sc_make(lr, neg_(li), 0), add_cut(sc_make(sr, neg_(si), 0), pd));
-    } else {
-        return add_cut(sc_make(lr, li, 0), sc_make(sr, si, 0));
     }
+    return add_cut(sc_make(lr, li, 0), sc_make(sr, si, 0));
 }
 
-// A fold of the burning ship: a part of Z + d has crossed zero.
+// A part of Z + d has crossed zero, or reached it.
 __device__ __forceinline__ bool folds(double z, double d) {
     return (hi_of(z) ^ hi_of(d)) < 0 && (bits_of(d) & 0x7fffffffffffffffull) >= (bits_of(z) & 0x7fffffffffffffffull);
 }
@@ -372,33 +378,27 @@ __device__ __noinline__ const AltStep* alt_search(const AltParams& p, int offset
     return nullptr;
 }
 
-__device__ __forceinline__ const AltStep* alt_lookup(const AltParams& p, int start, const Sc& d, const Fe& pn,
-                                                     int max_length) {
-    if (p.alt_index.levels == 0 || start < p.alt_start || max_length <= 0 || !sc_finite(d) || !fe_finite(pn)) {
-        return nullptr;
-    }
-    const int offset = start - p.alt_start;
-    if (offset < 0 || offset >= p.alt_index.count[0]) return nullptr;
+// Whether alt_search certainly finds no block for delta d at `offset`: no
+// block of two steps starts at an odd offset, and with E the exponent of d's
+// larger part (which is at least 2^(E - 1)) |d|^2 >= 2^(2E - 2), while
+// r2 < 2^r2.e.
+__device__ __forceinline__ bool no_block(const AltParams& p, int offset, const Sc& d) {
+    if (offset < 0 || offset >= p.alt_index.count[0] || (offset & 1) != 0) return true;
+    if ((offset >> 1) >= p.alt_index.count[1]) return false;
+    const AltStep* s = p.alt + p.alt_index.offset[1] + (offset >> 1);
+    const int high = __ldg(reinterpret_cast<const int*>(&s->r2.m) + 1);
+    const int e = __ldg(&s->r2.e);
+    const int top = imax(bexp(d.re), bexp(d.im));
+    return (high & 0x7ff00000) != 0x7ff00000 && is_normal(top)
+        && 2LL * (static_cast<long long>(d.e) + top - 1022) - 2 >= e;
+}
+
+__device__ const AltStep* alt_lookup(const AltParams& p, int start, const Sc& d, const Fe& pn, int max_length) {
+    if (p.alt_index.levels == 0 || max_length <= 0 || !sc_finite(d) || !fe_finite(pn)) return nullptr;
     int top = 31 - __clz(max_length);
     top = top < p.alt_index.levels - 1 ? top : p.alt_index.levels - 1;
-    // Only blocks of two or more steps are taken, and they start at even
-    // offsets.  At one start the radii never grow with the level (a merge
-    // keeps at most its first half's radius, times 1 - 2^-40; an unpaired
-    // entry is copied), so a delta outside the two-step block's finite
-    // radius is outside every longer block's too: one load settles the
-    // common case of a delta too large for any block, with the same result
-    // as the full top-down search.
-    if (top < 1 || (offset & 1) != 0) return nullptr;
-    if ((offset >> 1) < p.alt_index.count[1]) {
-        const Fe r2 = ld_fe(&p.alt[p.alt_index.offset[1] + (offset >> 1)].r2);
-        // With E the exponent of d's larger part (which is at least 2^(E - 1)),
-        // |d|^2 >= 2^(2E - 2), and r2 < 2^r2.e.
-        const int top_exponent = imax(bexp(d.re), bexp(d.im));
-        if (fe_finite(r2) && is_normal(top_exponent) && 2LL * (static_cast<long long>(d.e) + top_exponent - 1022) - 2 >= r2.e) {
-            return nullptr;
-        }
-    }
-    return alt_search(p, offset, d, pn, top);
+    if (top < 1 || no_block(p, start - p.alt_start, d)) return nullptr;
+    return alt_search(p, start - p.alt_start, d, pn, top);
 }
 
 __device__ __noinline__ Sc apply_alt(const AltStep* s, const Sc d, const Sc c) {
@@ -411,25 +411,37 @@ __device__ __noinline__ Sc apply_alt(const AltStep* s, const Sc d, const Sc c) {
     return sc_from_fe(rr, ri);
 }
 
-// One pixel's state between steps, so a lane can park it and carry on
-// later (the lane-refill queue below) or run it to the end at once.  delta,
-// total and pd are raw values where their range allows (raw_double.h).  The
-// total Z + delta is kept only once the orbit has ended (`past`): before
-// that it is formed where something reads it.
+// One pixel's state.  It lives in local memory: the raw loop below keeps
+// the few values it needs in registers, everything else is touched only on
+// the rare general turns.  delta and pd are raw values where their range
+// allows (raw_double.h); total is kept once the orbit has ended (`past`).
 template <bool WithPlanes>
 struct AltLane {
     long long index;
     Sc dc, pd, delta, total, tortoise;
+    Sc prior;   // total before the step whose escape test is pending, or of the escape
     Fe pn;
+    Nrm norm;   // escape norm of a pixel that has escaped
     Jac jac;
     int ref, it, power, length, hits;
+    int rounds; // rounds run in this launch
     unsigned ticks;
-    bool ready, past;
+    bool ready, past, pending;
 };
+
+enum AltOutcome { kAltContinue = 0, kAltDone, kAltEscaped };
 
 __device__ __forceinline__ void alt_store(const AltParams& p, long long index, float out, std::uint32_t count) {
     p.out[index] = out;
     if (p.counts) p.counts[index] = count;
+}
+
+template <bool WithPlanes>
+__device__ __forceinline__ AltOutcome alt_interior(const AltParams& p, long long index) {
+    if constexpr (WithPlanes) Planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2}.clear(index, p.max_iter);
+    alt_store(p, index, static_cast<float>(static_cast<double>(p.max_iter) - p.output_bias),
+              static_cast<std::uint32_t>(p.max_iter));
+    return kAltDone;
 }
 
 __device__ __noinline__ Sc alt_total(const AltParams& p, int ref, Sc delta) {
@@ -437,239 +449,322 @@ __device__ __noinline__ Sc alt_total(const AltParams& p, int ref, Sc delta) {
     return sc_add(ld_sc(&p.orbit[ref].z), delta);
 }
 
-__device__ __forceinline__ int raw_iteration(int formula, int n) {
-    return formula == kFormulaJulia ? n : (n - 1 > 0 ? n - 1 : 0);
-}
+// What an escaped pixel leaves for its outputs, parked in shared memory until
+// a warp has 32: the logarithms, hypot, atan2 and divisions are several
+// hundred FP64 instructions, which cost the same for one lane as for all.
+template <bool WithPlanes>
+struct AltEnd {
+    long long index;
+    Nrm norm;
+    int it;
+};
+template <>
+struct AltEnd<true> {
+    long long index;
+    Nrm norm;
+    Sc total;
+    Nrm prior;
+    Jac jac;
+    int it;
+};
+constexpr int kAltPark = 64;  // fewer than 32 waiting, and up to 32 more
 
-// Outputs of a pixel that escaped with `norm` at `total`; `prior` is the
-// total one step earlier (planes only).
 template <bool WithPlanes, int Formula>
-__device__ __noinline__ void alt_finish(const AltParams& p, long long index, int it, const Nrm norm, Sc total, Sc prior,
-                                        const Jac jac) {
+__device__ __noinline__ void alt_finish(const AltParams& p, const AltEnd<WithPlanes>& e) {
     if constexpr (WithPlanes) {
         const Planes planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2};
-        planes.escape(index, raw_iteration(Formula, it), normal_form(total), sc_norm2(normal_form(prior)),
-                      jac_normal(jac), p.pixel_spacing);
+        const int raw = Formula == kFormulaJulia ? e.it : (e.it - 1 > 0 ? e.it - 1 : 0);
+        planes.escape(e.index, raw, normal_form(e.total), e.prior, jac_normal(e.jac), p.pixel_spacing);
     }
-    alt_store(p, index, smooth_escape(it, norm, p.output_bias), static_cast<std::uint32_t>(it));
+    alt_store(p, e.index, smooth_escape(e.it, e.norm, p.output_bias), static_cast<std::uint32_t>(e.it));
 }
 
-// The escape test after a perturbation step to s.ref.  Returns true when the
-// pixel escaped.
-template <bool WithPlanes, int Formula>
-__device__ __forceinline__ bool alt_escaped(const AltParams& p, const AltLane<WithPlanes>& s, const Sc& prior) {
+// The escape test after a perturbation step to s.ref, s.prior being the
+// total before it.
+template <bool WithPlanes>
+__device__ __noinline__ bool alt_escaped(const AltParams& p, AltLane<WithPlanes>& s) {
     if (alt_inside(p, s.ref, s.delta)) return false;
     const Fe margin = alt_margin(p, s.ref, s.delta);
-    const Nrm norm = nrm_from_margin(margin, p.escape_mode);
-    if (!fe_positive(margin) && !nrm_outside(norm, p.escape_mode)) return false;
-    alt_finish<WithPlanes, Formula>(p, s.index, s.it, norm, WithPlanes ? alt_total(p, s.ref, s.delta) : sc_zero(), prior,
-                                    s.jac);
+    s.norm = nrm_from_margin(margin, p.escape_mode);
+    if (!fe_positive(margin) && !nrm_outside(s.norm, p.escape_mode)) return false;
+    if constexpr (WithPlanes) s.total = alt_total(p, s.ref, s.delta);
     return true;
 }
 
 // Start pixel `index`: coordinates, Julia series jump, first escape test.
-// Returns true when the pixel is finished (its outputs written).
 template <bool WithPlanes, int Formula>
-__device__ __noinline__ bool alt_begin(const AltParams& p, long long index, AltLane<WithPlanes>& s) {
+__device__ __noinline__ AltOutcome alt_begin(const AltParams& p, long long index, AltLane<WithPlanes>& s) {
     constexpr bool julia = Formula == kFormulaJulia;
     const int py = static_cast<int>(index / p.width);
     const int px = static_cast<int>(index - static_cast<long long>(py) * p.width);
-    const Planes planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2};
-    if constexpr (WithPlanes) planes.clear(index, p.max_iter);
+    if constexpr (WithPlanes) Planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2}.clear(index, p.max_iter);
     const double xf = pixel_offset(px, p.width, p.coordinate_mode) / static_cast<double>(p.width);
     const double yf = -pixel_offset(py, p.height, p.coordinate_mode) / static_cast<double>(p.height);
-    s.index = index;
-    s.dc = p.points ? sc_make(p.points[index].re, p.points[index].im, p.points[index].e)
-                    : sc_from_fe(fe_mul(p.view_width, xf), fe_mul(p.view_height, yf));
-    s.pd = julia ? sc_zero() : s.dc;
-    const Nrm pnorm = sc_norm2(s.pd);
-    s.pn = fe_make(pnorm.m, pnorm.e);
-    s.delta = s.dc;
-    s.jac = jac_identity();
-    s.ref = julia ? 0 : 1;
-    s.it = julia ? 0 : 1;
-    if (p.series_on && nrm_cmp(sc_norm2(s.dc), p.series_r2) <= 0) {
+    const Sc dc = p.points ? sc_make(p.points[index].re, p.points[index].im, p.points[index].e)
+                           : sc_from_fe(fe_mul(p.view_width, xf), fe_mul(p.view_height, yf));
+    const Nrm pnorm = julia ? nrm_make(0.0, 0) : sc_norm2(dc);
+    Sc delta = dc;
+    Jac jac = jac_identity();
+    int at = julia ? 0 : 1;
+    if (p.series_on && nrm_cmp(sc_norm2(dc), p.series_r2) <= 0) {
         Sc value = ld_sc(&p.series[p.series_terms - 1]);
         Sc poly = sc_zero();
         for (int k = p.series_terms - 1; k > 1; --k) {
-            if constexpr (WithPlanes) poly = sc_add(sc_mul(poly, s.dc), value);
-            value = sc_add(sc_mul(value, s.dc), ld_sc(&p.series[k - 1]));
+            if constexpr (WithPlanes) poly = sc_add(sc_mul(poly, dc), value);
+            value = sc_add(sc_mul(value, dc), ld_sc(&p.series[k - 1]));
         }
-        s.delta = sc_mul(value, s.dc);
-        if constexpr (WithPlanes) s.jac = jac_holomorphic(sc_add(sc_mul(poly, s.dc), value));
-        s.ref = p.series_iteration;
-        s.it = p.series_iteration;
+        delta = sc_mul(value, dc);
+        if constexpr (WithPlanes) jac = jac_holomorphic(sc_add(sc_mul(poly, dc), value));
+        at = p.series_iteration;
     }
+    s.index = index;
+    s.dc = dc;
+    s.pd = julia ? sc_zero() : to_raw(dc);
+    s.pn = fe_make(pnorm.m, pnorm.e);
+    s.delta = to_raw(delta);
+    s.jac = jac_pack(jac);
+    s.ref = at;
+    s.it = at;
     s.ticks = 0;
-    if (!alt_inside(p, s.ref, s.delta)) {
-        const Nrm norm = nrm_from_margin(alt_margin(p, s.ref, s.delta), p.escape_mode);
-        if (nrm_outside(norm, p.escape_mode)) {
-            alt_finish<WithPlanes, Formula>(p, index, s.it, norm, WithPlanes ? alt_total(p, s.ref, s.delta) : sc_zero(),
-                                            sc_zero(), s.jac);
-            return true;
-        }
-    }
-    s.pd = to_raw(s.pd);
-    s.delta = to_raw(s.delta);
-    s.jac = jac_pack(s.jac);
-    s.past = false;
-    s.total = sc_zero();
-    s.tortoise = sc_zero();
+    s.past = s.pending = s.ready = false;
+    s.total = s.tortoise = s.prior = sc_zero();
     s.power = 1;
     s.length = 0;
     s.hits = 0;
-    s.ready = false;
+    s.rounds = 0;
+    if (!alt_inside(p, at, s.delta)) {
+        s.norm = nrm_from_margin(alt_margin(p, at, s.delta), p.escape_mode);
+        if (nrm_outside(s.norm, p.escape_mode)) {
+            if constexpr (WithPlanes) s.total = alt_total(p, at, s.delta);
+            return kAltEscaped;
+        }
+    }
+    return kAltContinue;
+}
+
+// Up to `limit` exact steps on raw values, the hot loop: it stops before a
+// step that needs the general turn (a block may apply, a value out of range,
+// the orbit's end, the cap) and after one whose escape or cycle test the
+// general turn must settle (`pending`).  Returns the steps taken.
+//
+// FP64 instructions per step: 14 (12 for Julia), with planes 16 more (the
+// total and the Jacobian).
+template <bool WithPlanes, int Formula>
+__device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlanes>& s, int limit) {
+    constexpr bool julia = Formula == kFormulaJulia;
+    const Sc pd = s.pd;
+    Sc d = s.delta;
+    RawJac j{};
+    bool fits = !s.past && !s.pending && d.e == 0 && (julia || raw_value(pd));
+    if constexpr (WithPlanes) {
+        j = RawJac{s.jac.xa.m, s.jac.xb.m, s.jac.ya.m, s.jac.yb.m, s.jac.xa.e};
+        fits = fits && j.k == s.jac.xb.e && j.k == s.jac.ya.e && j.k == s.jac.yb.e;
+    }
+    if (!fits) return 0;
+    const int first = s.ref;
+    const int room = imin(imin(limit, p.max_iter - s.it), p.orbit_size - 1 - first);
+    const bool blocks = !p.disable_bla && p.alt_index.levels > 1;
+    const int cycle_from = p.cycle ? 2048 : INT_MAX;
+    const OrbitRec* r = p.orbit + first;
+    double2 z = __ldg(reinterpret_cast<const double2*>(r));
+    int flags = __ldg(&r->raw);
+    const float r2 = p.escape_mode == 1 ? 1.0e8f : 4.0f;
+    Sc prior = sc_zero();
+    int k = 0;
+    bool pending = false;
+#pragma unroll 1
+    while (k < room) {
+        if (!(flags & kRawOrbit) || !raw_part(d.re) || !raw_part(d.im)) break;
+        if (blocks && !no_block(p, first + k - p.alt_start, d)) break;
+        const double2 zn = __ldg(reinterpret_cast<const double2*>(r + 1));
+        const float4 head = __ldg(reinterpret_cast<const float4*>(&r[1].zf_re));
+        bool fold = false;
+        double2 constant{0.0, 0.0};
+        Sc total = sc_zero();
+        if constexpr (Formula == kFormulaBurningShip) {
+            fold = folds(z.x, d.re) || folds(z.y, d.im);
+            if (fold) {
+                if (!(flags & kRawFold)) break;
+                constant = make_double2(__ldg(&r->fold[0]), __ldg(&r->fold[1]));
+            }
+            total = sc_make(z.x + d.re, z.y + d.im, 0);
+        }
+        if constexpr (WithPlanes) {
+            if constexpr (Formula == kFormulaBurningShip) {
+                // add_cut with its sums at hand
+                const int diff = imax(bexp(z.x), bexp(z.y)) - imax(bexp(d.re), bexp(d.im));
+                prior = diff > 60 ? sc_make(z.x, z.y, 0) : (diff < -60 ? d : total);
+            } else {
+                prior = add_cut(sc_make(z.x, z.y, 0), d);
+            }
+            if (!jac_step_raw<Formula>(prior, j)) break;
+        }
+        d = alt_step_raw<Formula>(z, d, pd, fold, total, constant);
+        ++k;
+        ++r;
+        z = zn;
+        flags = __float_as_int(head.z);
+        // alt_inside at the new index.
+        const float dx = float_of(d.re, 0), dy = float_of(d.im, 0);
+        const float tx = head.x + dx, ty = head.y + dy;
+        const int it = s.it + k;
+        if (!(tx * tx + ty * ty < r2 * (1.0f - 0x1p-14f) && dx * dx + dy * dy < r2 * 16.0f)
+            || (it >= cycle_from && (it & 31) == 0)) {
+            pending = true;
+            break;
+        }
+    }
+    s.delta = d;
+    s.ref = first + k;
+    s.it += k;
+    s.pending = pending;
+    if constexpr (WithPlanes) {
+        s.prior = prior;
+        s.jac = Jac{fe_make(j.xa, j.k), fe_make(j.xb, j.k), fe_make(j.ya, j.k), fe_make(j.yb, j.k)};
+    }
+    return k;
+}
+
+// The bounded cycle, confirmed three times (non-strict renders only).
+template <bool WithPlanes>
+__device__ __noinline__ bool alt_cycle(const AltParams& p, AltLane<WithPlanes>& s) {
+    const Nrm total_norm = nrm_from_margin(alt_margin(p, s.ref, s.delta), p.escape_mode);
+    if (nrm_cmp(total_norm, nrm_make(0.75, 2)) >= 0) return false;
+    const Sc total = alt_total(p, s.ref, s.delta);
+    if (!s.ready) {
+        s.tortoise = total;
+        s.power = 1;
+        s.length = 0;
+        s.hits = 0;
+        s.ready = true;
+        return false;
+    }
+    const Nrm dist = sc_norm2(sc_sub(total, s.tortoise));
+    const int scale_e = total_norm.e > 0 ? total_norm.e : 0;
+    if (is_zero(dist.m) || dist.e <= scale_e - 78) {
+        if (++s.hits >= 3) return true;
+    } else {
+        s.hits = 0;
+    }
+    if (++s.length >= s.power) {
+        s.tortoise = total;
+        s.power = s.power * 2 < (1 << 20) ? s.power * 2 : (1 << 20);
+        s.length = 0;
+    }
     return false;
 }
 
-// Formula steps past the orbit's end (up to `turns`).  Returns true when the
-// pixel is finished.
+// Formula steps past the orbit's end, up to kAltRound.
 template <bool WithPlanes, int Formula>
-__device__ __forceinline__ bool alt_past(const AltParams& p, AltLane<WithPlanes>& s, unsigned long long deadline,
-                                         int turns) {
+__device__ __noinline__ AltOutcome alt_past(const AltParams& p, AltLane<WithPlanes>& s) {
     constexpr bool julia = Formula == kFormulaJulia;
-    if (!s.past) {
-        s.total = to_raw(alt_total(p, s.ref, s.delta));
-        s.past = true;
-    }
+    Sc total = s.past ? s.total : to_raw(alt_total(p, s.ref, s.delta));
+    s.past = true;
     const Sc parameter = to_raw(julia ? p.parameter : sc_add(p.parameter, s.dc));
-    const float estimate_bound = static_cast<float>(p.escape_mode == 1 ? 1.0e8 : 4.0) * (1.0f - 0x1p-14f);
-    for (int k = 0; k < turns && s.it < p.max_iter; ++k) {
-        if (k > 0 && deadline && ((s.ticks++ & 255U) == 0U) && global_ns() >= deadline) {
-            alt_store(p, s.index, nan_f(), 0u);
-            return true;
-        }
-        const Sc prior = s.total;
-        // Raw step: 3 products and 3 sums.  Squares of parts in range are
-        // normal; a sum that cancels is exact.
+    const float bound = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * (1.0f - 0x1p-14f);
+    int it = s.it;
+    AltOutcome outcome = kAltContinue;
+#pragma unroll 1
+    for (int k = 0; k < kAltRound && it < p.max_iter; ++k) {
+        const Sc prior = total;
+        // Raw step: 3 products and 3 sums.
         const bool raw = raw_value(prior) && parameter.e == 0;
-        if constexpr (WithPlanes) jac_advance<Formula>(prior, raw, s.jac);
-        ++s.it;
+        if constexpr (WithPlanes) {
+            bool stepped = false;
+            const Jac g = s.jac;
+            if (raw && g.xa.e == g.xb.e && g.xa.e == g.ya.e && g.xa.e == g.yb.e) {
+                RawJac j{g.xa.m, g.xb.m, g.ya.m, g.yb.m, g.xa.e};
+                stepped = jac_step_raw<Formula>(prior, j);
+                if (stepped) s.jac = Jac{fe_make(j.xa, j.k), fe_make(j.xb, j.k), fe_make(j.ya, j.k), fe_make(j.yb, j.k)};
+            }
+            if (!stepped) s.jac = jac_step_general(Formula, prior, g, !julia);
+        }
+        ++it;
         bool maybe_out = true;
         if (raw) {
-            const double cross = add_exp(prior.re * prior.im, 1);
             const bool negate = Formula == kFormulaTricorn
                 || (Formula == kFormulaBurningShip && (hi_of(prior.re) ^ hi_of(prior.im)) < 0);
-            const Sc square = sc_make(prior.re * prior.re - prior.im * prior.im, flip(cross, negate), 0);
-            s.total = add_cut(square, parameter);
-            const float tx = float_of(s.total.re, 0), ty = float_of(s.total.im, 0);
-            maybe_out = !(tx * tx + ty * ty < estimate_bound);
+            total = add_cut(sc_make(prior.re * prior.re - prior.im * prior.im,
+                                    flip(add_exp(prior.re * prior.im, 1), negate), 0), parameter);
+            const float tx = float_of(total.re, 0), ty = float_of(total.im, 0);
+            maybe_out = !(tx * tx + ty * ty < bound);
         } else {
-            s.total = to_raw(formula_step<Formula>(prior, parameter));
+            total = to_raw(formula_step<Formula>(prior, parameter));
         }
         if (maybe_out) {
-            const Nrm norm = sc_norm2(normal_form(s.total));
+            const Nrm norm = sc_norm2(normal_form(total));
             if (nrm_outside(norm, p.escape_mode)) {
-                alt_finish<WithPlanes, Formula>(p, s.index, s.it, norm, s.total, prior, s.jac);
-                return true;
+                s.norm = norm;
+                s.prior = prior;
+                outcome = kAltEscaped;
+                break;
             }
         }
     }
-    return false;
+    s.total = total;
+    s.it = it;
+    return outcome;
 }
 
-// One turn of the per-pixel loop: formula steps past the orbit's end, a BLA
-// block (or its exact replay), or one exact perturbation step with the
-// escape and cycle tests.  Returns true when the pixel is finished.
+// One general turn: a pending escape or cycle test, formula steps past the
+// orbit's end, a BLA block (or its exact replay), or one exact step.
 template <bool WithPlanes, int Formula>
-__device__ __forceinline__ bool alt_advance(const AltParams& p, AltLane<WithPlanes>& s, unsigned long long deadline,
-                                            int max_block) {
+__device__ __noinline__ AltOutcome alt_general(const AltParams& p, AltLane<WithPlanes>& s, int max_block) {
     constexpr bool julia = Formula == kFormulaJulia;
-    const long long index = s.index;
-    if (s.it >= p.max_iter) {
-        const Planes planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2};
-        if constexpr (WithPlanes) planes.clear(index, p.max_iter);
-        alt_store(p, index, static_cast<float>(static_cast<double>(p.max_iter) - p.output_bias),
-                  static_cast<std::uint32_t>(p.max_iter));
-        return true;
-    }
-    if (deadline && ((s.ticks++ & 255U) == 0U) && global_ns() >= deadline) {
-        alt_store(p, index, nan_f(), 0u);
-        return true;
-    }
-    if (s.ref + 1 >= p.orbit_size) return alt_past<WithPlanes, Formula>(p, s, deadline, kAltPastTurns);
-    const int remaining = p.max_iter - s.it;
-    const AltStep* step = !p.disable_bla
-        ? alt_lookup(p, s.ref, s.delta, s.pn, max_block < remaining ? max_block : remaining)
-        : nullptr;
-    int len = step != nullptr ? __ldg(&step->len) : 1;
-    if (step != nullptr && s.ref + len < p.orbit_size) {
-        const int end = s.ref + len;
-        const Sc cand = apply_alt(step, s.delta, s.pd);
-        const Fe cmargin = alt_margin(p, end, cand);
-        const Nrm cnorm = nrm_from_margin(cmargin, p.escape_mode);
-        const bool bad = !sc_finite(cand) || !fe_finite(cmargin) || !sc_finite(alt_total(p, end, cand))
-            || fe_positive(cmargin) || nrm_cmp(cnorm, nrm_make(0.75, 2)) >= 0;
-        if (!bad) {
-            s.delta = to_raw(cand);
-            if constexpr (WithPlanes) s.jac = jac_pack(jac_bla(step, s.jac, !julia));
-            s.ref = end;
-            s.it += len;
-            return false;
+    const AltStep* step = nullptr;
+    if (!s.pending) {
+        if (s.it >= p.max_iter) return alt_interior<WithPlanes>(p, s.index);
+        if (s.ref + 1 >= p.orbit_size) return alt_past<WithPlanes, Formula>(p, s);
+        const int remaining = p.max_iter - s.it;
+        if (!p.disable_bla) {
+            step = alt_lookup(p, s.ref, s.delta, s.pn, max_block < remaining ? max_block : remaining);
         }
-    } else {
-        step = nullptr;
-        len = 1;
-    }
-    // Exact steps: one, or the refused block's replay (whose steps have no
-    // cycle test of their own).
-    for (int k = 0; k < len && s.it < p.max_iter; ++k) {
-        const OrbitRec* r = p.orbit + s.ref;
-        const double2 z = __ldg(reinterpret_cast<const double2*>(&r->zd_re));
-        const bool raw = __ldg(&r->raw) != 0 && raw_value(s.delta) && (julia || raw_value(s.pd));
-        Sc prior = sc_zero();
-        if constexpr (WithPlanes) {
-            prior = raw ? add_cut(sc_make(z.x, z.y, 0), s.delta) : alt_total(p, s.ref, s.delta);
-            jac_advance<Formula>(prior, raw, s.jac);
-        }
-        if (raw && !(Formula == kFormulaBurningShip && (folds(z.x, s.delta.re) || folds(z.y, s.delta.im)))) {
-            s.delta = alt_step_raw<Formula>(z.x, z.y, s.delta, s.pd);
+        int len = step != nullptr ? __ldg(&step->len) : 1;
+        if (step != nullptr && s.ref + len < p.orbit_size) {
+            const int end = s.ref + len;
+            const Sc cand = apply_alt(step, s.delta, s.pd);
+            const Fe cmargin = alt_margin(p, end, cand);
+            const Nrm cnorm = nrm_from_margin(cmargin, p.escape_mode);
+            const bool bad = !sc_finite(cand) || !fe_finite(cmargin) || !sc_finite(alt_total(p, end, cand))
+                || fe_positive(cmargin) || nrm_cmp(cnorm, nrm_make(0.75, 2)) >= 0;
+            if (!bad) {
+                s.delta = to_raw(cand);
+                if constexpr (WithPlanes) s.jac = jac_pack(jac_bla(step, s.jac, !julia));
+                s.ref = end;
+                s.it += len;
+                return kAltContinue;
+            }
         } else {
+            step = nullptr;
+            len = 1;
+        }
+        // Exact steps: one, or the refused block's replay (whose steps have
+        // no cycle test of their own).
+        for (int k = 0; k < len && s.it < p.max_iter; ++k) {
+            if constexpr (WithPlanes) {
+                s.prior = alt_total(p, s.ref, s.delta);
+                s.jac = jac_step_general(Formula, s.prior, s.jac, !julia);
+            }
             s.delta = to_raw(alt_step<Formula>(p, s.ref, s.delta, s.pd));
-        }
-        ++s.ref;
-        ++s.it;
-        if (!sc_finite(s.delta)) {
-            alt_store(p, index, p.strict ? nan_f() : static_cast<float>(static_cast<double>(s.it) - p.output_bias),
-                      p.strict ? 0u : static_cast<std::uint32_t>(s.it));
-            return true;
-        }
-        if (alt_escaped<WithPlanes, Formula>(p, s, prior)) return true;
-    }
-    if (step != nullptr) return false;
-    // Bounded cycle confirmed three times (non-strict renders only).
-    if (!p.cycle || s.it < 2048 || (s.it & 31) != 0) return false;
-    const Nrm total_norm = nrm_from_margin(alt_margin(p, s.ref, s.delta), p.escape_mode);
-    if (nrm_cmp(total_norm, nrm_make(0.75, 2)) < 0) {
-        const Sc total = alt_total(p, s.ref, s.delta);
-        if (!s.ready) {
-            s.tortoise = total;
-            s.power = 1;
-            s.length = 0;
-            s.hits = 0;
-            s.ready = true;
-        } else {
-            const Nrm dist = sc_norm2(sc_sub(total, s.tortoise));
-            const int scale_e = total_norm.e > 0 ? total_norm.e : 0;
-            if (is_zero(dist.m) || dist.e <= scale_e - 78) {
-                if (++s.hits >= 3) {
-                    const Planes planes{p.p_iter, p.p_phase, p.p_dex, p.p_dey, p.p_t1, p.p_t2};
-                    if constexpr (WithPlanes) planes.clear(index, p.max_iter);
-                    alt_store(p, index, static_cast<float>(static_cast<double>(p.max_iter) - p.output_bias),
-                              static_cast<std::uint32_t>(p.max_iter));
-                    return true;
-                }
-            } else {
-                s.hits = 0;
+            ++s.ref;
+            ++s.it;
+            if (!sc_finite(s.delta)) {
+                alt_store(p, s.index,
+                          p.strict ? nan_f() : static_cast<float>(static_cast<double>(s.it) - p.output_bias),
+                          p.strict ? 0u : static_cast<std::uint32_t>(s.it));
+                return kAltDone;
             }
-            if (++s.length >= s.power) {
-                s.tortoise = total;
-                s.power = s.power * 2 < (1 << 20) ? s.power * 2 : (1 << 20);
-                s.length = 0;
-            }
+            if (alt_escaped<WithPlanes>(p, s)) return kAltEscaped;
         }
+        if (step != nullptr) return kAltContinue;
+    } else {
+        s.pending = false;
+        if (alt_escaped<WithPlanes>(p, s)) return kAltEscaped;
     }
-    return false;
+    if (p.cycle && s.it >= 2048 && (s.it & 31) == 0 && alt_cycle<WithPlanes>(p, s)) {
+        return alt_interior<WithPlanes>(p, s.index);
+    }
+    return kAltContinue;
 }
 
 __device__ __forceinline__ int alt_max_block(const AltParams& p) {
@@ -680,127 +775,181 @@ __device__ __forceinline__ unsigned long long alt_deadline(const AltParams& p) {
     return p.deadline_base ? *p.deadline_base + p.budget_ns : 0ull;
 }
 
-// One thread per pixel (point lists).
-template <bool WithPlanes, int Formula>
-__global__ void __launch_bounds__(128) alt_kernel(const AltParams p) {
-    const long long pixels = static_cast<long long>(p.width) * p.height;
-    const long long index = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (index >= pixels) return;
-    const unsigned long long deadline = alt_deadline(p);
-    const int max_block = alt_max_block(p);
-    AltLane<WithPlanes> begun;
-    bool done = alt_begin<WithPlanes, Formula>(p, index, begun);
-    AltLane<WithPlanes> s = begun;  // in registers: `begun` lives in memory for the call
-    while (!done) done = alt_advance<WithPlanes, Formula>(p, s, deadline, max_block);
-}
-
-// Lane-refill queue for Julia fields.  GB300 issues an FP64 warp
-// instruction at the same cost whatever the number of active lanes, and a
-// Julia view (the dynamic plane, crossed by the Julia set) mixes a few very
-// long orbits with many short ones: 99 % of pixels under 100 iterations,
-// some at the cap, so a warp that keeps a lane per pixel runs mostly empty.
-// Persistent warps instead keep every lane busy: each lane holds one
-// pixel's state, the warp runs kAltRound turns of the loop, and lanes whose
-// pixel finished take new ones (claimed for the whole warp with one atomic
-// on the launch's counter) once at least kAltRefill of them wait, or when
-// none has work left.  Parameter-plane views (burning ship, tricorn) have
-// escape times close together; there lanes that start together stay on the
-// same branch of the loop, and one thread per pixel is faster (measured:
-// 1.47 s against 2.23 s for a 3840x2160 burning-ship field at 1e94).
-constexpr int kAltRound = 16;
+// The lane-refill queue.  GB300 issues an FP64 warp instruction at the same
+// cost whatever the number of active lanes, and neighbouring pixels run for
+// different times: a lane per pixel left 8 of 32 lanes active on average on a
+// burning-ship view at 1e40 and 7 on a Julia view at 1e24.  So persistent
+// warps keep every lane busy: each lane holds one pixel, the warp runs rounds
+// of kAltRound raw steps and a general turn for the lanes that stopped, and
+// lanes whose pixel finished take new ones (one atomic per warp) once at
+// least kAltRefill of them wait.
+//
+// A pixel still running after its launch's budget of rounds is spilled with
+// its whole state to a list that the next launch takes as its input, so the
+// few long orbits (1 % of a Julia view, up to the cap) run 32 to a warp
+// instead of one in each.  The budgets grow by four; the last launch has
+// none, and a pixel that finds the list full runs on where it is.
 constexpr int kAltRefill = 8;
+constexpr int kAltPhases = 5;
+constexpr int kAltFirstBudget = 32;          // rounds: 512 steps
+constexpr long long kAltPhasePixels = 16384; // smaller fields run in one launch
 
-template <bool WithPlanes>
-__global__ void __launch_bounds__(128) alt_queue_kernel(const AltParams p, unsigned long long* counter) {
+template <bool WithPlanes, int Formula>
+__global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ AltParams p, unsigned long long* claim,
+                                                        const AltLane<WithPlanes>* source,
+                                                        const unsigned long long* source_count,
+                                                        AltLane<WithPlanes>* spill, unsigned long long* spill_count,
+                                                        unsigned long long spill_capacity, int budget) {
     constexpr unsigned kFull = 0xffffffffu;
+    __shared__ AltEnd<WithPlanes> parks[4][kAltPark];
+    AltEnd<WithPlanes>* park = parks[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
-    const long long pixels = static_cast<long long>(p.width) * p.height;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned long long items = static_cast<unsigned long long>(p.width) * static_cast<unsigned long long>(p.height);
+    if (source != nullptr) {
+        items = *source_count;
+        if (items > spill_capacity) items = spill_capacity;
+    }
     const unsigned long long deadline = alt_deadline(p);
     const int max_block = alt_max_block(p);
     AltLane<WithPlanes> s;
     bool have = false;
+    bool keep = false;  // the spill list was full: run on
     bool drained = false;
+    int parked = 0;
     while (true) {
+        AltOutcome outcome = kAltContinue;
         if (!drained) {
-            unsigned need = __ballot_sync(kFull, !have);
-            while (__popc(need) >= kAltRefill) {
-                const unsigned n = static_cast<unsigned>(__popc(need));
+            const unsigned need = __ballot_sync(kFull, !have);
+            const unsigned n = static_cast<unsigned>(__popc(need));
+            if (n >= kAltRefill) {
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(counter, static_cast<unsigned long long>(n));
+                if (lane == 0) base = atomicAdd(claim, static_cast<unsigned long long>(n));
                 base = __shfl_sync(kFull, base, 0);
-                if (!have) {
-                    const long long index = static_cast<long long>(base) + __popc(need & ((1u << lane) - 1u));
-                    if (index < pixels) {
-                        AltLane<WithPlanes> begun;
-                        have = !alt_begin<WithPlanes, kFormulaJulia>(p, index, begun);
-                        s = begun;
+                const unsigned long long item = base + static_cast<unsigned>(__popc(need & below));
+                if (!have && item < items) {
+                    have = true;
+                    keep = false;
+                    if (source == nullptr) {
+                        outcome = alt_begin<WithPlanes, Formula>(p, static_cast<long long>(item), s);
+                    } else {
+                        s = source[item];
+                        s.rounds = 0;
                     }
                 }
-                if (static_cast<long long>(base) + n >= pixels) {
-                    drained = true;
-                    break;
-                }
-                need = __ballot_sync(kFull, !have);
+                drained = base + n >= items;
             }
         }
         if (!__any_sync(kFull, have)) {
             if (drained) break;
             continue;
         }
-        // One copy of the loop body: unrolled, the turns would multiply the
-        // kernel's code and miss in the instruction cache.
-#pragma unroll 1
-        for (int k = 0; k < kAltRound; ++k) {
-            if (have && alt_advance<WithPlanes, kFormulaJulia>(p, s, deadline, max_block)) have = false;
+        bool stopped = false;
+        if (have && outcome == kAltContinue) {
+            stopped = alt_raw_run<WithPlanes, Formula>(p, s, kAltRound) < kAltRound || s.pending;
+            ++s.rounds;
+        }
+        if (stopped) outcome = alt_general<WithPlanes, Formula>(p, s, max_block);
+        if (have && outcome == kAltContinue && deadline && (s.ticks++ & 15u) == 0u && global_ns() >= deadline) {
+            alt_store(p, s.index, nan_f(), 0u);
+            outcome = kAltDone;
+        }
+        const unsigned ended = __ballot_sync(kFull, have && outcome == kAltEscaped);
+        if (ended != 0u) {
+            if (have && outcome == kAltEscaped) {
+                AltEnd<WithPlanes>& e = park[parked + __popc(ended & below)];
+                e.index = s.index;
+                e.norm = s.norm;
+                e.it = s.it;
+                if constexpr (WithPlanes) {
+                    e.total = s.total;
+                    e.prior = sc_norm2(normal_form(s.prior));
+                    e.jac = s.jac;
+                }
+            }
+            parked += __popc(ended);
+            __syncwarp();
+            if (parked >= 32) {
+                parked -= 32;
+                alt_finish<WithPlanes, Formula>(p, park[parked + static_cast<int>(lane)]);
+                __syncwarp();
+            }
+        }
+        if (outcome != kAltContinue) have = false;
+        if (budget > 0) {
+            const bool over = have && !keep && s.rounds >= budget;
+            const unsigned mask = __ballot_sync(kFull, over);
+            if (mask != 0u) {
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(spill_count, static_cast<unsigned long long>(__popc(mask)));
+                base = __shfl_sync(kFull, base, 0);
+                const unsigned long long slot = base + static_cast<unsigned>(__popc(mask & below));
+                if (over) {
+                    if (slot < spill_capacity) {
+                        spill[slot] = s;
+                        have = false;
+                    } else {
+                        keep = true;
+                    }
+                }
+            }
         }
     }
+    if (static_cast<int>(lane) < parked) alt_finish<WithPlanes, Formula>(p, park[lane]);
 }
 
-template <bool WithPlanes>
+template <bool WithPlanes, int Formula>
 int alt_queue_blocks() {
     static int blocks = 0;
     if (blocks == 0) {
         int per_sm = 0, sms = 0, device = 0;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alt_queue_kernel<WithPlanes>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alt_queue_kernel<WithPlanes, Formula>, 128, 0);
         blocks = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
     }
     return blocks;
 }
 
+// The launches of one field: `queue.counters` holds the claim counters and
+// spill counts (kAltQueueCounters words), `queue.spill` two lists.
+template <bool WithPlanes, int Formula>
+cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t stream) {
+    const long long pixels = static_cast<long long>(p.width) * p.height;
+    const int phases = pixels > kAltPhasePixels && queue.spill != nullptr && queue.capacity > 0 ? kAltPhases : 1;
+    const cudaError_t cleared =
+        cudaMemsetAsync(queue.counters, 0, sizeof(unsigned long long) * kAltQueueCounters, stream);
+    if (cleared != cudaSuccess) return cleared;
+    auto* lists = static_cast<AltLane<WithPlanes>*>(queue.spill);
+    const long long resident = alt_queue_blocks<WithPlanes, Formula>();
+    int budget = kAltFirstBudget;
+    for (int phase = 0; phase < phases; ++phase, budget *= 4) {
+        // A field (or a full list) smaller than the persistent grid needs no
+        // more warps than items / 32.
+        const long long items = phase == 0 ? pixels : std::min<long long>(queue.capacity, pixels);
+        const unsigned grid = static_cast<unsigned>(std::min<long long>(resident, (items + 127) / 128));
+        alt_queue_kernel<WithPlanes, Formula><<<grid, 128, 0, stream>>>(
+            p, queue.counters + phase, phase == 0 ? nullptr : lists + ((phase - 1) & 1) * queue.capacity,
+            phase == 0 ? nullptr : queue.counters + kAltPhases + phase - 1, lists + (phase & 1) * queue.capacity,
+            queue.counters + kAltPhases + phase, static_cast<unsigned long long>(queue.capacity),
+            phase + 1 < phases ? budget : 0);
+    }
+    return cudaGetLastError();
+}
+
 }  // namespace
 
-cudaError_t launch_plain_alternate(const AltParams& p, bool planes, bool stats, unsigned long long* queue_counter,
-                                   cudaStream_t stream) {
-    (void)stats;
-    const long long pixels = static_cast<long long>(p.width) * p.height;
-    if (queue_counter != nullptr && p.points == nullptr && p.formula == kFormulaJulia) {
-        const cudaError_t cleared = cudaMemsetAsync(queue_counter, 0, sizeof(unsigned long long), stream);
-        if (cleared != cudaSuccess) return cleared;
-        // A field smaller than the persistent grid needs no more warps than pixels / 32.
-        const long long needed = (pixels + 127) / 128;
-        if (planes) {
-            const long long grid = std::min<long long>(alt_queue_blocks<true>(), needed);
-            alt_queue_kernel<true><<<static_cast<unsigned>(grid), 128, 0, stream>>>(p, queue_counter);
-        } else {
-            const long long grid = std::min<long long>(alt_queue_blocks<false>(), needed);
-            alt_queue_kernel<false><<<static_cast<unsigned>(grid), 128, 0, stream>>>(p, queue_counter);
-        }
-        return cudaGetLastError();
-    }
-    const unsigned grid = static_cast<unsigned>((pixels + 127) / 128);
+std::size_t alt_spill_entry_bytes() { return sizeof(AltLane<true>); }
+
+cudaError_t launch_plain_alternate(const AltParams& p, bool planes, const AltQueue& queue, cudaStream_t stream) {
+    static_assert(2 * kAltPhases <= kAltQueueCounters, "claim counters and spill counts");
     const auto launch = [&](auto formula) {
-        if (planes) {
-            alt_kernel<true, formula.value><<<grid, 128, 0, stream>>>(p);
-        } else {
-            alt_kernel<false, formula.value><<<grid, 128, 0, stream>>>(p);
-        }
+        return planes ? alt_launch<true, formula.value>(p, queue, stream)
+                      : alt_launch<false, formula.value>(p, queue, stream);
     };
-    if (p.formula == kFormulaJulia) launch(std::integral_constant<int, kFormulaJulia>{});
-    else if (p.formula == kFormulaBurningShip) launch(std::integral_constant<int, kFormulaBurningShip>{});
-    else launch(std::integral_constant<int, kFormulaTricorn>{});
-    return cudaGetLastError();
+    if (p.formula == kFormulaJulia) return launch(std::integral_constant<int, kFormulaJulia>{});
+    if (p.formula == kFormulaBurningShip) return launch(std::integral_constant<int, kFormulaBurningShip>{});
+    return launch(std::integral_constant<int, kFormulaTricorn>{});
 }
 
 }  // namespace fgb

@@ -46,7 +46,8 @@ enum ScratchSlot {
     kScratchPlanesIn,
     kScratchPlanesOut,
     kScratchDiscard,  // planes a batch's plain kernels write but no caller asked for
-    kScratchAltQueue, // claim counters of the alternate-formula queue (one per lane stream + one)
+    kScratchAltQueue, // counters of the alternate-formula queue (one set per lane stream + one)
+    kScratchAltSpill, // its spill lists, likewise
     kScratchCount
 };
 
