@@ -345,6 +345,7 @@ struct AltQueues {
     char* counters = nullptr;
     char* spill = nullptr;
     long long capacity = 0;
+    std::size_t slot_bytes = 0;
 };
 
 // Sized for fields of up to `pixels` pixels in `slots` slots at once.
@@ -352,14 +353,16 @@ AltQueues alt_queues(ThreadRuntime& rt, long long pixels, int slots) {
     AltQueues q;
     q.counters = static_cast<char*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * kAltQueueStride));
     q.capacity = std::min<long long>(pixels, 65536);
-    q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill,
-                                         static_cast<std::size_t>(slots) * 2 * q.capacity * alt_spill_entry_bytes()));
+    q.slot_bytes = 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes() + alt_ready_bytes();
+    q.slot_bytes = (q.slot_bytes + 255) / 256 * 256;
+    q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill, slots * q.slot_bytes));
     return q;
 }
 
 AltQueue alt_queue_slot(const AltQueues& q, int counters, int list) {
-    return AltQueue{reinterpret_cast<unsigned long long*>(q.counters + counters * kAltQueueStride),
-                    q.spill + static_cast<std::size_t>(list) * 2 * q.capacity * alt_spill_entry_bytes(), q.capacity};
+    char* const lists = q.spill + list * q.slot_bytes;
+    return AltQueue{reinterpret_cast<unsigned long long*>(q.counters + counters * kAltQueueStride), lists, q.capacity,
+                    lists + 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes()};
 }
 
 // `queue`: the lane's slot of a batch; NULL takes the single-render slot.

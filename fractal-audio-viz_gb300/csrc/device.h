@@ -452,14 +452,17 @@ void render_floatexp_from_reference(ReferenceContext& ctx, const Outputs& out, i
 
 cudaError_t launch_plain_mandelbrot(const PlainParams& params, bool planes, bool stats, cudaStream_t stream);
 // Device memory of one alternate-formula render, which no other launch uses
-// at the same time: kAltQueueCounters words and two spill lists of `capacity`
-// entries each (alt_spill_entry_bytes; may be absent).
+// at the same time: kAltQueueCounters words, two spill lists of `capacity`
+// entries each (alt_spill_entry_bytes) and the warps' lists of started pixels
+// (alt_ready_bytes).
 constexpr int kAltQueueCounters = 16;
 struct AltQueue {
     unsigned long long* counters;
     void* spill;
     long long capacity;
+    void* ready;
 };
+std::size_t alt_ready_bytes();
 std::size_t alt_spill_entry_bytes();
 cudaError_t launch_plain_alternate(const AltParams& params, bool planes, const AltQueue& queue, cudaStream_t stream);
 // A batch of direct fields (one kernel over all of them); the batch struct

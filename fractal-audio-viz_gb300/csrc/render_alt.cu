@@ -176,13 +176,17 @@ __device__ __noinline__ Fe alt_margin(const AltParams& p, int i, Sc d) {
 // free; a NaN or an overflow fails.  The margin, the norm and the total cost
 // 11 FP64 instructions (880 cycles of a sub-partition) and only the sign
 // matters until the pixel escapes.
-__device__ __forceinline__ bool alt_inside(const AltParams& p, int i, const Sc& d) {
+// `bound` is R^2, or 3 for a block's endpoint (refused from there on).
+__device__ __forceinline__ bool alt_below(const AltParams& p, int i, const Sc& d, float bound) {
     const float2 z = __ldg(reinterpret_cast<const float2*>(&p.orbit[i].zf_re));
     const int e = imax(imin(d.e, 64), -4096);
     const float dx = float_of(d.re, e), dy = float_of(d.im, e);
     const float tx = z.x + dx, ty = z.y + dy;
-    const float r2 = p.escape_mode == 1 ? 1.0e8f : 4.0f;
-    return tx * tx + ty * ty < r2 * (1.0f - 0x1p-14f) && dx * dx + dy * dy < r2 * 16.0f;
+    return tx * tx + ty * ty < bound * (1.0f - 0x1p-14f) && dx * dx + dy * dy < bound * 16.0f;
+}
+
+__device__ __forceinline__ bool alt_inside(const AltParams& p, int i, const Sc& d) {
+    return alt_below(p, i, d, p.escape_mode == 1 ? 1.0e8f : 4.0f);
 }
 
 // Whether adding d to r changes which side of zero it is on (zero counts
@@ -723,11 +727,15 @@ __device__ __noinline__ AltOutcome alt_general(const AltParams& p, AltLane<WithP
         if (step != nullptr && s.ref + len < p.orbit_size) {
             const int end = s.ref + len;
             const Sc cand = apply_alt(step, s.delta, s.pd);
-            const Fe cmargin = alt_margin(p, end, cand);
-            const Nrm cnorm = nrm_from_margin(cmargin, p.escape_mode);
-            const bool bad = !sc_finite(cand) || !fe_finite(cmargin) || !sc_finite(alt_total(p, end, cand))
-                || fe_positive(cmargin) || nrm_cmp(cnorm, nrm_make(0.75, 2)) >= 0;
-            if (!bad) {
+            // Accepted where the endpoint stays inside (|Z + d|^2 < 3; the
+            // total is finite when the delta is).
+            bool good = sc_finite(cand);
+            if (good && !alt_below(p, end, cand, 3.0f)) {
+                const Fe cmargin = alt_margin(p, end, cand);
+                good = fe_finite(cmargin) && !fe_positive(cmargin)
+                    && nrm_cmp(nrm_from_margin(cmargin, p.escape_mode), nrm_make(0.75, 2)) < 0;
+            }
+            if (good) {
                 s.delta = to_raw(cand);
                 if constexpr (WithPlanes) s.jac = jac_pack(jac_bla(step, s.jac, !julia));
                 s.ref = end;
@@ -781,8 +789,13 @@ __device__ __forceinline__ unsigned long long alt_deadline(const AltParams& p) {
 // burning-ship view at 1e40 and 7 on a Julia view at 1e24.  So persistent
 // warps keep every lane busy: each lane holds one pixel, the warp runs rounds
 // of kAltRound raw steps and a general turn for the lanes that stopped, and
-// lanes whose pixel finished take new ones (one atomic per warp) once at
-// least kAltRefill of them wait.
+// lanes whose pixel finished take new ones once at least kAltRefill of them
+// wait.  A general turn is some 2000 instructions of mostly integer work, so
+// it is shared too: lanes that need one wait until kAltRefill do, and 32
+// neighbouring pixels are started together (one claim), run through their
+// first blocks, which neighbours take in step, and kept on the warp's list
+// of ready pixels.  Run by the lanes just refilled, the starts and blocks
+// took 80 % of the instructions.
 //
 // A pixel still running after its launch's budget of rounds is spilled with
 // its whole state to a list that the next launch takes as its input, so the
@@ -799,7 +812,8 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
                                                         const AltLane<WithPlanes>* source,
                                                         const unsigned long long* source_count,
                                                         AltLane<WithPlanes>* spill, unsigned long long* spill_count,
-                                                        unsigned long long spill_capacity, int budget) {
+                                                        unsigned long long spill_capacity, int budget,
+                                                        AltLane<WithPlanes>* ready_lists) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ AltEnd<WithPlanes> parks[4][kAltPark];
     AltEnd<WithPlanes>* park = parks[threadIdx.x >> 5];
@@ -815,69 +829,105 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
     AltLane<WithPlanes> s;
     bool have = false;
     bool keep = false;  // the spill list was full: run on
+    bool wait = false;  // the lane's pixel needs a general turn
     bool drained = false;
     int parked = 0;
+    int ready = 0;  // pixels on the warp's list
+    AltLane<WithPlanes>* list = ready_lists + static_cast<std::size_t>(blockIdx.x * 4 + (threadIdx.x >> 5)) * kAltPark;
+    // Park the escaped among the warp's lanes `l`; finish 32 when they are there.
+    const auto park_escaped = [&](bool escaped, const AltLane<WithPlanes>& l) {
+        const unsigned ended = __ballot_sync(kFull, escaped);
+        if (ended == 0u) return;
+        if (escaped) {
+            AltEnd<WithPlanes>& e = park[parked + __popc(ended & below)];
+            e.index = l.index;
+            e.norm = l.norm;
+            e.it = l.it;
+            if constexpr (WithPlanes) {
+                e.total = l.total;
+                e.prior = sc_norm2(normal_form(l.prior));
+                e.jac = l.jac;
+            }
+        }
+        parked += __popc(ended);
+        __syncwarp();
+        if (parked >= 32) {
+            parked -= 32;
+            alt_finish<WithPlanes, Formula>(p, park[parked + static_cast<int>(lane)]);
+            __syncwarp();
+        }
+    };
     while (true) {
         AltOutcome outcome = kAltContinue;
-        if (!drained) {
-            const unsigned need = __ballot_sync(kFull, !have);
-            const unsigned n = static_cast<unsigned>(__popc(need));
-            if (n >= kAltRefill) {
+        const unsigned need = __ballot_sync(kFull, !have);
+        const int n = __popc(need);
+        if (n >= kAltRefill && !(drained && ready == 0)) {
+            const int rank = __popc(need & below);
+            if (source != nullptr) {
                 unsigned long long base = 0;
                 if (lane == 0) base = atomicAdd(claim, static_cast<unsigned long long>(n));
                 base = __shfl_sync(kFull, base, 0);
-                const unsigned long long item = base + static_cast<unsigned>(__popc(need & below));
-                if (!have && item < items) {
+                if (!have && base + rank < items) {
+                    s = source[base + rank];
+                    s.rounds = 0;
                     have = true;
-                    keep = false;
-                    if (source == nullptr) {
-                        outcome = alt_begin<WithPlanes, Formula>(p, static_cast<long long>(item), s);
-                    } else {
-                        s = source[item];
-                        s.rounds = 0;
-                    }
                 }
                 drained = base + n >= items;
+            } else {
+                if (ready < n && !drained) {
+                    unsigned long long base = 0;
+                    if (lane == 0) base = atomicAdd(claim, 32ull);
+                    base = __shfl_sync(kFull, base, 0);
+                    AltLane<WithPlanes> t;
+                    AltOutcome started = kAltDone;
+                    if (base + lane < items) {
+                        started = alt_begin<WithPlanes, Formula>(p, static_cast<long long>(base + lane), t);
+                        while (started == kAltContinue && !p.disable_bla && p.alt_index.levels > 1
+                               && !no_block(p, t.ref - p.alt_start, t.delta)) {
+                            started = alt_general<WithPlanes, Formula>(p, t, max_block);
+                        }
+                    }
+                    drained = base + 32 >= items;
+                    __syncwarp();
+                    park_escaped(started == kAltEscaped, t);
+                    const unsigned kept = __ballot_sync(kFull, started == kAltContinue);
+                    if (started == kAltContinue) list[ready + __popc(kept & below)] = t;
+                    ready += __popc(kept);
+                    __syncwarp();
+                }
+                if (!have && rank < ready) {
+                    s = list[ready - 1 - rank];
+                    have = true;
+                }
+                ready -= n < ready ? n : ready;
+                __syncwarp();
+            }
+            if ((need >> lane) & 1u) {
+                keep = false;
+                wait = false;
             }
         }
         if (!__any_sync(kFull, have)) {
-            if (drained) break;
+            if (drained && ready == 0) break;
             continue;
         }
-        bool stopped = false;
-        if (have && outcome == kAltContinue) {
-            stopped = alt_raw_run<WithPlanes, Formula>(p, s, kAltRound) < kAltRound || s.pending;
+        if (have && !wait) {
+            wait = alt_raw_run<WithPlanes, Formula>(p, s, kAltRound) < kAltRound || s.pending;
             ++s.rounds;
         }
-        if (stopped) outcome = alt_general<WithPlanes, Formula>(p, s, max_block);
+        const int waiting = __popc(__ballot_sync(kFull, have && wait));
+        if (waiting >= kAltRefill || !__any_sync(kFull, have && !wait)) {
+            if (have && wait) outcome = alt_general<WithPlanes, Formula>(p, s, max_block);
+            wait = false;
+        }
         if (have && outcome == kAltContinue && deadline && (s.ticks++ & 15u) == 0u && global_ns() >= deadline) {
             alt_store(p, s.index, nan_f(), 0u);
             outcome = kAltDone;
         }
-        const unsigned ended = __ballot_sync(kFull, have && outcome == kAltEscaped);
-        if (ended != 0u) {
-            if (have && outcome == kAltEscaped) {
-                AltEnd<WithPlanes>& e = park[parked + __popc(ended & below)];
-                e.index = s.index;
-                e.norm = s.norm;
-                e.it = s.it;
-                if constexpr (WithPlanes) {
-                    e.total = s.total;
-                    e.prior = sc_norm2(normal_form(s.prior));
-                    e.jac = s.jac;
-                }
-            }
-            parked += __popc(ended);
-            __syncwarp();
-            if (parked >= 32) {
-                parked -= 32;
-                alt_finish<WithPlanes, Formula>(p, park[parked + static_cast<int>(lane)]);
-                __syncwarp();
-            }
-        }
+        park_escaped(outcome == kAltEscaped, s);
         if (outcome != kAltContinue) have = false;
         if (budget > 0) {
-            const bool over = have && !keep && s.rounds >= budget;
+            const bool over = have && !wait && !keep && s.rounds >= budget;
             const unsigned mask = __ballot_sync(kFull, over);
             if (mask != 0u) {
                 unsigned long long base = 0;
@@ -932,7 +982,7 @@ cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t s
             p, queue.counters + phase, phase == 0 ? nullptr : lists + ((phase - 1) & 1) * queue.capacity,
             phase == 0 ? nullptr : queue.counters + kAltPhases + phase - 1, lists + (phase & 1) * queue.capacity,
             queue.counters + kAltPhases + phase, static_cast<unsigned long long>(queue.capacity),
-            phase + 1 < phases ? budget : 0);
+            phase + 1 < phases ? budget : 0, static_cast<AltLane<WithPlanes>*>(queue.ready));
     }
     return cudaGetLastError();
 }
@@ -940,6 +990,15 @@ cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t s
 }  // namespace
 
 std::size_t alt_spill_entry_bytes() { return sizeof(AltLane<true>); }
+
+// One list of kAltPark pixels per warp of the largest grid.
+std::size_t alt_ready_bytes() {
+    const int blocks = std::max({alt_queue_blocks<true, kFormulaJulia>(), alt_queue_blocks<false, kFormulaJulia>(),
+                                 alt_queue_blocks<true, kFormulaBurningShip>(),
+                                 alt_queue_blocks<false, kFormulaBurningShip>(),
+                                 alt_queue_blocks<true, kFormulaTricorn>(), alt_queue_blocks<false, kFormulaTricorn>()});
+    return static_cast<std::size_t>(blocks) * 4 * kAltPark * sizeof(AltLane<true>);
+}
 
 cudaError_t launch_plain_alternate(const AltParams& p, bool planes, const AltQueue& queue, cudaStream_t stream) {
     static_assert(2 * kAltPhases <= kAltQueueCounters, "claim counters and spill counts");
