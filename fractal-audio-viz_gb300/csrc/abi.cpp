@@ -335,8 +335,8 @@ void launch_deep_mandelbrot(ReferenceContext& ctx, DeviceTables& dev, const Outp
 
 // Counters and spill lists of the alternate-formula queue: one slot per lane
 // stream of a batch, and one (the last) for single renders.  A list holds up
-// to 65,536 pixels (the ones of a field that outlast a launch's budget;
-// beyond that they run on where they are).
+// to 524,288 pixels of 128 bytes (the ones of a field that outlast a launch's
+// budget: 10 % of a Julia view; beyond that they run on where they are).
 constexpr int kAltQueueSlots = ThreadRuntime::kPlainLanes + 1;
 constexpr std::size_t kAltQueueStride = 256;
 static_assert(kAltQueueCounters * sizeof(unsigned long long) <= kAltQueueStride, "one slot");
@@ -352,7 +352,7 @@ struct AltQueues {
 AltQueues alt_queues(ThreadRuntime& rt, long long pixels, int slots) {
     AltQueues q;
     q.counters = static_cast<char*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * kAltQueueStride));
-    q.capacity = std::min<long long>(pixels, 65536);
+    q.capacity = std::min<long long>(pixels, 1ll << 19);
     q.slot_bytes = 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes() + alt_ready_bytes();
     q.slot_bytes = (q.slot_bytes + 255) / 256 * 256;
     q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill, slots * q.slot_bytes));
@@ -376,6 +376,7 @@ void launch_deep_alternate(ReferenceContext& ctx, DeviceTables& dev, const Outpu
     p.alt = dev.alt;
     p.alt_index = dev.alt_index;
     p.alt_start = ctx.alt_start;
+    p.block_top = dev.block_top;
     p.alt_input_radius2 = ctx.alt_input_radius2;
     p.series = dev.series;
     p.series_terms = dev.series_terms;

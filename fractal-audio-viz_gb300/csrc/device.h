@@ -80,6 +80,7 @@ struct DeviceTables {
     LevelIndex deep_linear_index;
     AltStep* alt = nullptr;
     LevelIndex alt_index;
+    int block_top = 0;  // see AltParams
     fx::Sc* series = nullptr;
     int series_terms = 0;
     // floatexp mirrors (built on the first floatexp render)
@@ -153,6 +154,7 @@ struct AltParams {
     const AltStep* alt;
     LevelIndex alt_index;
     int alt_start;
+    int block_top;  // no block's squared radius reaches 2^block_top
     fx::Fe alt_input_radius2;
     const fx::Sc* series;
     int series_terms;

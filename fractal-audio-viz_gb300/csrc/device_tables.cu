@@ -6,11 +6,13 @@
 // same way, renderer.cpp:9077-9245).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <stdexcept>
 #include <string>
 #include <vector>
 
+#include "bla_math.h"
 #include "device.h"
 #include "runtime.h"
 
@@ -193,6 +195,11 @@ std::shared_ptr<DeviceTables> device_tables(ReferenceContext& ctx) {
         const std::vector<OrbitRec> records = make_orbit_records(ctx);
         t.orbit = upload(records);
         t.orbit_size = static_cast<int>(records.size());
+        // A 2x2 block's radius is at most that of its first step, the
+        // tolerance times max(|Z|, 1) (or less): merging only shrinks it.
+        int top = 0;
+        for (const OrbitRec& r : records) top = std::max(top, r.top - 1022);
+        t.block_top = 2 * (bla_tolerance().e + top + 2);
         t.series = upload(ctx.series.coeff);
         t.series_terms = static_cast<int>(ctx.series.coeff.size());
         if (!ctx.bla_on_device) {

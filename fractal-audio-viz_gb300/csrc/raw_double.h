@@ -11,8 +11,8 @@
 // 21 of 27 cycles for instructions).  Two rules remain:
 //   * a ScaledComplex sum drops the whole smaller operand when the shared
 //     exponents differ by more than 60 (add_cut);
-//   * a zero component has no exponent; values with one take the general
-//     path where its sign could be seen.
+//   * the sign of a zero may differ (FloatExp products and exact sums give
+//     +0): a zero is accepted where it meets a nonzero value next.
 // "Raw" below: a ScaledComplex whose exponent word is 0 and whose parts are
 // the values themselves, not normalised.
 //
@@ -36,6 +36,7 @@ constexpr unsigned kRawSpan = 410;    // 2^-400 .. 2^10
 constexpr unsigned kJacSpan = 800;    // 2^-400 .. 2^400
 
 FX_HD bool raw_part(double v) { return static_cast<unsigned>(bexp(v) - kRawLow) <= kRawSpan; }
+FX_HD bool raw_or_zero(double v) { return raw_part(v) || is_zero(v); }
 FX_HD bool raw_value(const Sc& v) { return v.e == 0 && raw_part(v.re) && raw_part(v.im); }
 
 // The normal form of a value in either form.

@@ -931,6 +931,7 @@ std::vector<OrbitRec> make_orbit_records(const ReferenceContext& ctx) {
         const bool raw = fx::raw_value(fx::sc_make(fx::sc_re_d(r.z), fx::sc_im_d(r.z), 0))
             && r.zd_re == fx::sc_re_d(r.z) && r.zd_im == fx::sc_im_d(r.z);
         r.raw = raw ? kRawOrbit : 0;
+        r.top = fx::imax(fx::bexp(r.zd_re), fx::bexp(r.zd_im));
         r.parts = fx::sc_to_fec(orbit.scaled[i]);
         // Mandelbrot rebuilds the escape margin from the compact orbit
         // (renderer.cpp:8374-8390); the other formulas use the MPFR margin

@@ -62,7 +62,7 @@ struct alignas(128) OrbitRec {
     float zf_re;       // Z_i rounded to float: the estimates that settle a
     float zf_im;       // test far from its bound without FP64
     int raw;           // kRawOrbit, kRawFold (raw_double.h)
-    int pad;
+    int top;           // biased exponent of the larger part of Z_i
     fx::Sc z;          // compact orbit value Z_i
     fx::Fec parts;     // Z_i components as FloatExp (escape margin input)
     fx::Fe margin;     // |Z_i|^2 - R^2 (escape margin constant term)

@@ -347,7 +347,7 @@ __device__ __forceinline__ Sc alt_step_raw(const double2& z, const Sc& d, const 
         return sc_make(tr + choose(fold, sr, pd.re), flip(ti, s) + choose(fold, fabs_(si), pd.im), 0);
     }
     const double sr = d.re * d.re - d.im * d.im;
-    const double si = add_exp(d.re * d.im, 1);
+    const double si = twice_raw(d.re * d.im);
     if constexpr (Formula == kFormulaTricorn) {
         return add_cut(sc_make(lr, neg_(li), 0), add_cut(sc_make(sr, neg_(si), 0), pd));
     }
@@ -433,6 +433,18 @@ struct AltLane {
     bool ready, past, pending;
 };
 
+// A pixel between rounds, as it waits on a list: 128 bytes.  Only pixels
+// without cycle state are listed.
+struct alignas(128) AltSaved {
+    long long index;
+    Sc dc;
+    Sc value;  // delta, or total past the orbit's end
+    Jac jac;
+    int ref;   // -1 past the orbit's end
+    int it;
+};
+static_assert(sizeof(AltSaved) == 128, "one cache line");
+
 enum AltOutcome { kAltContinue = 0, kAltDone, kAltEscaped };
 
 __device__ __forceinline__ void alt_store(const AltParams& p, long long index, float out, std::uint32_t count) {
@@ -495,6 +507,45 @@ __device__ __noinline__ bool alt_escaped(const AltParams& p, AltLane<WithPlanes>
     return true;
 }
 
+template <bool WithPlanes>
+__device__ __forceinline__ void alt_save(const AltLane<WithPlanes>& s, AltSaved& e) {
+    e.index = s.index;
+    e.dc = s.dc;
+    e.value = s.past ? s.total : s.delta;
+    if constexpr (WithPlanes) e.jac = s.jac;
+    e.ref = s.past ? -1 : s.ref;
+    e.it = s.it;
+}
+
+// What does not change from step to step, from the pixel's offset dc.
+template <bool WithPlanes, int Formula>
+__device__ __forceinline__ void alt_reset(AltLane<WithPlanes>& s, const Sc& dc) {
+    constexpr bool julia = Formula == kFormulaJulia;
+    const Nrm pnorm = julia ? nrm_make(0.0, 0) : sc_norm2(dc);
+    s.dc = dc;
+    s.pd = julia ? sc_zero() : to_raw(dc);
+    s.pn = fe_make(pnorm.m, pnorm.e);
+    s.total = s.tortoise = s.prior = sc_zero();
+    s.ticks = 0;
+    s.past = s.pending = s.ready = false;
+    s.power = 1;
+    s.length = 0;
+    s.hits = 0;
+    s.rounds = 0;
+}
+
+template <bool WithPlanes, int Formula>
+__device__ __noinline__ void alt_restore(const AltParams& p, const AltSaved& e, AltLane<WithPlanes>& s) {
+    alt_reset<WithPlanes, Formula>(s, e.dc);
+    s.index = e.index;
+    s.past = e.ref < 0;
+    s.delta = e.value;
+    if (s.past) s.total = e.value;
+    if constexpr (WithPlanes) s.jac = e.jac;
+    s.ref = s.past ? p.orbit_size - 1 : e.ref;
+    s.it = e.it;
+}
+
 // Start pixel `index`: coordinates, Julia series jump, first escape test.
 template <bool WithPlanes, int Formula>
 __device__ __noinline__ AltOutcome alt_begin(const AltParams& p, long long index, AltLane<WithPlanes>& s) {
@@ -506,7 +557,6 @@ __device__ __noinline__ AltOutcome alt_begin(const AltParams& p, long long index
     const double yf = -pixel_offset(py, p.height, p.coordinate_mode) / static_cast<double>(p.height);
     const Sc dc = p.points ? sc_make(p.points[index].re, p.points[index].im, p.points[index].e)
                            : sc_from_fe(fe_mul(p.view_width, xf), fe_mul(p.view_height, yf));
-    const Nrm pnorm = julia ? nrm_make(0.0, 0) : sc_norm2(dc);
     Sc delta = dc;
     Jac jac = jac_identity();
     int at = julia ? 0 : 1;
@@ -521,21 +571,12 @@ __device__ __noinline__ AltOutcome alt_begin(const AltParams& p, long long index
         if constexpr (WithPlanes) jac = jac_holomorphic(sc_add(sc_mul(poly, dc), value));
         at = p.series_iteration;
     }
+    alt_reset<WithPlanes, Formula>(s, dc);
     s.index = index;
-    s.dc = dc;
-    s.pd = julia ? sc_zero() : to_raw(dc);
-    s.pn = fe_make(pnorm.m, pnorm.e);
     s.delta = to_raw(delta);
     s.jac = jac_pack(jac);
     s.ref = at;
     s.it = at;
-    s.ticks = 0;
-    s.past = s.pending = s.ready = false;
-    s.total = s.tortoise = s.prior = sc_zero();
-    s.power = 1;
-    s.length = 0;
-    s.hits = 0;
-    s.rounds = 0;
     if (!alt_inside(p, at, s.delta)) {
         s.norm = nrm_from_margin(alt_margin(p, at, s.delta), p.escape_mode);
         if (nrm_outside(s.norm, p.escape_mode)) {
@@ -546,20 +587,37 @@ __device__ __noinline__ AltOutcome alt_begin(const AltParams& p, long long index
     return kAltContinue;
 }
 
+// Square of a value below 2^128 in magnitude, low to about 2^-19, from its
+// high word.
+__device__ __forceinline__ float square_estimate(double v) {
+    const float f = __int_as_float(imax((hi_of(v) & 0x7fffffff) - (896 << 20), 0) << 3);
+    return f * f;
+}
+
+// High words of magnitudes: they order values to 2^-20.
+constexpr int kHighLow = kRawLow << 20;                                 // 2^-400
+constexpr int kHighTop = (kRawLow + static_cast<int>(kRawSpan)) << 20;  // 2^10
+constexpr int kHighJac = (1023 + 300) << 20;
+__device__ __forceinline__ int high(double v) { return hi_of(v) & 0x7fffffff; }
+
 // Up to `limit` exact steps on raw values, the hot loop: it stops before a
 // step that needs the general turn (a block may apply, a value out of range,
 // the orbit's end, the cap) and after one whose escape or cycle test the
 // general turn must settle (`pending`).  Returns the steps taken.
 //
 // FP64 instructions per step: 14 (12 for Julia), with planes 16 more (the
-// total and the Jacobian).
+// total and the Jacobian).  Long orbits run few to an SM, where a step costs
+// its instructions' issue and latency, so the usual step (`plain`) has every
+// test on high words: nonzero parts in range, no block as large as the
+// delta, and exponents near enough that no shared-exponent sum drops an
+// operand (2 Z d and d^2 differ by the exponents of 2 Z and d, to within 4).
+// The other steps on raw values take the longer form.
 template <bool WithPlanes, int Formula>
 __device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlanes>& s, int limit) {
-    constexpr bool julia = Formula == kFormulaJulia;
     const Sc pd = s.pd;
     Sc d = s.delta;
     RawJac j{};
-    bool fits = !s.past && !s.pending && d.e == 0 && (julia || raw_value(pd));
+    bool fits = !s.past && !s.pending && d.e == 0 && pd.e == 0 && raw_or_zero(pd.re) && raw_or_zero(pd.im);
     if constexpr (WithPlanes) {
         j = RawJac{s.jac.xa.m, s.jac.xb.m, s.jac.ya.m, s.jac.yb.m, s.jac.xa.e};
         fits = fits && j.k == s.jac.xb.e && j.k == s.jac.ya.e && j.k == s.jac.yb.e;
@@ -568,52 +626,125 @@ __device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlane
     const int first = s.ref;
     const int room = imin(imin(limit, p.max_iter - s.it), p.orbit_size - 1 - first);
     const bool blocks = !p.disable_bla && p.alt_index.levels > 1;
+    // |d|^2 >= 2^(2E - 2) with E = top - 1022: no block from this top on.
+    const int block_top = blocks ? imin(imax(p.block_top, -4000), 4000) : -4000;
     const int cycle_from = p.cycle ? 2048 : INT_MAX;
+    const int pd_top = imax(bexp(pd.re), bexp(pd.im));
     const OrbitRec* r = p.orbit + first;
     double2 z = __ldg(reinterpret_cast<const double2*>(r));
-    int flags = __ldg(&r->raw);
-    const float r2 = p.escape_mode == 1 ? 1.0e8f : 4.0f;
+    int4 head = __ldg(reinterpret_cast<const int4*>(&r->zf_re));
+    const float bound = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * (1.0f - 0x1p-14f);
+    const float far = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * 16.0f;
+    Sc total = sc_make(z.x + d.re, z.y + d.im, 0);  // kept with planes only
     Sc prior = sc_zero();
     int k = 0;
     bool pending = false;
 #pragma unroll 1
     while (k < room) {
-        if (!(flags & kRawOrbit) || !raw_part(d.re) || !raw_part(d.im)) break;
-        if (blocks && !no_block(p, first + k - p.alt_start, d)) break;
-        const double2 zn = __ldg(reinterpret_cast<const double2*>(r + 1));
-        const float4 head = __ldg(reinterpret_cast<const float4*>(&r[1].zf_re));
+        const int flags = head.z;
+        if (!(flags & kRawOrbit)) break;
+        const int dr = high(d.re), di = high(d.im);
+        const int most = imax(dr, di), top = most >> 20;
+        bool plain = imin(dr, di) >= kHighLow && most <= kHighTop && 2 * (top - 1023) >= block_top
+            && static_cast<unsigned>(head.w + 1 - top + 55) <= 110u;
+        if constexpr (WithPlanes) {
+            const int a = high(j.xa), b = high(j.xb), c = high(j.ya), e = high(j.yb);
+            plain = plain && imin(imin(a, b), imin(c, e)) >= kHighLow && imax(imax(a, b), imax(c, e)) <= kHighJac
+                && imin(high(total.re), high(total.im)) >= kHighLow;
+            if constexpr (Formula != kFormulaJulia) plain = plain && static_cast<unsigned>(j.k + 400) <= 1000u;
+        }
+        bool with_pd = true;
+        if constexpr (Formula == kFormulaTricorn) {
+            // d^2 and pd: near enough to add, or pd dropped.
+            const int apart = 2 * top - 1023 - pd_top;
+            with_pd = apart < 60;
+            plain = plain && (apart > 65 || static_cast<unsigned>(apart + 55) <= 110u);
+        }
         bool fold = false;
         double2 constant{0.0, 0.0};
-        Sc total = sc_zero();
         if constexpr (Formula == kFormulaBurningShip) {
             fold = folds(z.x, d.re) || folds(z.y, d.im);
             if (fold) {
                 if (!(flags & kRawFold)) break;
                 constant = make_double2(__ldg(&r->fold[0]), __ldg(&r->fold[1]));
             }
-            total = sc_make(z.x + d.re, z.y + d.im, 0);
+            if (!WithPlanes) total = sc_make(z.x + d.re, z.y + d.im, 0);
         }
-        if constexpr (WithPlanes) {
-            if constexpr (Formula == kFormulaBurningShip) {
-                // add_cut with its sums at hand
-                const int diff = imax(bexp(z.x), bexp(z.y)) - imax(bexp(d.re), bexp(d.im));
-                prior = diff > 60 ? sc_make(z.x, z.y, 0) : (diff < -60 ? d : total);
-            } else {
-                prior = add_cut(sc_make(z.x, z.y, 0), d);
+        const double2 zn = __ldg(reinterpret_cast<const double2*>(r + 1));
+        head = __ldg(reinterpret_cast<const int4*>(&r[1].zf_re));
+        if (plain) {
+            if constexpr (WithPlanes) {
+                prior = total;
+                const double tr = add_exp(total.re, 1), ti = add_exp(total.im, 1);
+                int sign = Formula == kFormulaTricorn ? static_cast<int>(0x80000000u) : 0;
+                if constexpr (Formula == kFormulaBurningShip) {
+                    sign = (hi_of(tr) ^ hi_of(ti)) & static_cast<int>(0x80000000u);
+                }
+                double xa = tr * j.xa - ti * j.ya, yb = ti * j.xb + tr * j.yb;
+                const double xb = tr * j.xb - ti * j.yb, ya = ti * j.xa + tr * j.ya;
+                yb = from_hilo(hi_of(yb) ^ sign, lo_of(yb));
+                if constexpr (Formula != kFormulaJulia) {
+                    const double one = from_hilo((1023 - j.k) << 20, 0);
+                    xa = xa + one;
+                    yb = yb + one;
+                }
+                j.xa = xa;
+                j.xb = xb;
+                j.ya = from_hilo(hi_of(ya) ^ sign, lo_of(ya));
+                j.yb = yb;
             }
-            if (!jac_step_raw<Formula>(prior, j)) break;
+            const double z2r = add_exp(z.x, 1), z2i = add_exp(z.y, 1);
+            const double lr = z2r * d.re - z2i * d.im, li = z2r * d.im + z2i * d.re;
+            if constexpr (Formula == kFormulaBurningShip) {
+                const double u = choose(fold, total.re, d.re), v = choose(fold, total.im, d.im);
+                const double sr = u * u - v * v, si = twice_raw(u * v);
+                const bool flipped = !fold && (hi_of(z.x) ^ hi_of(z.y)) < 0;
+                const double xr = choose(fold, constant.x, lr) + choose(fold, pd.re, sr);
+                const double xi = choose(fold, constant.y, li) + choose(fold, pd.im, si);
+                d.re = xr + choose(fold, sr, pd.re);
+                d.im = flip(xi, flipped) + choose(fold, fabs_(si), pd.im);
+            } else {
+                const double sr = d.re * d.re - d.im * d.im;
+                double si = add_exp(d.re * d.im, 1);
+                if constexpr (Formula == kFormulaTricorn) {
+                    si = neg_(si);
+                    if (with_pd) {
+                        // This sum may cancel, so the outer one is checked.
+                        d = add_cut(sc_make(lr, neg_(li), 0), sc_make(sr + pd.re, si + pd.im, 0));
+                    } else {
+                        d.re = lr + sr;
+                        d.im = si - li;
+                    }
+                } else {
+                    d.re = lr + sr;
+                    d.im = li + si;
+                }
+            }
+        } else {
+            if (!raw_or_zero(d.re) || !raw_or_zero(d.im)) break;
+            if (blocks && !no_block(p, first + k - p.alt_start, d)) break;
+            if constexpr (WithPlanes) {
+                prior = add_cut(sc_make(z.x, z.y, 0), d);
+                if (!jac_step_raw<Formula>(prior, j)) break;
+            }
+            d = alt_step_raw<Formula>(z, d, pd, fold, total, constant);
         }
-        d = alt_step_raw<Formula>(z, d, pd, fold, total, constant);
         ++k;
         ++r;
         z = zn;
-        flags = __float_as_int(head.z);
-        // alt_inside at the new index.
-        const float dx = float_of(d.re, 0), dy = float_of(d.im, 0);
-        const float tx = head.x + dx, ty = head.y + dy;
+        // alt_inside at the new index: with planes from the total, which the
+        // next step reads; else from FP32 estimates of both terms.
+        bool inside;
+        if constexpr (WithPlanes) {
+            total = sc_make(z.x + d.re, z.y + d.im, 0);
+            inside = square_estimate(total.re) + square_estimate(total.im) < bound;
+        } else {
+            const float dx = float_of(d.re, 0), dy = float_of(d.im, 0);
+            const float tx = __int_as_float(head.x) + dx, ty = __int_as_float(head.y) + dy;
+            inside = tx * tx + ty * ty < bound && dx * dx + dy * dy < far;
+        }
         const int it = s.it + k;
-        if (!(tx * tx + ty * ty < r2 * (1.0f - 0x1p-14f) && dx * dx + dy * dy < r2 * 16.0f)
-            || (it >= cycle_from && (it & 31) == 0)) {
+        if (!inside || (it >= cycle_from && (it & 31) == 0)) {
             pending = true;
             break;
         }
@@ -800,20 +931,20 @@ __device__ __forceinline__ unsigned long long alt_deadline(const AltParams& p) {
 // A pixel still running after its launch's budget of rounds is spilled with
 // its whole state to a list that the next launch takes as its input, so the
 // few long orbits (1 % of a Julia view, up to the cap) run 32 to a warp
-// instead of one in each.  The budgets grow by four; the last launch has
-// none, and a pixel that finds the list full runs on where it is.
+// instead of one in each.  The budgets double; the last launch has none,
+// and a pixel that finds the list full runs on where it is.
 constexpr int kAltRefill = 8;
-constexpr int kAltPhases = 5;
+constexpr int kAltPhases = 8;
 constexpr int kAltFirstBudget = 32;          // rounds: 512 steps
 constexpr long long kAltPhasePixels = 16384; // smaller fields run in one launch
 
 template <bool WithPlanes, int Formula>
 __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ AltParams p, unsigned long long* claim,
-                                                        const AltLane<WithPlanes>* source,
+                                                        const AltSaved* source,
                                                         const unsigned long long* source_count,
-                                                        AltLane<WithPlanes>* spill, unsigned long long* spill_count,
+                                                        AltSaved* spill, unsigned long long* spill_count,
                                                         unsigned long long spill_capacity, int budget,
-                                                        AltLane<WithPlanes>* ready_lists) {
+                                                        AltSaved* ready_lists) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ AltEnd<WithPlanes> parks[4][kAltPark];
     AltEnd<WithPlanes>* park = parks[threadIdx.x >> 5];
@@ -833,7 +964,7 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
     bool drained = false;
     int parked = 0;
     int ready = 0;  // pixels on the warp's list
-    AltLane<WithPlanes>* list = ready_lists + static_cast<std::size_t>(blockIdx.x * 4 + (threadIdx.x >> 5)) * kAltPark;
+    AltSaved* list = ready_lists + static_cast<std::size_t>(blockIdx.x * 4 + (threadIdx.x >> 5)) * kAltPark;
     // Park the escaped among the warp's lanes `l`; finish 32 when they are there.
     const auto park_escaped = [&](bool escaped, const AltLane<WithPlanes>& l) {
         const unsigned ended = __ballot_sync(kFull, escaped);
@@ -868,8 +999,7 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
                 if (lane == 0) base = atomicAdd(claim, static_cast<unsigned long long>(n));
                 base = __shfl_sync(kFull, base, 0);
                 if (!have && base + rank < items) {
-                    s = source[base + rank];
-                    s.rounds = 0;
+                    alt_restore<WithPlanes, Formula>(p, source[base + rank], s);
                     have = true;
                 }
                 drained = base + n >= items;
@@ -891,12 +1021,12 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
                     __syncwarp();
                     park_escaped(started == kAltEscaped, t);
                     const unsigned kept = __ballot_sync(kFull, started == kAltContinue);
-                    if (started == kAltContinue) list[ready + __popc(kept & below)] = t;
+                    if (started == kAltContinue) alt_save(t, list[ready + __popc(kept & below)]);
                     ready += __popc(kept);
                     __syncwarp();
                 }
                 if (!have && rank < ready) {
-                    s = list[ready - 1 - rank];
+                    alt_restore<WithPlanes, Formula>(p, list[ready - 1 - rank], s);
                     have = true;
                 }
                 ready -= n < ready ? n : ready;
@@ -927,7 +1057,7 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
         park_escaped(outcome == kAltEscaped, s);
         if (outcome != kAltContinue) have = false;
         if (budget > 0) {
-            const bool over = have && !wait && !keep && s.rounds >= budget;
+            const bool over = have && !wait && !keep && s.rounds >= budget && !s.ready;
             const unsigned mask = __ballot_sync(kFull, over);
             if (mask != 0u) {
                 unsigned long long base = 0;
@@ -936,7 +1066,7 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
                 const unsigned long long slot = base + static_cast<unsigned>(__popc(mask & below));
                 if (over) {
                     if (slot < spill_capacity) {
-                        spill[slot] = s;
+                        alt_save(s, spill[slot]);
                         have = false;
                     } else {
                         keep = true;
@@ -966,14 +1096,18 @@ int alt_queue_blocks() {
 template <bool WithPlanes, int Formula>
 cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t stream) {
     const long long pixels = static_cast<long long>(p.width) * p.height;
-    const int phases = pixels > kAltPhasePixels && queue.spill != nullptr && queue.capacity > 0 ? kAltPhases : 1;
+    int phases = 1;
+    if (pixels > kAltPhasePixels && queue.spill != nullptr && queue.capacity > 0) {
+        long long steps = static_cast<long long>(kAltFirstBudget) * kAltRound;
+        for (; phases < kAltPhases && steps < p.max_iter; ++phases) steps *= 2;
+    }
     const cudaError_t cleared =
         cudaMemsetAsync(queue.counters, 0, sizeof(unsigned long long) * kAltQueueCounters, stream);
     if (cleared != cudaSuccess) return cleared;
-    auto* lists = static_cast<AltLane<WithPlanes>*>(queue.spill);
+    auto* lists = static_cast<AltSaved*>(queue.spill);
     const long long resident = alt_queue_blocks<WithPlanes, Formula>();
     int budget = kAltFirstBudget;
-    for (int phase = 0; phase < phases; ++phase, budget *= 4) {
+    for (int phase = 0; phase < phases; ++phase, budget *= 2) {
         // A field (or a full list) smaller than the persistent grid needs no
         // more warps than items / 32.
         const long long items = phase == 0 ? pixels : std::min<long long>(queue.capacity, pixels);
@@ -982,14 +1116,14 @@ cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t s
             p, queue.counters + phase, phase == 0 ? nullptr : lists + ((phase - 1) & 1) * queue.capacity,
             phase == 0 ? nullptr : queue.counters + kAltPhases + phase - 1, lists + (phase & 1) * queue.capacity,
             queue.counters + kAltPhases + phase, static_cast<unsigned long long>(queue.capacity),
-            phase + 1 < phases ? budget : 0, static_cast<AltLane<WithPlanes>*>(queue.ready));
+            phase + 1 < phases ? budget : 0, static_cast<AltSaved*>(queue.ready));
     }
     return cudaGetLastError();
 }
 
 }  // namespace
 
-std::size_t alt_spill_entry_bytes() { return sizeof(AltLane<true>); }
+std::size_t alt_spill_entry_bytes() { return sizeof(AltSaved); }
 
 // One list of kAltPark pixels per warp of the largest grid.
 std::size_t alt_ready_bytes() {
@@ -997,7 +1131,7 @@ std::size_t alt_ready_bytes() {
                                  alt_queue_blocks<true, kFormulaBurningShip>(),
                                  alt_queue_blocks<false, kFormulaBurningShip>(),
                                  alt_queue_blocks<true, kFormulaTricorn>(), alt_queue_blocks<false, kFormulaTricorn>()});
-    return static_cast<std::size_t>(blocks) * 4 * kAltPark * sizeof(AltLane<true>);
+    return static_cast<std::size_t>(blocks) * 4 * kAltPark * sizeof(AltSaved);
 }
 
 cudaError_t launch_plain_alternate(const AltParams& p, bool planes, const AltQueue& queue, cudaStream_t stream) {
