@@ -329,14 +329,13 @@ void launch_deep_mandelbrot(ReferenceContext& ctx, DeviceTables& dev, const Outp
     p.stats = collect_stats ? rt.stats : nullptr;
     p.points = points ? points->points : nullptr;
     p.exact_flags = points ? points->exact_flags : nullptr;
-    check_cuda(launch_plain_mandelbrot(p, out.p_iter != nullptr, collect_stats, stream),
+    check_cuda(launch_plain_mandelbrot(p, out.p_dex != nullptr, collect_stats, stream),
                "plain Mandelbrot kernel launch");
 }
 
 // Counters and spill lists of the alternate-formula queue: one slot per lane
 // stream of a batch, and one (the last) for single renders.  A list holds up
-// to 524,288 pixels of 128 bytes (the ones of a field that outlast a launch's
-// budget: 10 % of a Julia view; beyond that they run on where they are).
+// to 262,144 pixels of 128 bytes: more than the lanes of a launch.
 constexpr int kAltQueueSlots = ThreadRuntime::kPlainLanes + 1;
 constexpr std::size_t kAltQueueStride = 256;
 static_assert(kAltQueueCounters * sizeof(unsigned long long) <= kAltQueueStride, "one slot");
@@ -352,7 +351,7 @@ struct AltQueues {
 AltQueues alt_queues(ThreadRuntime& rt, long long pixels, int slots) {
     AltQueues q;
     q.counters = static_cast<char*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * kAltQueueStride));
-    q.capacity = std::min<long long>(pixels, 1ll << 19);
+    q.capacity = std::min<long long>(pixels, 1ll << 18);
     q.slot_bytes = 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes() + alt_ready_bytes();
     q.slot_bytes = (q.slot_bytes + 255) / 256 * 256;
     q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill, slots * q.slot_bytes));
@@ -423,7 +422,7 @@ void launch_deep_alternate(ReferenceContext& ctx, DeviceTables& dev, const Outpu
     }
     const AltQueue slot = queue ? *queue
         : alt_queue_slot(alt_queues(rt, static_cast<long long>(width) * height, 1), kAltQueueSlots - 1, 0);
-    check_cuda(launch_plain_alternate(p, out.p_iter != nullptr, slot, stream), "plain alternate-formula kernel launch");
+    check_cuda(launch_plain_alternate(p, out.p_dex != nullptr, slot, stream), "plain alternate-formula kernel launch");
 }
 
 // Spill-list entries for a direct batch of `pixels` pixels: enough for the
@@ -1630,8 +1629,6 @@ void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRunti
     // it there, so the FP64 and FP32 pipes work at once.  Two or more
     // plain-form launches are dealt over the lane streams instead (all forked
     // from and joined back to the caller's stream), so their tails overlap.
-    // Fields that asked for derivative planes only share one discard region
-    // for the planes nobody reads; concurrent lanes may write it in any order.
     const int lanes = plain_lanes(plan);
     const bool fork = (!plan.direct.empty() && (!plan.floatexp.empty() || !plan.plain.empty()))
         || (!plan.plain.empty() && !plan.floatexp.empty());
@@ -1954,9 +1951,6 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
     std::size_t direct_doubles = 0;
     bool centre_parsed = false;
     long double cx = 0.0L, cy = 0.0L;
-    // Planes no caller asked for but the plain kernels write (they take all
-    // six or none): one shared discard region sized for the largest field.
-    long long plane_pixels = 0;
     for (std::size_t i = 0; i < fields.size(); ++i) {
         const FieldRequest& f = fields[i];
         if (!f.out.field || !f.zoom_text || !valid_iterations(f.max_iter) || !valid_dims(f.width, f.height)) {
@@ -1965,28 +1959,7 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
         if ((f.flags & ~FRACTAL_GB300_KEYFRAME_SHALLOW) != 0) {
             throw Failure{"invalid native keyframe " + std::to_string(i) + " flags"};
         }
-        if (f.out.p_dex) plane_pixels = std::max(plane_pixels, static_cast<long long>(f.width) * f.height);
     }
-    Outputs discard;
-    if (plane_pixels > 0) {
-        auto* base = static_cast<char*>(scratch(rt, kScratchDiscard, static_cast<std::size_t>(plane_pixels) * 32));
-        discard.p_iter = reinterpret_cast<std::int64_t*>(base);
-        discard.p_phase = reinterpret_cast<double*>(base + plane_pixels * 8);
-        discard.p_t1 = reinterpret_cast<double*>(base + plane_pixels * 16);
-        discard.p_t2 = reinterpret_cast<double*>(base + plane_pixels * 24);
-    }
-    // All six planes for the plain kernels: the caller's derivative planes,
-    // the rest into the discard region.
-    auto plain_outputs = [&](const Outputs& out) {
-        Outputs full = out;
-        if (out.p_dex) {
-            full.p_iter = discard.p_iter;
-            full.p_phase = discard.p_phase;
-            full.p_t1 = discard.p_t1;
-            full.p_t2 = discard.p_t2;
-        }
-        return full;
-    };
     auto direct_group = [](int formula, const Outputs& out) { return formula | (out.p_dex ? 0x100 : 0); };
     for (std::size_t i = 0; i < fields.size(); ++i) {
         const FieldRequest& frame = fields[i];
@@ -1999,7 +1972,7 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
                 cy = parse_coordinate(y_center, "imaginary");
                 centre_parsed = true;
             }
-            const Outputs out = plain_outputs(frame.out);
+            const Outputs& out = frame.out;
             auto& group = plan.direct[direct_group(kFormulaMandelbrot, out)];
             group.push_back(make_direct_params(out, width, height, parse_zoom_direct(frame.zoom_text), cx, cy,
                                                frame.max_iter, kFormulaMandelbrot, 0.0, 0.0, o));
@@ -2031,7 +2004,7 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
             continue;
         }
         const fx::Fe zoom = parse_zoom_fe(frame.zoom_text, ctx->precision_bits);
-        const Outputs out = plain_outputs(frame.out);
+        const Outputs& out = frame.out;
         if (fe_log10(zoom) < 6.0L || direct_path) {
             auto& group = plan.direct[direct_group(ctx->formula, out)];
             group.push_back(make_direct_params(out, width, height, parse_zoom_direct(frame.zoom_text), ctx->x_center,

@@ -10,6 +10,7 @@
 // step once the reference orbit ends, and the Jacobian carried for the
 // analytic-DE plane.  Compiled with --fmad=false like the Mandelbrot plain
 // form, so results match the reference release build bit for bit.
+#define FX_OUTLINE 1
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -17,6 +18,7 @@
 #include <type_traits>
 
 #include "device.h"
+#include "int_mul.h"
 
 namespace fgb {
 namespace {
@@ -125,15 +127,28 @@ __device__ bool de_matrix(const Sc& total, const Jac& j, const Fe& spacing, doub
     return is_finite(ox) && is_finite(oy);
 }
 
+// Render planes: the derivative pair, and the other four or none (a batch
+// asks for the pair only).
 struct Planes {
     std::int64_t* iter;
     double *phase, *dex, *dey, *t1, *t2;
     __device__ void clear(long long i, int max_iter) const {
+        dex[i] = dey[i] = 0.0;
+        if (iter == nullptr) return;
         iter[i] = max_iter;
-        phase[i] = dex[i] = dey[i] = t1[i] = t2[i] = 0.0;
+        phase[i] = t1[i] = t2[i] = 0.0;
     }
     __device__ void escape(long long i, int raw, const Sc& total, const Nrm& test2, const Jac& j,
                            const Fe& spacing) const {
+        double ox = 0.0, oy = 0.0;
+        if (de_matrix(total, j, spacing, ox, oy)) {
+            dex[i] = ox;
+            dey[i] = oy;
+        } else {
+            dex[i] = 0.0;
+            dey[i] = 0.0;
+        }
+        if (iter == nullptr) return;
         iter[i] = raw;
         const double re = sc_re_d(total), im = sc_im_d(total);
         double ph = 0.0;
@@ -143,14 +158,6 @@ struct Planes {
             if (!is_finite(ph)) ph = 0.0;
         }
         phase[i] = ph;
-        double ox = 0.0, oy = 0.0;
-        if (de_matrix(total, j, spacing, ox, oy)) {
-            dex[i] = ox;
-            dey[i] = oy;
-        } else {
-            dex[i] = 0.0;
-            dey[i] = 0.0;
-        }
         t1[i] = nrm_to_d(sc_norm2(total));
         t2[i] = nrm_to_d(test2);
     }
@@ -428,7 +435,6 @@ struct AltLane {
     Nrm norm;   // escape norm of a pixel that has escaped
     Jac jac;
     int ref, it, power, length, hits;
-    int rounds; // rounds run in this launch
     unsigned ticks;
     bool ready, past, pending;
 };
@@ -531,7 +537,6 @@ __device__ __forceinline__ void alt_reset(AltLane<WithPlanes>& s, const Sc& dc) 
     s.power = 1;
     s.length = 0;
     s.hits = 0;
-    s.rounds = 0;
 }
 
 template <bool WithPlanes, int Formula>
@@ -668,59 +673,96 @@ __device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlane
                 if (!(flags & kRawFold)) break;
                 constant = make_double2(__ldg(&r->fold[0]), __ldg(&r->fold[1]));
             }
-            if (!WithPlanes) total = sc_make(z.x + d.re, z.y + d.im, 0);
+            if (!WithPlanes && fold) total = sc_make(z.x + d.re, z.y + d.im, 0);
+            plain = plain && (!fold || imin(high(total.re), high(total.im)) >= kHighLow);
         }
         const double2 zn = __ldg(reinterpret_cast<const double2*>(r + 1));
         head = __ldg(reinterpret_cast<const int4*>(&r[1].zf_re));
         if (plain) {
+            // Products on the integer pipe, sums in FP64 beside them
+            // (int_mul.h).
+            const double z2r = add_exp(z.x, 1), z2i = add_exp(z.y, 1);
+            std::uint32_t low = ~0u;
+            RawJac nj = j;
+            Sc nd = d;
             if constexpr (WithPlanes) {
-                prior = total;
                 const double tr = add_exp(total.re, 1), ti = add_exp(total.im, 1);
+                const FactorA fr = factor_a(tr), fi = factor_a(ti);
+                const FactorB fxa = factor_b(j.xa), fya = factor_b(j.ya);
+                const double rxa = int_mul(fr, fxa, low), iya = int_mul(fi, fya, low);
+                const double ixa = int_mul(fi, fxa, low), rya = int_mul(fr, fya, low);
+                const FactorB fxb = factor_b(j.xb), fyb = factor_b(j.yb);
+                const double rxb = int_mul(fr, fxb, low), iyb = int_mul(fi, fyb, low);
+                const double ixb = int_mul(fi, fxb, low), ryb = int_mul(fr, fyb, low);
                 int sign = Formula == kFormulaTricorn ? static_cast<int>(0x80000000u) : 0;
                 if constexpr (Formula == kFormulaBurningShip) {
                     sign = (hi_of(tr) ^ hi_of(ti)) & static_cast<int>(0x80000000u);
                 }
-                double xa = tr * j.xa - ti * j.ya, yb = ti * j.xb + tr * j.yb;
-                const double xb = tr * j.xb - ti * j.yb, ya = ti * j.xa + tr * j.ya;
+                double xa = rxa - iya, yb = ixb + ryb;
+                const double xb = rxb - iyb, ya = ixa + rya;
                 yb = from_hilo(hi_of(yb) ^ sign, lo_of(yb));
                 if constexpr (Formula != kFormulaJulia) {
-                    const double one = from_hilo((1023 - j.k) << 20, 0);
-                    xa = xa + one;
-                    yb = yb + one;
+                    // The +1, 2^-k here, does not move a sum 60 binades above it.
+                    if (imin(bexp(xa), bexp(yb)) <= 1023 - j.k + 60) {
+                        const double one = from_hilo((1023 - j.k) << 20, 0);
+                        xa = xa + one;
+                        yb = yb + one;
+                    }
                 }
-                j.xa = xa;
-                j.xb = xb;
-                j.ya = from_hilo(hi_of(ya) ^ sign, lo_of(ya));
-                j.yb = yb;
+                nj.xa = xa;
+                nj.xb = xb;
+                nj.ya = from_hilo(hi_of(ya) ^ sign, lo_of(ya));
+                nj.yb = yb;
             }
-            const double z2r = add_exp(z.x, 1), z2i = add_exp(z.y, 1);
-            const double lr = z2r * d.re - z2i * d.im, li = z2r * d.im + z2i * d.re;
+            const FactorA fr = factor_a(d.re), fi = factor_a(d.im);
+            const FactorB gr = factor_b(z2r), gi = factor_b(z2i);
+            const double rr = int_mul(fr, gr, low), ii = int_mul(fi, gi, low);
+            const double ri = int_mul(fi, gr, low), ir = int_mul(fr, gi, low);
             if constexpr (Formula == kFormulaBurningShip) {
                 const double u = choose(fold, total.re, d.re), v = choose(fold, total.im, d.im);
-                const double sr = u * u - v * v, si = twice_raw(u * v);
+                const FactorA eu = factor_a(u), ev = factor_a(v);
+                const FactorB hu = factor_b(u), hv = factor_b(v);
+                const double uu = int_mul(eu, hu, low), vv = int_mul(ev, hv, low), uv = int_mul(eu, hv, low);
+                const double lr = rr - ii, li = ri + ir;
+                const double sr = uu - vv, si = add_exp(uv, 1);
                 const bool flipped = !fold && (hi_of(z.x) ^ hi_of(z.y)) < 0;
-                const double xr = choose(fold, constant.x, lr) + choose(fold, pd.re, sr);
-                const double xi = choose(fold, constant.y, li) + choose(fold, pd.im, si);
-                d.re = xr + choose(fold, sr, pd.re);
-                d.im = flip(xi, flipped) + choose(fold, fabs_(si), pd.im);
+                double xr = choose(fold, constant.x, lr) + choose(fold, pd.re, sr);
+                double xi = choose(fold, constant.y, li) + choose(fold, pd.im, si);
+                xi = flip(xi, flipped);
+                // pd does not move a sum 60 binades above it.
+                if (fold || imin(bexp(xr), bexp(xi)) <= pd_top + 60) {
+                    xr = xr + choose(fold, sr, pd.re);
+                    xi = xi + choose(fold, fabs_(si), pd.im);
+                }
+                nd.re = xr;
+                nd.im = xi;
             } else {
-                const double sr = d.re * d.re - d.im * d.im;
-                double si = add_exp(d.re * d.im, 1);
+                const FactorB hr = factor_b(d.re), hi = factor_b(d.im);
+                const double uu = int_mul(fr, hr, low), vv = int_mul(fi, hi, low), uv = int_mul(fr, hi, low);
+                const double lr = rr - ii, li = ri + ir;
+                const double sr = uu - vv, si = add_exp(uv, 1);
                 if constexpr (Formula == kFormulaTricorn) {
-                    si = neg_(si);
                     if (with_pd) {
                         // This sum may cancel, so the outer one is checked.
-                        d = add_cut(sc_make(lr, neg_(li), 0), sc_make(sr + pd.re, si + pd.im, 0));
+                        nd = add_cut(sc_make(lr, neg_(li), 0), sc_make(sr + pd.re, pd.im - si, 0));
                     } else {
-                        d.re = lr + sr;
-                        d.im = si - li;
+                        nd.re = lr + sr;
+                        nd.im = neg_(li + si);
                     }
                 } else {
-                    d.re = lr + sr;
-                    d.im = li + si;
+                    nd.re = lr + sr;
+                    nd.im = li + si;
                 }
             }
-        } else {
+            // A product that may be a tie: the longer form multiplies in FP64.
+            plain = low != 0u;
+            if (plain) {
+                if constexpr (WithPlanes) prior = total;
+                j = nj;
+                d = nd;
+            }
+        }
+        if (!plain) {
             if (!raw_or_zero(d.re) || !raw_or_zero(d.im)) break;
             if (blocks && !no_block(p, first + k - p.alt_start, d)) break;
             if constexpr (WithPlanes) {
@@ -928,22 +970,33 @@ __device__ __forceinline__ unsigned long long alt_deadline(const AltParams& p) {
 // of ready pixels.  Run by the lanes just refilled, the starts and blocks
 // took 80 % of the instructions.
 //
-// A pixel still running after its launch's budget of rounds is spilled with
-// its whole state to a list that the next launch takes as its input, so the
-// few long orbits (1 % of a Julia view, up to the cap) run 32 to a warp
-// instead of one in each.  The budgets double; the last launch has none,
-// and a pixel that finds the list full runs on where it is.
+// Once no pixel is left to take, a warp that has run kAltPatience rounds with
+// fewer than kAltLeave active lanes leaves: it spills them to a list that the next launch takes as
+// its input, so the few long orbits (10 % of a Julia view past 500 steps, 1 %
+// to the cap) run 32 to a warp instead of one in each.  Lifetimes are
+// close to exponential whatever their scale, so a rule on lanes suits every
+// view where a budget of steps suits one; the patience lets pixels that all
+// end soon end where they are (a burning-ship view's, 8.4 ms without it and
+// 5.8 ms with it).  A list short enough to give every
+// SM sub-partition one warp gains nothing from another launch and runs to its end.
 constexpr int kAltRefill = 8;
 constexpr int kAltPhases = 8;
-constexpr int kAltFirstBudget = 32;          // rounds: 512 steps
+constexpr int kAltLeave = 20;
+constexpr int kAltPatience = 24;  // rounds: 384 steps
+constexpr int kAltShort = 32 * 4 * 152;      // pixels: one full warp per SM sub-partition
+constexpr int kAltBusyWarps = 8 * 152;       // warps that keep the FP64 pipe busy
 constexpr long long kAltPhasePixels = 16384; // smaller fields run in one launch
 
+// Registers: the parameter-plane formulas, whose general turns wait for
+// instructions, gain from four blocks (1280x720 with planes: 10.0 against
+// 10.6 ms); the long Julia orbits of the last launch from none spilled
+// (43.8 against 49.1 ms).
 template <bool WithPlanes, int Formula>
-__global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ AltParams p, unsigned long long* claim,
+__global__ void __launch_bounds__(128, Formula == kFormulaJulia ? 3 : 4) alt_queue_kernel(const __grid_constant__ AltParams p, unsigned long long* claim,
                                                         const AltSaved* source,
                                                         const unsigned long long* source_count,
                                                         AltSaved* spill, unsigned long long* spill_count,
-                                                        unsigned long long spill_capacity, int budget,
+                                                        unsigned long long spill_capacity, int leave,
                                                         AltSaved* ready_lists) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ AltEnd<WithPlanes> parks[4][kAltPark];
@@ -954,16 +1007,22 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
     if (source != nullptr) {
         items = *source_count;
         if (items > spill_capacity) items = spill_capacity;
+        // Warps beyond the busy ones (taken round the blocks) do not start.
+        const unsigned long long rank = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        const unsigned long long warps = (items + 31) / 32;
+        if (rank >= (warps < kAltBusyWarps ? warps : static_cast<unsigned long long>(kAltBusyWarps))) return;
+        if (items <= kAltShort) leave = 0;
     }
     const unsigned long long deadline = alt_deadline(p);
     const int max_block = alt_max_block(p);
     AltLane<WithPlanes> s;
     bool have = false;
-    bool keep = false;  // the spill list was full: run on
+    bool keep = false;  // the list was full: run on
     bool wait = false;  // the lane's pixel needs a general turn
     bool drained = false;
     int parked = 0;
     int ready = 0;  // pixels on the warp's list
+    int lean = 0;   // rounds with few lanes
     AltSaved* list = ready_lists + static_cast<std::size_t>(blockIdx.x * 4 + (threadIdx.x >> 5)) * kAltPark;
     // Park the escaped among the warp's lanes `l`; finish 32 when they are there.
     const auto park_escaped = [&](bool escaped, const AltLane<WithPlanes>& l) {
@@ -1043,7 +1102,6 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
         }
         if (have && !wait) {
             wait = alt_raw_run<WithPlanes, Formula>(p, s, kAltRound) < kAltRound || s.pending;
-            ++s.rounds;
         }
         const int waiting = __popc(__ballot_sync(kFull, have && wait));
         if (waiting >= kAltRefill || !__any_sync(kFull, have && !wait)) {
@@ -1056,15 +1114,16 @@ __global__ void __launch_bounds__(128) alt_queue_kernel(const __grid_constant__ 
         }
         park_escaped(outcome == kAltEscaped, s);
         if (outcome != kAltContinue) have = false;
-        if (budget > 0) {
-            const bool over = have && !wait && !keep && s.rounds >= budget && !s.ready;
-            const unsigned mask = __ballot_sync(kFull, over);
-            if (mask != 0u) {
+        if (leave > 0 && drained && ready == 0) {
+            const unsigned left = __ballot_sync(kFull, have);
+            const unsigned mask = __ballot_sync(kFull, have && !wait && !keep && !s.ready);
+            if (__popc(left) < leave) ++lean;
+            if (lean > kAltPatience && mask != 0u) {
                 unsigned long long base = 0;
                 if (lane == 0) base = atomicAdd(spill_count, static_cast<unsigned long long>(__popc(mask)));
                 base = __shfl_sync(kFull, base, 0);
                 const unsigned long long slot = base + static_cast<unsigned>(__popc(mask & below));
-                if (over) {
+                if ((mask >> lane) & 1u) {
                     if (slot < spill_capacity) {
                         alt_save(s, spill[slot]);
                         have = false;
@@ -1096,27 +1155,22 @@ int alt_queue_blocks() {
 template <bool WithPlanes, int Formula>
 cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t stream) {
     const long long pixels = static_cast<long long>(p.width) * p.height;
-    int phases = 1;
-    if (pixels > kAltPhasePixels && queue.spill != nullptr && queue.capacity > 0) {
-        long long steps = static_cast<long long>(kAltFirstBudget) * kAltRound;
-        for (; phases < kAltPhases && steps < p.max_iter; ++phases) steps *= 2;
-    }
+    const int phases = pixels > kAltPhasePixels && queue.spill != nullptr && queue.capacity > 0 ? kAltPhases : 1;
     const cudaError_t cleared =
         cudaMemsetAsync(queue.counters, 0, sizeof(unsigned long long) * kAltQueueCounters, stream);
     if (cleared != cudaSuccess) return cleared;
     auto* lists = static_cast<AltSaved*>(queue.spill);
     const long long resident = alt_queue_blocks<WithPlanes, Formula>();
-    int budget = kAltFirstBudget;
-    for (int phase = 0; phase < phases; ++phase, budget *= 2) {
-        // A field (or a full list) smaller than the persistent grid needs no
-        // more warps than items / 32.
-        const long long items = phase == 0 ? pixels : std::min<long long>(queue.capacity, pixels);
-        const unsigned grid = static_cast<unsigned>(std::min<long long>(resident, (items + 127) / 128));
+    for (int phase = 0; phase < phases; ++phase) {
+        // A field smaller than the persistent grid needs no more warps than
+        // pixels / 32.
+        const long long blocks = phase == 0 ? resident : std::min<long long>(resident, kAltBusyWarps / 4);
+        const unsigned grid = static_cast<unsigned>(std::min<long long>(blocks, (pixels + 127) / 128));
         alt_queue_kernel<WithPlanes, Formula><<<grid, 128, 0, stream>>>(
             p, queue.counters + phase, phase == 0 ? nullptr : lists + ((phase - 1) & 1) * queue.capacity,
             phase == 0 ? nullptr : queue.counters + kAltPhases + phase - 1, lists + (phase & 1) * queue.capacity,
             queue.counters + kAltPhases + phase, static_cast<unsigned long long>(queue.capacity),
-            phase + 1 < phases ? budget : 0, static_cast<AltSaved*>(queue.ready));
+            phase + 1 < phases ? kAltLeave : 0, static_cast<AltSaved*>(queue.ready));
     }
     return cudaGetLastError();
 }

@@ -169,10 +169,11 @@ __device__ void write_inside(const DirectParams& p, int local) {
     p.out[local] = static_cast<float>(static_cast<double>(p.max_iter) - p.output_bias);
     if (p.counts) p.counts[local] = static_cast<std::uint32_t>(p.max_iter);
     if constexpr (Planes) {
-        p.p_iter[local] = p.max_iter;
-        p.p_phase[local] = 0.0;
         p.p_dex[local] = 0.0;
         p.p_dey[local] = 0.0;
+        if (p.p_iter == nullptr) return;  // the derivative pair alone
+        p.p_iter[local] = p.max_iter;
+        p.p_phase[local] = 0.0;
         p.p_t1[local] = 0.0;
         p.p_t2[local] = 0.0;
     }
@@ -192,13 +193,6 @@ __device__ void write_escape_planes(const DirectParams& p, const Lane& l, double
     const int local = l.local;
     p.out[local] = smooth_value(p, l.it, m2);
     if (p.counts) p.counts[local] = static_cast<std::uint32_t>(l.it + 1);
-    p.p_iter[local] = l.it;
-    double phase = 0.0;
-    if (p.need_phase && is_finite(l.zr) && is_finite(l.zi)) {
-        phase = atan2(l.zi, l.zr) / kTwoPi;
-        phase -= floor(phase);
-    }
-    p.p_phase[local] = phase;
     double de_re = 0.0, de_im = 0.0;
     if (has_de && p.need_de && is_finite(l.zr) && is_finite(l.zi) && is_finite(l.dr) && is_finite(l.di)) {
         if (!direct_de(l.zr, l.zi, l.dr, l.di, fe_from(p.pixel_spacing, 0), de_re, de_im)) {
@@ -208,6 +202,14 @@ __device__ void write_escape_planes(const DirectParams& p, const Lane& l, double
     }
     p.p_dex[local] = de_re;
     p.p_dey[local] = de_im;
+    if (p.p_iter == nullptr) return;
+    p.p_iter[local] = l.it;
+    double phase = 0.0;
+    if (p.need_phase && is_finite(l.zr) && is_finite(l.zi)) {
+        phase = atan2(l.zi, l.zr) / kTwoPi;
+        phase -= floor(phase);
+    }
+    p.p_phase[local] = phase;
     p.p_t1[local] = l.test1;
     p.p_t2[local] = l.test2;
 }
@@ -863,10 +865,10 @@ cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scr
     b.coords = reinterpret_cast<double*>(static_cast<char*>(scratch) + 256);
     b.chunk = shape.chunk > 0 ? shape.chunk : 64;
     const int formula = fields[0].formula;
-    const bool planes = fields[0].p_iter != nullptr;
+    const bool planes = fields[0].p_dex != nullptr;
     long long pixels = 0, coords = 0;
     for (int f = 0; f < count; ++f) {
-        if (fields[f].formula != formula || (fields[f].p_iter != nullptr) != planes) return cudaErrorInvalidValue;
+        if (fields[f].formula != formula || (fields[f].p_dex != nullptr) != planes) return cudaErrorInvalidValue;
         b.field[f] = fields[f];
         b.first[f] = pixels;
         b.coord_offset[f] = static_cast<int>(coords);

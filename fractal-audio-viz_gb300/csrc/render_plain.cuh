@@ -143,6 +143,8 @@ __device__ bool plane_de(const Sc& total, const Sc& derivative, const Fe& spacin
     return is_finite(out_re) && is_finite(out_im);
 }
 
+// Render planes: the derivative pair, and the other four or none (a batch
+// asks for the pair only).
 struct PlaneOut {
     std::int64_t* iter;
     double* phase;
@@ -152,17 +154,16 @@ struct PlaneOut {
     double* t2;
 
     __device__ void clear(long long i, int max_iter) const {
-        iter[i] = max_iter;
-        phase[i] = 0.0;
         dex[i] = 0.0;
         dey[i] = 0.0;
+        if (iter == nullptr) return;
+        iter[i] = max_iter;
+        phase[i] = 0.0;
         t1[i] = 0.0;
         t2[i] = 0.0;
     }
     __device__ void escape(long long i, int raw, const Sc& total, const Nrm& test1, const Nrm& test2,
                            const Sc& derivative, const Fe& spacing) const {
-        iter[i] = raw;
-        phase[i] = plane_phase(total);
         double de_re = 0.0, de_im = 0.0;
         if (plane_de(total, derivative, spacing, de_re, de_im)) {
             dex[i] = de_re;
@@ -171,6 +172,9 @@ struct PlaneOut {
             dex[i] = 0.0;
             dey[i] = 0.0;
         }
+        if (iter == nullptr) return;
+        iter[i] = raw;
+        phase[i] = plane_phase(total);
         t1[i] = nrm_to_d(test1);
         t2[i] = nrm_to_d(test2);
     }

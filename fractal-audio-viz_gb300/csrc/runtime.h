@@ -45,7 +45,6 @@ enum ScratchSlot {
     kScratchPoints,
     kScratchPlanesIn,
     kScratchPlanesOut,
-    kScratchDiscard,  // planes a batch's plain kernels write but no caller asked for
     kScratchAltQueue, // counters of the alternate-formula queue (one set per lane stream + one)
     kScratchAltSpill, // its spill lists, likewise
     kScratchCount

@@ -8,7 +8,8 @@ definition written with frexp, ldexp and floating-point comparisons
 nearly equal mantissas, zeros of both signs, subnormals, infinities and NaN,
 exponents near and far apart.  Host build; the device build runs the same
 code and is compared with the reference's fields by test_gpu_parity.py.  The
-raw-double sums of csrc/raw_double.h are compared with the same definitions.
+raw-double sums of csrc/raw_double.h are compared with the same definitions,
+and the integer products of csrc/int_mul.h with the FP64 product.
 """
 
 from __future__ import annotations
@@ -19,6 +20,7 @@ import subprocess
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fractal-audio-viz_gb300", "csrc")
 
 DRIVER = r"""
+#include "int_mul.h"
 #include "raw_double.h"
 #include "scaled.h"
 #include <cstdio>
@@ -206,6 +208,11 @@ int main(int, char** argv) {
         check("add_cut", sum.re == want.re && sum.im == want.im && sum.e == want.e);
         eq("to_raw", normal_form(to_raw(xn)), xn);
         check("to_raw in range", to_raw(xn).e == 0 || d_zero(xn));
+        // Integer products: normal operands and result.
+        const double fa = std::ldexp(mant(), (int)(g() % 800) - 400), fb = std::ldexp(mant(), (int)(g() % 800) - 400);
+        std::uint32_t low = ~0u;
+        const double product = int_mul(factor_a(fa), factor_b(fb), low);
+        check("int_mul", low == 0 || same(product, fa * fb));
         if (is_finite(s.re) && is_finite(s.im)) { Sc n = s; d_normalize(n); eq("to_raw any", normal_form(to_raw(n)), n); }
     }
     std::printf("bad %ld\n", bad);
