@@ -427,7 +427,7 @@ void launch_deep_alternate(ReferenceContext& ctx, DeviceTables& dev, const Outpu
 
 // Spill-list entries for a direct batch of `pixels` pixels: enough for the
 // long-running pixels of interior-heavy views (a full list only costs speed).
-long long spill_entries(long long pixels) { return std::min<long long>(pixels, 1ll << 20); }
+long long spill_entries(long long pixels) { return std::min<long long>(pixels, 1ll << 19); }
 
 DirectParams make_direct_params(const Outputs& out, int width, int height, long double zoom, long double x_center,
                                 long double y_center, int max_iter, int formula, double julia_re, double julia_im,
@@ -1647,7 +1647,7 @@ void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRunti
             for (int f = 0; f < n; ++f) pixels += static_cast<long long>(fields[i + f].width) * fields[i + f].height;
             last_direct_noalloc = false;
             check_cuda(launch_direct_batch(fields.data() + i, n, direct_scratch, shapes.direct, spill_entries(pixels),
-                                           direct_stream, plan.fast_smooth),
+                                           direct_stream, plan.fast_smooth, !plan.floatexp.empty()),
                        "direct batch launch");
         }
     }

@@ -471,7 +471,7 @@ cudaError_t launch_plain_alternate(const AltParams& params, bool planes, const A
 // travels as a __grid_constant__ kernel parameter.
 constexpr int kMaxDirectFields = 64;
 // A pixel that ran past its iteration budget, parked with its whole state
-// so that another warp resumes it bit for bit; `ready` carries the batch's
+// so that the next launch resumes it bit for bit; `ready` carries the batch's
 // generation once the entry is written.
 struct alignas(128) DirectSpill {
     double zr, zi, dr, di, test1, test2;
@@ -482,12 +482,13 @@ struct alignas(128) DirectSpill {
 // Device counters of a direct batch (at the start of its scratch).
 enum DirectCounter {
     kClaimFresh = 0,   // pixels claimed
-    kSpillReserved,    // spill slots taken by producers
-    kSpillClaimed,     // spill slots taken by consumers
     kStepsExecuted,    // iterations computed
     kQueueError,       // a wait on a spill entry gave up
-    kGeneration,       // batch generation (not reset; bumped per launch)
+    kSpillMade,        // per launch: spill slots taken by producers
+    kSpillTaken = kSpillMade + 4,   // per launch: and by consumers
+    kGeneration = kSpillTaken + 4,  // batch generation (not reset; bumped per batch)
 };
+constexpr int kDirectLaunches = 4;  // one for fresh pixels, three for spilled ones
 struct DirectBatch {
     DirectParams field[kMaxDirectFields];
     long long first[kMaxDirectFields + 1];  // pixel prefix over the batch
@@ -498,13 +499,12 @@ struct DirectBatch {
     double* coords;
     unsigned long long* counter;            // DirectCounter slots
     // A fresh pixel still running after `budget` steps is spilled (when the
-    // list has room) and resumed, to its end, by whichever warp refills
-    // first: long orbits end up 32 to a warp and start early.
+    // list has room); the launches that follow take the list 32 to a warp.
     int budget;
-    int steps;                              // steps between refills (fresh pixels in the warp)
-    int long_steps;                         // steps between refills (only resumed pixels)
+    int steps;                              // steps between refills (fresh pixels)
+    int long_steps;                         // steps between refills (spilled pixels)
     int fast_smooth;                        // smooth value in FP32 (floatexp form's direct levels)
-    DirectSpill* spill;
+    DirectSpill* spill;                     // two lists of spill_capacity entries
     long long spill_capacity;
     // Bound on a consumer's wait for a spilled entry's generation mark (then
     // kQueueError is set and the entry is dropped), and a fault-injection
@@ -516,11 +516,12 @@ struct DirectBatch {
 // direct launches (tests of the queue's error path); 0, 0 restores the
 // defaults (1 << 22 spins, publish).
 void set_direct_fault_injection(int spin_limit, int withhold_publish);
-// Device scratch for one batch: counters, coordinate tables and a spill list
-// of `spill_entries` (0: no spilling).
+// Device scratch for one batch: counters, coordinate tables and two spill
+// lists of `spill_entries` (0: no spilling).
 std::size_t direct_scratch_bytes(const DirectParams* fields, int count, long long spill_entries);
 cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scratch, const QueueShape& shape,
-                                long long spill_entries, cudaStream_t stream, bool fast_smooth = false);
+                                long long spill_entries, cudaStream_t stream, bool fast_smooth = false,
+                                bool beside_fp32 = false);
 // One direct field with its scratch taken from a fixed array compiled into
 // the library (render_noalloc.cu): no device allocation at all.
 bool launch_direct_noalloc(const DirectParams& params, cudaStream_t stream, std::string& why);

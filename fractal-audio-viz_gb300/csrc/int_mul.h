@@ -10,10 +10,12 @@
 //
 // The product of two 53-bit mantissas is formed exactly and rounded to
 // nearest: one operand scaled by 2 and the other by 2^11 puts the top 53 or
-// 54 bits in the upper word.  A tie needs the whole low half to be zero,
-// which shows as a zero lowest 32-bit word: int_mul reports that word, and
-// the caller multiplies in FP64 when it is zero (operands of few bits, or
-// one product in 2^32).  Operands and result must be normal.
+// 54 bits in the upper word.  A tie needs the low half to be zero but for its
+// top bit, so its lowest 32-bit word is zero: int_mul reports that word, and
+// where it is zero the caller takes int_mul_even, which rounds ties to even.
+// That happens for operands with 20 trailing zero bits between them: one
+// product in 50,000 of full mantissas, but every one that follows a deep
+// cancellation.  Operands and result must be normal.
 #pragma once
 
 #include "scaled.h"
@@ -65,8 +67,8 @@ FX_HD std::uint64_t wide_mad(std::uint32_t a, std::uint32_t b, std::uint64_t c) 
 #endif
 }
 
-// The correctly rounded product; `low` becomes zero where it may be a tie.
-FX_HD double int_mul(const FactorA& a, const FactorB& b, std::uint32_t& low) {
+template <bool Even>
+FX_HD double int_product(const FactorA& a, const FactorB& b, std::uint32_t& low) {
     const std::uint64_t t0 = wide_mad(a.l, b.l, 0);
     const std::uint64_t t1 = wide_mad(a.h, b.l, t0 >> 32);
     const std::uint64_t t2 = wide_mad(a.l, b.h, static_cast<std::uint32_t>(t1));
@@ -79,14 +81,30 @@ FX_HD double int_mul(const FactorA& a, const FactorB& b, std::uint32_t& low) {
     const std::uint64_t r = top + ((static_cast<std::uint32_t>(t2) >> 31) | c);
     const std::uint32_t rl = static_cast<std::uint32_t>(r), rh = static_cast<std::uint32_t>(r >> 32);
 #ifdef __CUDA_ARCH__
-    const std::uint32_t ol = __funnelshift_r(rl, rh, c);
+    std::uint32_t ol = __funnelshift_r(rl, rh, c);
 #else
-    const std::uint32_t ol = static_cast<std::uint32_t>(r >> c);
+    std::uint32_t ol = static_cast<std::uint32_t>(r >> c);
 #endif
+    if (Even) {
+        // Exactly half: the dropped bit set and nothing below it.
+        const std::uint32_t next = static_cast<std::uint32_t>(t2), last = static_cast<std::uint32_t>(t0);
+        const bool half = last == 0 && (c ? next == 0 && (static_cast<std::uint32_t>(top) & 1u) != 0
+                                          : next == 0x80000000u);
+        if (half) ol &= ~1u;
+    }
     // Sign and exponent words add; the mantissa carries its leading bit.
     const std::uint32_t oh = (rh >> c) + (c << 20)
         + (static_cast<std::uint32_t>(a.x) + static_cast<std::uint32_t>(b.x) - (1024u << 20));
     return from_hilo(static_cast<int>(oh), ol);
+}
+
+// The correctly rounded product; `low` becomes zero where it may be a tie.
+FX_HD double int_mul(const FactorA& a, const FactorB& b, std::uint32_t& low) { return int_product<false>(a, b, low); }
+
+// The correctly rounded product, ties included.
+FX_HD double int_mul_even(const FactorA& a, const FactorB& b) {
+    std::uint32_t low = 0;
+    return int_product<true>(a, b, low);
 }
 
 }  // namespace fx

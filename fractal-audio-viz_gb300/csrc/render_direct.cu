@@ -9,9 +9,11 @@
 // |z|^2 > R^2 and smooth value n + 1 - log(log|z|)/log 2.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "device.h"
+#include "int_mul.h"
 
 namespace fgb {
 namespace {
@@ -69,24 +71,70 @@ __device__ bool direct_de(double zr, double zi, double dr, double di, const Fe& 
     return is_finite(out_re) && is_finite(out_im);
 }
 
-// 2 a b for doubles a, b, formed as the product a*b with its exponent raised
-// by one.  That equals the reference's (2 a) b bit for bit when a*b lies in
-// the normal range away from its lowest binade (rounding commutes with the
-// exact doubling there) and below the overflow binade; an exactly zero
-// operand gives the signed zero of the product.  Everything else (underflow,
-// subnormal, huge, infinite, NaN) returns false and the caller multiplies.
-__device__ __forceinline__ bool twice_product(double a, double b, double& out) {
-    const double product = a * b;
-    const long long bits = __double_as_longlong(product);
-    const unsigned biased = static_cast<unsigned>((bits >> 52) & 0x7ff);
-    if (biased - 2u < 2044u) {
-        out = __longlong_as_double(bits + (1ll << 52));
+// The cross term of a step in FP64, as the reference orders it; out of line,
+// for the few operands the integer product does not take.
+template <int Formula>
+__device__ __noinline__ double cross_general(double zr, double zi) {
+    if constexpr (Formula == kFormulaBurningShip) return 2.0 * fabs_(zr) * fabs_(zi);
+    if constexpr (Formula == kFormulaTricorn) return -2.0 * zr * zi;
+    return 2.0 * zr * zi;
+}
+__device__ __noinline__ double square_general(double v) { return v * v; }
+
+// Parts whose products with each other stay normal: 2^-500 to 2^500.
+__device__ __forceinline__ bool product_range(double v) {
+    return static_cast<unsigned>((hi_of(v) & 0x7fffffff) - (523 << 20)) < (1000u << 20);
+}
+
+// (2 zr) zi (signs as the formula has them) on the integer pipe: the exact
+// product rounded once, doubled by its exponent, which is the reference's
+// (2 zr) zi bit for bit in this range.  A zero factor gives the signed zero
+// of the product.  Returns false where the value is not to be used.
+//
+// Beside the FP32 queue, which needs the issue slots (85 % taken) and leaves
+// the FP64 pipe alone, the product is an FP64 one (`Integer` false): the 1e100
+// atlas step took 16.8 ms with integer products in its direct levels.
+template <int Formula, bool Integer>
+__device__ __forceinline__ bool cross_product(double zr, double zi, double& cross) {
+    if constexpr (!Integer) {
+        const double product = Formula == kFormulaBurningShip ? fabs_(zr) * fabs_(zi) : zr * zi;
+        const bool zero = is_zero(zr) || is_zero(zi);
+        const bool fits = static_cast<unsigned>(bexp(product) - 2) < 2044u;
+        cross = fits ? add_exp(product, 1) : product;
+        if constexpr (Formula == kFormulaTricorn) cross = neg_(cross);
+        return fits || zero;
+    }
+    FactorA a = factor_a(zr);
+    FactorB b = factor_b(zi);
+    if constexpr (Formula == kFormulaBurningShip) {
+        a.x &= 0x7ff00000;
+        b.x &= 0x7ff00000;
+    } else if constexpr (Formula == kFormulaTricorn) {
+        a.x ^= static_cast<int>(0x80000000u);
+    }
+    std::uint32_t low = ~0u;
+    const int sign = (a.x ^ b.x) & static_cast<int>(0x80000000u);
+    a.x += 1 << 20;
+    cross = int_mul(a, b, low);
+    if (low == 0u) cross = int_mul_even(a, b);
+    const bool zero = is_zero(zr) || is_zero(zi);
+    if (zero) cross = from_hilo(sign, 0);
+    return zero ? is_finite(zr) && is_finite(zi) : product_range(zr) && product_range(zi);
+}
+
+template <bool Integer>
+__device__ __forceinline__ bool square_product(double v, double& square) {
+    if constexpr (!Integer) {
+        square = v * v;
         return true;
     }
-    out = product;
-    const unsigned long long magnitude = 0x7fffffffffffffffull;
-    return (static_cast<unsigned long long>(__double_as_longlong(a)) & magnitude) == 0
-        || (static_cast<unsigned long long>(__double_as_longlong(b)) & magnitude) == 0;
+    std::uint32_t low = ~0u;
+    FactorA a = factor_a(v);
+    const FactorB b = factor_b(v);
+    square = int_mul(a, b, low);
+    if (low == 0u) square = int_mul_even(a, b);
+    if (is_zero(v)) square = 0.0;
+    return is_zero(v) || product_range(v);
 }
 
 __device__ __forceinline__ unsigned long long dbits(double v) {
@@ -162,6 +210,66 @@ struct Lane {
 __device__ __forceinline__ int budget_stop(const DirectBatch& b, int max_iter) {
     if (b.budget <= 0 || b.spill_capacity <= 0) return max_iter;
     return b.budget < max_iter ? b.budget : max_iter;
+}
+
+// Up to `limit` steps of a spilled pixel on the integer and FP64 pipes, each
+// with its tests on single words: it stops before a step that escapes, may
+// close a cycle or moves the cycle marks (multiples of 64; spilled pixels are
+// past 64 steps), or whose parts are out of range, which the general step
+// then repeats.  Returns the steps taken.  Spilled pixels give each
+// sub-partition few warps, where a step costs its instructions: 110 here
+// against 250.
+template <int Formula>
+__device__ __forceinline__ int direct_run(Lane& l, int limit) {
+    const int room = min(min(limit, l.max_iter - 1 - l.it), 63 - (l.it & 63));
+    if (room <= 0 || !product_range(l.zr) || !product_range(l.zi)) return 0;
+    const int bound = hi_of(l.escape2) - (1 << 20);  // both squares below R^2 / 2 cannot escape
+    const unsigned saved = lo_of(__longlong_as_double(static_cast<long long>(l.saved_r)));
+    const unsigned mark = lo_of(__longlong_as_double(static_cast<long long>(l.mark_r)));
+    double zr = l.zr, zi = l.zi, rs = l.rs, is = l.is;
+    FactorA fr = factor_a(zr);
+    FactorB gi = factor_b(zi);
+    int k = 0;
+#pragma unroll 1
+    for (; k < room; ++k) {
+        FactorA f = fr;
+        FactorB g = gi;
+        if constexpr (Formula == kFormulaBurningShip) {
+            f.x &= 0x7ff00000;
+            g.x &= 0x7ff00000;
+        } else if constexpr (Formula == kFormulaTricorn) {
+            f.x ^= static_cast<int>(0x80000000u);
+        }
+        f.x += 1 << 20;
+        std::uint32_t low = ~0u;
+        double cross = int_mul(f, g, low);
+        if (low == 0u) cross = int_mul_even(f, g);
+        const double nr = (rs - is) + l.pr;
+        const double ni = cross + l.pi;
+        const int hr = hi_of(nr) & 0x7fffffff, hi = hi_of(ni) & 0x7fffffff;
+        fr = factor_a(nr);
+        gi = factor_b(ni);
+        const FactorB gr = factor_b(nr);
+        const FactorA fi = factor_a(ni);
+        low = ~0u;
+        double nrs = int_mul(fr, gr, low), nis = int_mul(fi, gi, low);
+        if (low == 0u) {
+            nrs = int_mul_even(fr, gr);
+            nis = int_mul_even(fi, gi);
+        }
+        if (min(hr, hi) < (523 << 20) || max(hr, hi) >= (1523 << 20) || lo_of(nr) == saved || lo_of(nr) == mark) break;
+        if (max(hi_of(nrs), hi_of(nis)) >= bound && sum_exceeds(dbits(nrs), dbits(nis), dbits(l.escape2))) break;
+        zr = nr;
+        zi = ni;
+        rs = nrs;
+        is = nis;
+    }
+    l.zr = zr;
+    l.zi = zi;
+    l.rs = rs;
+    l.is = is;
+    l.it += k;
+    return k;
 }
 
 template <bool Planes>
@@ -398,34 +506,63 @@ __device__ void finish_parked(const DirectBatch& b, const ParkSlot& e) {
 // output bit unchanged:
 //   * the squares zr*zr and zi*zi of the escape test are the next step's
 //     squares, and 2 zr zi is formed as the product zr*zi with its exponent
-//     raised by one (exact for normal numbers; the multiply otherwise);
+//     raised by one; the three products run on the integer pipe (int_mul.h)
+//     beside the three FP64 sums;
 //   * an orbit that returns bit for bit to an earlier z repeats forever and
 //     can never escape, so it is settled as interior at once (interior
 //     outputs do not depend on z); z is kept at every power of two (Brent's
 //     probe, any period) and at every multiple of 64 steps (short periods
 //     found within ~64 steps of the orbit settling).
-// FP64 is the bottleneck on this part (1/64 of the FP32 rate), so a warp
-// never waits on a finished lane: each warp claims chunks of pixels from a
-// device counter over all fields of the batch and refills idle lanes every
-// step from its start stack; escapes are parked and finished 32 at a time.
-// Capped at 64 registers (a few spills): beside the FP32 queue on one SM, a
-// block then takes as many registers as an FP32-queue block, so two of each
-// kind fit where 80-register blocks left room for fewer.
-template <int Formula, bool Planes>
-__global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_constant__ DirectBatch b) {
+// FP64 is the bottleneck on this part (one warp instruction takes an SM
+// sub-partition 80 cycles, whatever its active lanes), so a warp never waits
+// on a finished lane: each warp claims chunks of pixels from a device counter
+// over all fields of the batch and refills idle lanes every step from its
+// start stack; escapes are parked and finished 32 at a time.  A pixel past
+// b.budget steps goes to a list that later launches (`Resume`) take 32 to a
+// warp.  Resumed by whichever warp had idle lanes, while others still ran
+// fresh pixels, the long orbits of a 1920x1080 whole-set view were spread
+// over all warps, a few lanes in each (16.4 ms; 3.3 ms now, most of it the
+// latency of the orbits that run to the cap).
+//
+// The launch of fresh pixels is capped at 64 registers (a few spills): beside
+// the FP32 queue on one SM, a block then takes as many registers as an
+// FP32-queue block, so two of each kind fit where 80-register blocks left
+// room for fewer.
+constexpr int kRefill = 8;                // idle lanes before a resuming warp takes more
+constexpr int kLeave = 20;                // active lanes below which it gives its pixels back ...
+constexpr int kPatience = 16;             // ... after so many rounds,
+constexpr int kShortList = 32 * 4 * 152;  // unless the list gives a warp to each sub-partition at most
+constexpr int kResumeBlocks = 2;          // per SM: two warps for each sub-partition
+
+template <int Formula, bool Planes, bool Resume, bool Integer>
+__global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const __grid_constant__ DirectBatch b,
+                                                                           int launch) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ WarpStage stages[4];
     WarpStage& st = stages[threadIdx.x >> 5];
     const unsigned lane_id = threadIdx.x & 31u;
     const unsigned below = (1u << lane_id) - 1u;
     unsigned long long* claim = b.counter + kClaimFresh;
-    unsigned long long* reserved = b.counter + kSpillReserved;
-    unsigned long long* taken = b.counter + kSpillClaimed;
     const unsigned long long generation = *(b.counter + kGeneration);
     const long long total = b.first[b.count];
+    // This launch's input list (Resume) and the list it spills to.
+    DirectSpill* const made_list = b.spill + (launch & 1) * b.spill_capacity;
+    const DirectSpill* const list = b.spill + ((launch + 1) & 1) * b.spill_capacity;
+    unsigned long long* const made = b.counter + kSpillMade + launch;
+    unsigned long long items = 0;
+    int leave = 0;
+    if constexpr (Resume) {
+        items = *(b.counter + kSpillMade + launch - 1);
+        if (items > static_cast<unsigned long long>(b.spill_capacity)) {
+            items = static_cast<unsigned long long>(b.spill_capacity);
+        }
+        const unsigned long long rank = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        if (rank >= (items + 31) / 32) return;
+        leave = launch + 1 < kDirectLaunches && items > kShortList ? kLeave : 0;
+    }
     WarpQueue q{0, 0, 0, 0, 0, false};
     bool active = false;
-    bool resumed = false;  // the lane's pixel came from the spill list
+    int lean = 0;  // rounds with few lanes (Resume)
     unsigned long long executed = 0;  // steps this lane computed for a pixel
     Lane l;
     l.field = 0;
@@ -439,88 +576,48 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
     l.stop_at = 0;
     l.local = 0;
 
-    unsigned rounds = 0;
     while (true) {
-        unsigned idle = __ballot_sync(kFull, !active);
-        bool pending = false;  // spilled pixels exist that nobody has taken yet
-        // The spill counters live in L2: look at them every 32nd refill round
-        // (a long pixel waits a few dozen steps at most) or once the fresh
-        // queue is drained, not on every step.
-        const bool poll = (++rounds & 31u) == 0u || q.drained;
-        if (idle != 0u && b.spill_capacity > 0 && poll) {
-            // Spilled (long) pixels first: claim up to one per idle lane.
-            unsigned long long base = 0, got = 0;
-            if (lane_id == 0) {
-                unsigned long long seen = *const_cast<volatile unsigned long long*>(taken);
-                for (int attempt = 0; attempt < 64; ++attempt) {
-                    unsigned long long made = *const_cast<volatile unsigned long long*>(reserved);
-                    if (made > static_cast<unsigned long long>(b.spill_capacity)) {
-                        made = static_cast<unsigned long long>(b.spill_capacity);
-                    }
-                    if (seen >= made) break;
-                    const unsigned long long want = made - seen < static_cast<unsigned long long>(__popc(idle))
-                                                        ? made - seen
-                                                        : static_cast<unsigned long long>(__popc(idle));
-                    const unsigned long long old = atomicCAS(taken, seen, seen + want);
-                    if (old == seen) {
-                        base = seen;
-                        got = want;
-                        break;
-                    }
-                    seen = old;
+        const unsigned idle = __ballot_sync(kFull, !active);
+        const int need = __popc(idle);
+        const int rank = __popc(idle & below);
+        if constexpr (Resume) {
+            if (need >= kRefill && !q.drained) {
+                unsigned long long base = 0;
+                if (lane_id == 0) {
+                    base = atomicAdd(b.counter + kSpillTaken + launch, static_cast<unsigned long long>(need));
                 }
+                base = __shfl_sync(kFull, base, 0);
+                if (!active && base + rank < items) {
+                    // Written by an earlier launch; the wait for the entry's
+                    // generation mark is bounded.
+                    const DirectSpill& e = list[base + rank];
+                    bool ready = false;
+                    for (int spin = 0; spin < b.spin_limit; ++spin) {
+                        if (*reinterpret_cast<const volatile unsigned long long*>(&e.ready) == generation) {
+                            ready = true;
+                            break;
+                        }
+                    }
+                    if (ready) {
+                        resume_pixel<Formula>(b, e, l);
+                        active = true;
+                    } else {
+                        atomicExch(b.counter + kQueueError, 1ull);
+                    }
+                }
+                q.drained = base + need >= items;
             }
-            base = __shfl_sync(kFull, base, 0);
-            got = __shfl_sync(kFull, got, 0);
-            const int rank = __popc(idle & below);
-            const bool mine = ((idle >> lane_id) & 1u) != 0u && static_cast<unsigned long long>(rank) < got;
-            if (mine) {
-                // The producer reserved this slot before writing it; wait
-                // (bounded) for its generation mark.
-                const DirectSpill& e = b.spill[base + rank];
-                bool ready = false;
-                for (int spin = 0; spin < b.spin_limit; ++spin) {
-                    if (*reinterpret_cast<const volatile unsigned long long*>(&e.ready) == generation) {
-                        ready = true;
-                        break;
-                    }
-                }
-                __threadfence();
-                if (ready) {
-                    resume_pixel<Formula>(b, e, l);
-                    active = true;
-                    resumed = true;
-                } else {
-                    atomicExch(b.counter + kQueueError, 1ull);
-                }
-            }
-            idle &= ~__ballot_sync(kFull, mine);
-            pending = got != 0;
-        }
-        if (idle != 0u) {
-            const int need = __popc(idle);
+        } else if (need != 0) {
             while (q.starts < need && !q.drained) classify<Formula, Planes>(b, q, st, claim, lane_id, below, total);
-            const int rank = __popc(idle & below);
-            if (((idle >> lane_id) & 1u) != 0u && rank < q.starts) {
+            if (!active && rank < q.starts) {
                 begin_pixel<Formula>(b, st.start[q.starts - 1 - rank], l);
                 active = true;
-                resumed = false;
             }
             q.starts -= need < q.starts ? need : q.starts;
             __syncwarp();
         }
         if (__ballot_sync(kFull, active) == 0u) {
-            if (pending) continue;
-            // No work in hand: stop unless spilled pixels are waiting.
-            bool waiting = false;
-            if (b.spill_capacity > 0 && lane_id == 0) {
-                unsigned long long made = *const_cast<volatile unsigned long long*>(reserved);
-                if (made > static_cast<unsigned long long>(b.spill_capacity)) {
-                    made = static_cast<unsigned long long>(b.spill_capacity);
-                }
-                waiting = *const_cast<volatile unsigned long long*>(taken) < made;
-            }
-            if (__shfl_sync(kFull, waiting, 0)) continue;
+            if (Resume && !q.drained) continue;  // every entry taken was unpublished
             // Drained: finish what is parked (fewer than 32) and stop.
             if constexpr (!Planes) {
                 if (static_cast<int>(lane_id) < q.parked) finish_parked(b, st.park[lane_id]);
@@ -538,7 +635,15 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
         bool running = active;
         bool escaped = false, inside = false, spill = false;
         double rs_at_escape = 0.0, is_at_escape = 0.0;
-        const int steps = __all_sync(kFull, !active || resumed) ? b.long_steps : b.steps;
+        int steps = Resume ? b.long_steps : b.steps;
+        if constexpr (Resume && !Planes && Integer) {
+            if (active) {
+                const int taken = direct_run<Formula>(l, steps);
+                executed += static_cast<unsigned>(taken);
+                running = taken < steps;
+            }
+            steps = 1;
+        }
         for (int s = 0; s < steps; ++s) {
             if (!__any_sync(kFull, running)) break;
             executed += running ? 1u : 0u;
@@ -553,20 +658,19 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
                     l.di = ndi;
                 }
             }
-            const double ar = Formula == kFormulaBurningShip ? fabs_(l.zr) : l.zr;
-            const double ai = Formula == kFormulaBurningShip ? fabs_(l.zi) : l.zi;
             double cross;
-            const bool fast = twice_product(ar, ai, cross);
-            if (__any_sync(kFull, running && !fast)) {
-                if (!fast) cross = Formula == kFormulaTricorn ? -2.0 * l.zr * l.zi : 2.0 * ar * ai;
-                else if (Formula == kFormulaTricorn) cross = -cross;
-            } else if (Formula == kFormulaTricorn) {
-                cross = -cross;
+            const bool crossed = cross_product<Formula, Integer>(l.zr, l.zi, cross);
+            if (__any_sync(kFull, running && !crossed)) {
+                if (!crossed) cross = cross_general<Formula>(l.zr, l.zi);
             }
             const double nr = (l.rs - l.is) + l.pr;
             const double ni = cross + l.pi;
-            const double rs = nr * nr;
-            const double is = ni * ni;
+            double rs, is;
+            const bool squared_r = square_product<Integer>(nr, rs), squared_i = square_product<Integer>(ni, is);
+            if (__any_sync(kFull, running && !(squared_r && squared_i))) {
+                if (!squared_r) rs = square_general(nr);
+                if (!squared_i) is = square_general(ni);
+            }
             if (!running) continue;
             l.zr = nr;
             l.zi = ni;
@@ -599,9 +703,16 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
                 l.mark_r = br;
                 l.mark_i = bi;
             }
-            if (l.it >= l.stop_at) {
+            if (!Resume && l.it >= l.stop_at) {
                 spill = true;
                 running = false;
+            }
+        }
+        if constexpr (Resume) {
+            if (leave > 0 && q.drained) {
+                const bool going = active && !escaped && !inside;
+                if (__popc(__ballot_sync(kFull, going)) < leave) ++lean;
+                spill = lean > kPatience && going && l.stop_at == l.max_iter;
             }
         }
         if (inside) {
@@ -610,19 +721,19 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
         }
         const unsigned spilling = __ballot_sync(kFull, spill);
         if (spilling != 0u) {
-            // Hand lanes past the budget to the spill list (one reservation
-            // per warp, the entry's generation mark written last); a full
-            // list lets them run on here.
+            // Hand the lanes to the spill list (one reservation per warp, the
+            // entry's generation mark written last); a full list lets them
+            // run on here.
             const int leader = __ffs(spilling) - 1;
             unsigned long long base = 0;
             if (static_cast<int>(lane_id) == leader) {
-                base = atomicAdd(reserved, static_cast<unsigned long long>(__popc(spilling)));
+                base = atomicAdd(made, static_cast<unsigned long long>(__popc(spilling)));
             }
             base = __shfl_sync(kFull, base, leader);
             if (spill) {
                 const long long slot = static_cast<long long>(base) + __popc(spilling & below);
                 if (slot < b.spill_capacity) {
-                    DirectSpill& e = b.spill[slot];
+                    DirectSpill& e = made_list[slot];
                     e.zr = l.zr;
                     e.zi = l.zi;
                     e.dr = l.dr;
@@ -641,7 +752,7 @@ __global__ void __launch_bounds__(128, 8) direct_queue_kernel(const __grid_const
                     if (!b.withhold_publish) *reinterpret_cast<volatile unsigned long long*>(&e.ready) = generation;
                     active = false;
                 } else {
-                    l.stop_at = l.max_iter;
+                    l.stop_at = Resume ? l.max_iter + 1 : l.max_iter;  // (never offered again)
                 }
             }
         }
@@ -705,12 +816,12 @@ __global__ void direct_coords_kernel(const __grid_constant__ DirectBatch b) {
     }
 }
 
-template <int Formula, bool Planes>
+template <int Formula, bool Planes, bool Integer>
 cudaError_t launch_queue(const DirectBatch& b, int sms, int blocks_per_sm, cudaStream_t s) {
     static int per_sm = 0;
     if (per_sm == 0) {
         int blocks = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, direct_queue_kernel<Formula, Planes>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, direct_queue_kernel<Formula, Planes, false, Integer>, 128, 0);
         per_sm = blocks > 0 ? blocks : 1;
     }
     const long long pixels = b.first[b.count];
@@ -719,17 +830,21 @@ cudaError_t launch_queue(const DirectBatch& b, int sms, int blocks_per_sm, cudaS
     const long long needed = (pixels + 127) / 128;
     if (grid > needed) grid = needed;
     if (grid < 1) grid = 1;
-    direct_queue_kernel<Formula, Planes><<<static_cast<unsigned>(grid), 128, 0, s>>>(b);
+    direct_queue_kernel<Formula, Planes, false, Integer><<<static_cast<unsigned>(grid), 128, 0, s>>>(b, 0);
+    const long long resume = std::min<long long>(static_cast<long long>(sms) * kResumeBlocks, needed);
+    for (int launch = 1; launch < kDirectLaunches && b.spill_capacity > 0; ++launch) {
+        direct_queue_kernel<Formula, Planes, true, Integer><<<static_cast<unsigned>(resume), 128, 0, s>>>(b, launch);
+    }
     return cudaGetLastError();
 }
 
-template <bool Planes>
+template <bool Planes, bool Integer>
 cudaError_t launch_formula(const DirectBatch& b, int formula, int sms, int blocks_per_sm, cudaStream_t s) {
     switch (formula) {
-        case kFormulaMandelbrot: return launch_queue<kFormulaMandelbrot, Planes>(b, sms, blocks_per_sm, s);
-        case kFormulaJulia: return launch_queue<kFormulaJulia, Planes>(b, sms, blocks_per_sm, s);
-        case kFormulaBurningShip: return launch_queue<kFormulaBurningShip, Planes>(b, sms, blocks_per_sm, s);
-        default: return launch_queue<kFormulaTricorn, Planes>(b, sms, blocks_per_sm, s);
+        case kFormulaMandelbrot: return launch_queue<kFormulaMandelbrot, Planes, Integer>(b, sms, blocks_per_sm, s);
+        case kFormulaJulia: return launch_queue<kFormulaJulia, Planes, Integer>(b, sms, blocks_per_sm, s);
+        case kFormulaBurningShip: return launch_queue<kFormulaBurningShip, Planes, Integer>(b, sms, blocks_per_sm, s);
+        default: return launch_queue<kFormulaTricorn, Planes, Integer>(b, sms, blocks_per_sm, s);
     }
 }
 
@@ -811,12 +926,12 @@ cudaError_t launch_stamp_time(unsigned long long* slot, cudaStream_t stream) {
 }
 
 cudaError_t direct_queue_attributes(cudaFuncAttributes* attributes) {
-    return cudaFuncGetAttributes(attributes, direct_queue_kernel<kFormulaMandelbrot, false>);
+    return cudaFuncGetAttributes(attributes, direct_queue_kernel<kFormulaMandelbrot, false, false, false>);
 }
 
 int direct_queue_occupancy() {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, direct_queue_kernel<kFormulaMandelbrot, false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, direct_queue_kernel<kFormulaMandelbrot, false, false, false>, 128, 0);
     return blocks > 0 ? blocks : 1;
 }
 
@@ -826,7 +941,7 @@ std::size_t direct_scratch_bytes(const DirectParams* fields, int count, long lon
     std::size_t bytes = 256 + doubles * sizeof(double);
     if (spill_entries > 0) {
         bytes = (bytes + 255) / 256 * 256;
-        bytes += static_cast<std::size_t>(spill_entries) * sizeof(DirectSpill);
+        bytes += 2 * static_cast<std::size_t>(spill_entries) * sizeof(DirectSpill);
     }
     return bytes;
 }
@@ -854,7 +969,7 @@ void set_direct_fault_injection(int spin_limit, int withhold_publish) {
 }
 
 cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scratch, const QueueShape& shape,
-                                long long spill_entries, cudaStream_t stream, bool fast_smooth) {
+                                long long spill_entries, cudaStream_t stream, bool fast_smooth, bool beside_fp32) {
     if (count < 1 || count > kMaxDirectFields || !scratch) return cudaErrorInvalidValue;
     DirectBatch b{};
     b.spin_limit = fault_spin_limit;
@@ -891,8 +1006,9 @@ cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scr
     direct_coords_kernel<<<static_cast<unsigned>((coords + 255) / 256), 256, 0, stream>>>(b);
     cudaError_t status = cudaGetLastError();
     if (status != cudaSuccess) return status;
-    return planes ? launch_formula<true>(b, formula, sms, shape.blocks_per_sm, stream)
-                  : launch_formula<false>(b, formula, sms, shape.blocks_per_sm, stream);
+    if (planes) return launch_formula<true, true>(b, formula, sms, shape.blocks_per_sm, stream);
+    return beside_fp32 ? launch_formula<false, false>(b, formula, sms, shape.blocks_per_sm, stream)
+                       : launch_formula<false, true>(b, formula, sms, shape.blocks_per_sm, stream);
 }
 
 cudaError_t launch_aurora(const float* field, std::uint8_t* rgb, long long pixels, const std::uint8_t* lut,

@@ -213,6 +213,11 @@ int main(int, char** argv) {
         std::uint32_t low = ~0u;
         const double product = int_mul(factor_a(fa), factor_b(fb), low);
         check("int_mul", low == 0 || same(product, fa * fb));
+        check("int_mul_even", same(int_mul_even(factor_a(fa), factor_b(fb)), fa * fb));
+        // Products of short mantissas: exact ones and ties.
+        const int bits = (int)(g() % 30) + 1;
+        const double ga = (double)(2 * (g() % (1ull << bits)) + 1), gb = (double)(2 * (g() % (1ull << (53 - bits))) + 1);
+        check("int_mul_even tie", same(int_mul_even(factor_a(ga), factor_b(gb)), ga * gb));
         if (is_finite(s.re) && is_finite(s.im)) { Sc n = s; d_normalize(n); eq("to_raw any", normal_form(to_raw(n)), n); }
     }
     std::printf("bad %ld\n", bad);
