@@ -779,108 +779,59 @@ void* create_handle(const char* x, const char* y, const char* zoom, int max_iter
 // the host exactly as the reference does and cached per thread.
 namespace {
 
-struct AuroraCache {
+// The aurora waves' cosine / sine table (the part of aurora_palette_for that
+// depends on the iteration cap alone, renderer.cpp:4841-4860) of the calling
+// thread's last cap, on the device.
+struct AuroraWaves {
     int max_iter = -1;
-    double phase = 0, vocal = 0, pitch = 0;
-    bool accented = false;
-    std::array<std::uint8_t, 9> accents{};
-    std::vector<std::uint8_t> rgb;
     int device = -1;
-    std::uint8_t* device_lut = nullptr;
-    std::size_t device_capacity = 0;
+    const void* at = nullptr;
 };
 
-std::uint8_t colour_byte(double value) { return static_cast<std::uint8_t>(std::clamp(value, 0.0, 255.0)); }
-
-// aurora_palette_for (renderer.cpp:4841-4923); with `accents` (three RGB
-// triples) the three waves are projected through the accents before the hue
-// rotation.
-void build_aurora(AuroraCache& cache, int max_iter, double phase, double vocal, double pitch,
-                  const std::uint8_t* accents) {
-    const int size = std::min(65536, std::max(4096, max_iter * 4));
-    std::vector<float> cosine(static_cast<std::size_t>(size)), sine(static_cast<std::size_t>(size));
-    const double denominator = std::max(1, size - 1);
-    for (int i = 0; i < size; ++i) {
-        const double angle = 0.15 * static_cast<double>(max_iter) * static_cast<double>(i) / denominator;
-        cosine[static_cast<std::size_t>(i)] = static_cast<float>(std::cos(angle));
-        sine[static_cast<std::size_t>(i)] = static_cast<float>(std::sin(angle));
+// The device palette for the parameters, made on `stream`, which waits for
+// earlier users of the scratch buffers first.
+const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_iter, double phase, double vocal,
+                               double pitch, int& size, const std::uint8_t* accents = nullptr) {
+    thread_local AuroraWaves cache;
+    size = std::min(65536, std::max(4096, max_iter * 4));
+    auto* waves = static_cast<float2*>(scratch(rt, kScratchWaves, static_cast<std::size_t>(size) * sizeof(float2)));
+    if (cache.max_iter != max_iter || cache.device != rt.device || cache.at != waves) {
+        std::vector<float2> table(static_cast<std::size_t>(size));
+        const double denominator = std::max(1, size - 1);
+        for (int i = 0; i < size; ++i) {
+            const double angle = 0.15 * static_cast<double>(max_iter) * static_cast<double>(i) / denominator;
+            table[static_cast<std::size_t>(i)].x = static_cast<float>(std::cos(angle));
+            table[static_cast<std::size_t>(i)].y = static_cast<float>(std::sin(angle));
+        }
+        cache.max_iter = -1;
+        // Earlier frames may still read the previous table.
+        wait_scratch(rt, rt.stream);
+        check_cuda(cudaMemcpyAsync(waves, table.data(), table.size() * sizeof(float2), cudaMemcpyHostToDevice,
+                                   rt.stream), "upload aurora waves");
+        check_cuda(cudaStreamSynchronize(rt.stream), "upload aurora waves");
+        cache = AuroraWaves{max_iter, rt.device, waves};
     }
+    AuroraPalette p{};
     const double mix = std::clamp(vocal, 0.0, 1.0);
     const double split = 5.0 * mix * mix;
-    const double rc = std::cos(phase), rs = std::sin(phase);
-    const double gc = std::cos(phase + split * 0.4), gs = std::sin(phase + split * 0.4);
-    const double bc = std::cos(phase + split), bs = std::sin(phase + split);
+    p.rc = std::cos(phase);
+    p.rs = std::sin(phase);
+    p.gc = std::cos(phase + split * 0.4);
+    p.gs = std::sin(phase + split * 0.4);
+    p.bc = std::cos(phase + split);
+    p.bs = std::sin(phase + split);
     const double two_pi = 6.283185307179586476925286766559005768;
     const double signed_pitch = std::clamp(2.0 * (pitch - 0.5), -1.0, 1.0);
     const double hue = signed_pitch * 0.16 * two_pi;
-    const bool rotate = std::abs(hue) > 1.0e-15;
-    const double hcos = rotate ? std::cos(hue) : 1.0;
-    const double hsin = rotate ? std::sin(hue) : 0.0;
-    cache.rgb.resize(static_cast<std::size_t>(size) * 3);
-    for (int i = 0; i < size; ++i) {
-        const double c = cosine[static_cast<std::size_t>(i)];
-        const double s = sine[static_cast<std::size_t>(i)];
-        double r = (0.5 - 0.5 * (c * rc + s * rs)) * 140.0;
-        double g = (0.5 - 0.5 * (c * gc + s * gs)) * 140.0;
-        double b = (0.5 - 0.5 * (c * bc + s * bs)) * 140.0;
-        if (accents != nullptr) {
-            const double wr = std::clamp(static_cast<double>(colour_byte(r)) / 140.0, 0.0, 1.0);
-            const double wg = std::clamp(static_cast<double>(colour_byte(g)) / 140.0, 0.0, 1.0);
-            const double wb = std::clamp(static_cast<double>(colour_byte(b)) / 140.0, 0.0, 1.0);
-            const double ar = (wr * static_cast<double>(accents[0]) + wg * static_cast<double>(accents[3])
-                               + wb * static_cast<double>(accents[6])) / 1.8;
-            const double ag = (wr * static_cast<double>(accents[1]) + wg * static_cast<double>(accents[4])
-                               + wb * static_cast<double>(accents[7])) / 1.8;
-            const double ab = (wr * static_cast<double>(accents[2]) + wg * static_cast<double>(accents[5])
-                               + wb * static_cast<double>(accents[8])) / 1.8;
-            r = ar;
-            g = ag;
-            b = ab;
-        }
-        if (rotate) {
-            // Chroma rotation in YIQ (renderer.cpp:4815-4833).
-            const double y = 0.299 * r + 0.587 * g + 0.114 * b;
-            const double ii = 0.596 * r - 0.275 * g - 0.321 * b;
-            const double q = 0.212 * r - 0.523 * g + 0.311 * b;
-            const double ri = ii * hcos - q * hsin;
-            const double rq = ii * hsin + q * hcos;
-            const double nr = y + 0.956 * ri + 0.621 * rq;
-            const double ng = y - 0.272 * ri - 0.647 * rq;
-            const double nb = y - 1.106 * ri + 1.703 * rq;
-            r = nr;
-            g = ng;
-            b = nb;
-        }
-        cache.rgb[3 * static_cast<std::size_t>(i)] = colour_byte(r);
-        cache.rgb[3 * static_cast<std::size_t>(i) + 1] = colour_byte(g);
-        cache.rgb[3 * static_cast<std::size_t>(i) + 2] = colour_byte(b);
-    }
-    cache.max_iter = max_iter;
-    cache.phase = phase;
-    cache.vocal = vocal;
-    cache.pitch = pitch;
-    cache.accented = accents != nullptr;
-    if (accents != nullptr) std::copy(accents, accents + 9, cache.accents.begin());
-}
-
-// Returns the device LUT for the parameters; uploads when they change.
-const std::uint8_t* aurora_lut(ThreadRuntime& rt, int max_iter, double phase, double vocal, double pitch,
-                               int& size, const std::uint8_t* accents = nullptr) {
-    thread_local AuroraCache cache;
-    const bool same = cache.max_iter == max_iter && cache.phase == phase && cache.vocal == vocal
-        && cache.pitch == pitch && !cache.rgb.empty() && cache.accented == (accents != nullptr)
-        && (accents == nullptr || std::equal(accents, accents + 9, cache.accents.begin()));
-    if (!same) build_aurora(cache, max_iter, phase, vocal, pitch, accents);
-    size = static_cast<int>(cache.rgb.size() / 3);
-    if (!same || cache.device != rt.device || cache.device_lut == nullptr) {
-        std::uint8_t* lut = static_cast<std::uint8_t*>(scratch(rt, kScratchLut, cache.rgb.size()));
-        check_cuda(cudaMemcpyAsync(lut, cache.rgb.data(), cache.rgb.size(), cudaMemcpyHostToDevice, rt.stream),
-                   "upload aurora LUT");
-        check_cuda(cudaStreamSynchronize(rt.stream), "upload aurora LUT");
-        cache.device_lut = lut;
-        cache.device = rt.device;
-    }
-    return cache.device_lut;
+    p.rotate = std::abs(hue) > 1.0e-15 ? 1 : 0;
+    p.hue_cos = p.rotate ? std::cos(hue) : 1.0;
+    p.hue_sin = p.rotate ? std::sin(hue) : 0.0;
+    p.accented = accents != nullptr ? 1 : 0;
+    if (accents != nullptr) std::copy(accents, accents + 9, p.accents);
+    auto* lut = static_cast<std::uint8_t*>(scratch(rt, kScratchLut, static_cast<std::size_t>(size) * 3));
+    wait_scratch(rt, stream);
+    check_cuda(launch_aurora_lut(waves, size, p, lut, stream), "aurora palette launch");
+    return lut;
 }
 
 bool valid_colour_controls(double a, double b, double c, double d) {
@@ -1433,10 +1384,10 @@ AtlasLaunch atlas_colour_launch(const AtlasRequest& r, double phase, double voca
     return a;
 }
 
-void attach_aurora(ThreadRuntime& rt, AtlasLaunch& a, double phase, double vocal, double pitch,
+void attach_aurora(ThreadRuntime& rt, cudaStream_t stream, AtlasLaunch& a, double phase, double vocal, double pitch,
                    const std::uint8_t* accents) {
     int lut_size = 0;
-    a.lut = aurora_lut(rt, a.palette_iter, phase, vocal, pitch, lut_size, accents);
+    a.lut = aurora_lut(rt, stream, a.palette_iter, phase, vocal, pitch, lut_size, accents);
     a.lut_size = lut_size;
     a.index_scale = static_cast<float>(lut_size - 1) / static_cast<float>(a.palette_iter);
 }
@@ -2573,7 +2524,7 @@ int colourise_field(const float* field, uint8_t* output, int width, int height, 
         wait_scratch(rt, rt.stream);
         const std::size_t pixels = static_cast<std::size_t>(width) * static_cast<std::size_t>(height);
         int lut_size = 0;
-        const std::uint8_t* lut = aurora_lut(rt, max_iter, phase, vocal, pitch, lut_size, accents);
+        const std::uint8_t* lut = aurora_lut(rt, rt.stream, max_iter, phase, vocal, pitch, lut_size, accents);
         float* d_field = static_cast<float*>(scratch(rt, kScratchField, pixels * sizeof(float)));
         std::uint8_t* d_rgb = static_cast<std::uint8_t*>(scratch(rt, kScratchRgb, pixels * 3));
         check_cuda(cudaMemcpyAsync(d_field, field, pixels * sizeof(float), cudaMemcpyHostToDevice, rt.stream),
@@ -2764,10 +2715,8 @@ int fractal_gb300_colourise_device(const float* field, uint8_t* rgb, int width, 
         ThreadRuntime& rt = thread_runtime();
         cudaStream_t stream = stream_handle ? static_cast<cudaStream_t>(stream_handle) : rt.stream;
         int lut_size = 0;
-        wait_scratch(rt, rt.stream);
-        const std::uint8_t* lut = aurora_lut(rt, max_iter, phase, vocal, pitch, lut_size);
+        const std::uint8_t* lut = aurora_lut(rt, stream, max_iter, phase, vocal, pitch, lut_size);
         const float scale = static_cast<float>(lut_size - 1) / static_cast<float>(max_iter);
-        check_cuda(cudaStreamSynchronize(rt.stream), "aurora palette");
         check_cuda(launch_aurora(field, rgb, static_cast<long long>(width) * height, lut, lut_size, scale, max_iter,
                                  stream), "aurora kernel launch");
         release_scratch(rt, stream);
@@ -3075,7 +3024,7 @@ int atlas_colourise_common(const float* parent, int parent_width, int parent_hei
         AtlasLaunch a = atlas_colour_launch(r, phase, vocal, instrumental, pitch, interior_color);
         ThreadRuntime& rt = thread_runtime();
         wait_scratch(rt, rt.stream);
-        attach_aurora(rt, a, phase, vocal, pitch, accents);
+        attach_aurora(rt, rt.stream, a, phase, vocal, pitch, accents);
         atlas_from_host(rt, a, parent, child, output, false);
     });
 }
@@ -3620,7 +3569,7 @@ int crop_colourise_common(const float* source, int source_width, int source_heig
         for (int c = 0; c < 3; ++c) a.interior[c] = interior_color ? interior_color[c] : 0;
         ThreadRuntime& rt = thread_runtime();
         wait_scratch(rt, rt.stream);
-        attach_aurora(rt, a, phase, vocal, pitch, accents);
+        attach_aurora(rt, rt.stream, a, phase, vocal, pitch, accents);
         atlas_from_host(rt, a, source, nullptr, output, false);
     });
 }
@@ -3803,9 +3752,7 @@ int fractal_gb300_atlas_colourise_device(const float* parent, int parent_width, 
         AtlasLaunch a = atlas_colour_launch(r, phase, vocal, instrumental, pitch, interior_rgb);
         ThreadRuntime& rt = thread_runtime();
         cudaStream_t stream = stream_handle ? static_cast<cudaStream_t>(stream_handle) : rt.stream;
-        wait_scratch(rt, rt.stream);
-        attach_aurora(rt, a, phase, vocal, pitch, accents);
-        wait_scratch(rt, stream);
+        attach_aurora(rt, stream, a, phase, vocal, pitch, accents);
         a.parent = parent;
         a.child = child;
         a.rgb = output;

@@ -636,6 +636,17 @@ cudaError_t launch_pack_frame(const std::uint8_t* rgb, int width, int height, in
 
 // Records %globaltimer into *slot (the time-budget origin of the next kernel).
 cudaError_t launch_stamp_time(unsigned long long* slot, cudaStream_t stream);
+// The aurora palette's entries from the waves' cosine / sine table (two floats
+// per entry) and the frame's controls; the scalars are formed on the host.
+struct AuroraPalette {
+    double rc, rs, gc, gs, bc, bs;  // the three waves' phases
+    double hue_cos, hue_sin;
+    int rotate;
+    int accented;
+    std::uint8_t accents[9];
+};
+cudaError_t launch_aurora_lut(const float2* waves, int size, const AuroraPalette& palette, std::uint8_t* lut,
+                              cudaStream_t stream);
 cudaError_t launch_aurora(const float* field, std::uint8_t* rgb, long long pixels,
                           const std::uint8_t* lut, int lut_size, float index_scale, int max_iter,
                           cudaStream_t stream, std::uint32_t interior = 0);  // interior RGB as 0xBBGGRR

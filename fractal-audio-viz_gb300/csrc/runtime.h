@@ -33,6 +33,7 @@ enum ScratchSlot {
     kScratchTest2,
     kScratchRgb,
     kScratchLut,
+    kScratchWaves,  // the aurora palette's cosine / sine table
     kScratchKfpSamples,
     kScratchKfpAux,
     kScratchWork,
