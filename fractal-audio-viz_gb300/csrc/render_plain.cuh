@@ -16,6 +16,8 @@
 #include <cstdint>
 
 #include "device.h"
+#include "pixel_fraction.h"
+#include "raw_series.h"
 
 namespace fgb {
 namespace plain {
@@ -30,12 +32,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
-}
-
-__device__ __forceinline__ double pixel_offset(int index, int dimension, int mode) {
-    const double origin = mode == 1 ? static_cast<double>(dimension / 2)
-                                    : static_cast<double>(dimension - 1) / 2.0;
-    return static_cast<double>(index) - origin;
 }
 
 __device__ __forceinline__ float encode(double value, double bias) {
@@ -305,44 +301,126 @@ struct OrbitView {
     }
 };
 
+// How a pixel left its loops.  The logarithms of an escape are evaluated once
+// per warp after them: inside, each lane's own escape step ran them again.
+enum Exit { kExitNone, kExitNorm, kExitTail, kExitRecord };
+
+// High words of magnitudes: they order values to 2^-20.
+constexpr int kHighLow = kRawLow << 20;                                 // 2^-400
+constexpr int kHighTop = (kRawLow + static_cast<int>(kRawSpan)) << 20;  // 2^10
+constexpr int kHighUnit = (1023 - 300) << 20;
+__device__ __forceinline__ int high(double v) { return hi_of(v) & 0x7fffffff; }
+__device__ __forceinline__ bool same(const Sc& a, const Sc& b) {
+    return bits_of(a.re) == bits_of(b.re) && bits_of(a.im) == bits_of(b.im) && a.e == b.e;
+}
+// a < b for values >= +0.
+__device__ __forceinline__ bool below(double a, double b) { return bits_of(a) < bits_of(b); }
+
+__device__ __forceinline__ double2 ld_zd(const OrbitRec* r) { return __ldg(reinterpret_cast<const double2*>(r)); }
+__device__ __forceinline__ int4 ld_head(const OrbitRec* r) { return __ldg(reinterpret_cast<const int4*>(&r->zf_re)); }
+
+// derivative <- 2 total derivative + 1 on plain values, where the + 1 does not
+// move it (60 binades below) and the parts are in range; else false.
+__device__ __forceinline__ bool derivative_run(double re, double im, const Sc& v, Sc& out) {
+    const int low = imin(imin(high(re), high(im)) - kHighLow, imin(high(v.re), high(v.im)) - kHighUnit);
+    if (low < 0 || imax(high(re), high(im)) > kHighTop || static_cast<unsigned>(v.e) >= 1u << 28) return false;
+    const FactorA tr = factor_a(re), ti = factor_a(im);
+    const FactorB vr = factor_b(v.re), vi = factor_b(v.im);
+    const double xr = int_mul_even(tr, vr) - int_mul_even(ti, vi);
+    const double xi = int_mul_even(ti, vr) + int_mul_even(tr, vi);
+    const int shift = imax(bexp(xr), bexp(xi)) - 1022;
+    out = sc_make(add_exp(xr, -shift), add_exp(xi, -shift), v.e + shift + 1);
+    return imin(bexp(xr), bexp(xi)) >= 100 && out.e > 60;
+}
+
+// Up to `room` steps total <- total^2 + parameter on plain doubles whose
+// tests an FP32 estimate settles (tail_run's bound on it): 4 FP64
+// instructions each, 2 more with planes.  `open` as in tail_run.
+template <bool Planes>
+__device__ __forceinline__ int exact_run(const PlainParams& p, const Sc& parameter, int iteration, int room,
+                                         int cycle_min, Sc& total, Sc& prior, Sc& derivative, bool& open) {
+    const float bound = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * (1.0f - 0x1p-14f);
+    int made = 0;
+    while (made < room) {
+        const int hr = high(total.re), hi = high(total.im);
+        if (imin(hr, hi) < kHighLow || imax(hr, hi) > kHighTop) break;
+        if constexpr (Planes) {
+            Sc next;
+            if (!derivative_run(total.re, total.im, derivative, next)) break;
+            derivative = next;
+            prior = total;
+        }
+        const FactorA fr = factor_a(total.re), fi = factor_a(total.im);
+        const FactorB gr = factor_b(total.re), gi = factor_b(total.im);
+        const double rr = int_mul_even(fr, gr), ii = int_mul_even(fi, gi), ri = int_mul_even(fr, gi);
+        total = add_cut(sc_make(rr - ii, add_exp(ri, 1), 0), parameter);
+        ++made;
+        const float x = float_of(total.re, 0), y = float_of(total.im, 0);
+        const int it = iteration + made;
+        if (!(x * x + y * y < bound) || (p.cycle && it >= cycle_min && (it & 31) == 0)) {
+            open = true;
+            break;
+        }
+    }
+    return made;
+}
+
 // Exact scaled recurrence from the reconstructed total once the pixel has
 // left the compact reference (renderer.cpp:13053-13146 and 13155-13250).
+// kExitNorm with the last total, its norm and the one before for a value that
+// the caller finishes.
 template <bool Planes, bool Stats>
-__device__ __noinline__ void exact_continuation(const PlainParams& p, const OrbitView& orbit, long long index,
-                                   const Sc& dc, Sc total, Nrm total_norm, Sc derivative, int& iteration,
-                                   StatSink<Stats>& st, unsigned& ticks, unsigned long long deadline_ns,
-                                   float& out_value, std::uint32_t& out_count, bool& deadline,
-                                   const PlaneOut& planes) {
+__device__ __forceinline__ Exit exact_continuation(const PlainParams& p, const OrbitView& orbit, const Sc& dc, Sc& total,
+                                   Nrm& total_norm, Nrm& prior, Sc& derivative, int& iteration, StatSink<Stats>& st,
+                                   unsigned& ticks, unsigned long long deadline_ns, float& out_value,
+                                   std::uint32_t& out_count, bool& deadline) {
     const Sc parameter = sc_add(orbit.z(1), dc);
+    const Sc plain_parameter = to_raw(parameter);
+    const bool plain = plain_parameter.e == 0 && raw_or_zero(plain_parameter.re) && raw_or_zero(plain_parameter.im);
     Sc tortoise = sc_zero();
     int power = 1, length = 0;
     bool ready = false;
     const int cycle_min = p.strict_cycle ? 2048 : 512;
     const int cycle_margin = p.strict_cycle ? 78 : 60;
-    bool escaped = false;
+    out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
+    out_count = static_cast<std::uint32_t>(p.max_iter);
     while (iteration < p.max_iter) {
-        if (deadline_ns && ((ticks++ & 255U) == 0U) && global_ns() >= deadline_ns) {
+        if (deadline_ns && (ticks & 255U) == 0U && global_ns() >= deadline_ns) {
             out_value = nan_f();
             out_count = 0;
             deadline = true;
             st.add(kDeadlineAborts);
             st.add(kUnresolvedPixels);
-            return;
+            return kExitNone;
         }
-        const Nrm prior = total_norm;
-        if constexpr (Planes) derivative = sc_add(sc_twice(sc_mul(total, derivative)), sc_one());
-        total = sc_add(sc_mul(total, total), parameter);
-        ++iteration;
-        st.add(kLogical);
-        st.add(kExactSteps);
+        prior = total_norm;
+        int made = 0;
+        bool open = false;
+        total = to_raw(total);
+        if (plain && total.e == 0) {
+            Sc before = sc_zero();
+            const int room = imin(p.max_iter - iteration, deadline_ns ? 256 - static_cast<int>(ticks & 255U) : INT_MAX);
+            made = exact_run<Planes>(p, plain_parameter, iteration, room, cycle_min, total, before, derivative, open);
+            if constexpr (Planes) {
+                if (made > 1) prior = sc_norm2(normal_form(before));
+            }
+        }
+        total = normal_form(total);
+        if (made == 0) {
+            if constexpr (Planes) derivative = sc_add(sc_twice(sc_mul(total, derivative)), sc_one());
+            total = sc_add(sc_sqr(total), parameter);
+            made = 1;
+            open = true;
+        }
+        ticks += static_cast<unsigned>(made);
+        iteration += made;
+        st.add(kLogical, static_cast<unsigned long long>(made));
+        st.add(kExactSteps, static_cast<unsigned long long>(made));
         total_norm = sc_norm2(total);
+        if (!open) continue;
         if (nrm_outside(total_norm, p.escape_mode)) {
-            out_value = smooth_escape(iteration, total_norm, p.output_bias);
             out_count = static_cast<std::uint32_t>(iteration);
-            if constexpr (Planes) planes.escape(index, kalles_raw(iteration), total, total_norm, prior,
-                                                derivative, p.pixel_spacing);
-            escaped = true;
-            break;
+            return kExitNorm;
         }
         if (p.cycle) {
             if (iteration >= cycle_min && (iteration & 31) == 0 && nrm_cmp(total_norm, nrm_make(0.75, 2)) < 0) {
@@ -354,12 +432,7 @@ __device__ __noinline__ void exact_continuation(const PlainParams& p, const Orbi
                 } else {
                     const Nrm dist = sc_norm2(sc_sub(total, tortoise));
                     const int scale_e = total_norm.e > 0 ? total_norm.e : 0;
-                    if (is_zero(dist.m) || dist.e <= scale_e - cycle_margin) {
-                        out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
-                        out_count = static_cast<std::uint32_t>(p.max_iter);
-                        escaped = true;
-                        break;
-                    }
+                    if (is_zero(dist.m) || dist.e <= scale_e - cycle_margin) return kExitNone;
                     if (++length >= power) {
                         tortoise = total;
                         power = power * 2 < (1 << 20) ? power * 2 : (1 << 20);
@@ -369,72 +442,215 @@ __device__ __noinline__ void exact_continuation(const PlainParams& p, const Orbi
             }
         }
     }
-    if (!escaped) {
-        out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
-        out_count = static_cast<std::uint32_t>(p.max_iter);
-    }
+    return kExitNone;
 }
 
-// render_scaled_double_tail (renderer.cpp:12451-12669).  Returns true when
-// the tail was pathological (too many steps or rebases).
+// State of the double tail that its hot loop advances.
+template <bool Planes>
+struct Tail {
+    double dr, di;
+    Sc derivative;
+    double prior_re, prior_im;  // Z + d before the last step
+    int ref, steps, rebases;    // steps since the last rebase
+    bool ready;                 // a cycle reference is set
+};
+
+// Up to `room` tail steps whose tests FP32 estimates settle, rebases
+// included, products on the integer pipe (int_mul.h).  It stops before a step
+// it does not cover (a value out of range, the orbit's end) and after one
+// whose tests the caller must settle (`open`).  Returns the steps taken.
+//
+// A step is 5 FP64 instructions, 7 while dc reaches the sum, and 4 more with
+// planes, where the same step written out is 28 (38 with planes); the integer
+// instructions beside them take about as long.  |Z + d|^2 and |d|^2 are known
+// from FP32 to 2^-17 of the larger: R^2 is passed only above (1 - 2^-14) R^2
+// or with |d| > 4 R, and one is the smaller for certain when the estimates
+// differ by 2^-8 (the larger not below 2^-100).
+template <bool Planes>
+__device__ __forceinline__ int tail_run(const PlainParams& p, double dc_re, double dc_im, int room, Tail<Planes>& t,
+                                        bool& open) {
+    constexpr int kMaxRebases = 64;
+    double dr = t.dr, di = t.di;
+    int at = t.ref, made = 0;
+    double2 z = ld_zd(p.orbit + at);
+    int4 head = ld_head(p.orbit + at);
+    const float bound = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * (1.0f - 0x1p-14f);
+    const float far = (p.escape_mode == 1 ? 1.0e8f : 4.0f) * 16.0f;
+    const int dc_top = imax(bexp(dc_re), bexp(dc_im));
+    double total_re = 0.0, total_im = 0.0;
+    if constexpr (Planes) {
+        total_re = z.x + dr;
+        total_im = z.y + di;
+    }
+    while (made < room && at + 1 < p.orbit_size) {
+        const bool origin = is_zero(z.x) && is_zero(z.y);  // after a rebase
+        if (!origin && !(head.z & kRawOrbit)) break;
+        const int hr = high(dr), hi = high(di);
+        if (imin(hr, hi) < kHighLow || imax(hr, hi) > kHighTop) break;
+        const OrbitRec* const next = p.orbit + at + 1;
+        const double2 zn = ld_zd(next);
+        const int4 hn = ld_head(next);
+        Sc derivative = sc_zero();
+        if constexpr (Planes) {
+            if (!derivative_run(total_re, total_im, t.derivative, derivative)) break;
+        }
+        const FactorA fr = factor_a(dr), fi = factor_a(di);
+        const FactorB zr = factor_b(add_exp(z.x, 1)), zi = factor_b(add_exp(z.y, 1));
+        const double rr = int_mul_even(fr, zr), ii = int_mul_even(fi, zi);
+        const double ri = int_mul_even(fi, zr), ir = int_mul_even(fr, zi);
+        const FactorB gr = factor_b(dr), gi = factor_b(di);
+        const double uu = int_mul_even(fr, gr), vv = int_mul_even(fi, gi), uv = int_mul_even(fr, gi);
+        const double sr = uu - vv, si = add_exp(uv, 1);
+        double xr = (rr - ii) + sr, xi = (ri + ir) + si;
+        xr = choose(origin, sr, xr);
+        xi = choose(origin, si, xi);
+        // dc does not move a sum 60 binades above it.
+        if (imin(bexp(xr), bexp(xi)) <= dc_top + 60) {
+            xr = xr + dc_re;
+            xi = xi + dc_im;
+        }
+        dr = xr;
+        di = xi;
+        ++at;
+        ++made;
+        if constexpr (Planes) {
+            t.derivative = derivative;
+            t.prior_re = total_re;
+            t.prior_im = total_im;
+            total_re = zn.x + dr;
+            total_im = zn.y + di;
+        }
+        const float dx = float_of(dr, 0), dy = float_of(di, 0);
+        const float tx = __int_as_float(hn.x) + dx, ty = __int_as_float(hn.y) + dy;
+        const float m = tx * tx + ty * ty, dm = dx * dx + dy * dy;
+        const int steps = t.steps + 1;
+        const bool keep = m > dm * (1.0f + 0x1p-8f) && m > 0x1p-100f;
+        const bool move = m * (1.0f + 0x1p-8f) < dm && dm > 0x1p-100f && t.rebases < kMaxRebases;
+        if (!(m < bound && dm < far) || !(keep || move) || (p.cycle && steps >= 64 && (steps & 31) == 0)) {
+            open = true;
+            break;
+        }
+        t.steps = steps;
+        z = zn;
+        head = hn;
+        if (move) {
+            if constexpr (Planes) {
+                dr = total_re;
+                di = total_im;
+            } else {
+                dr = zn.x + dr;
+                di = zn.y + di;
+            }
+            at = 0;
+            t.steps = 0;
+            t.ready = false;
+            ++t.rebases;
+            z = ld_zd(p.orbit);
+            head = ld_head(p.orbit);
+            if constexpr (Planes) {
+                total_re = z.x + dr;
+                total_im = z.y + di;
+            }
+        }
+    }
+    t.dr = dr;
+    t.di = di;
+    t.ref = at;
+    return made;
+}
+
+// render_scaled_double_tail (renderer.cpp:12451-12669). Returns kExitTail,
+// with |Z + d|^2 in `exit_mag2`, for a value that the caller finishes.
 template <bool Planes, bool Stats>
-__device__ __noinline__ bool double_tail(const PlainParams& p, const OrbitView& orbit, long long index, const Sc& dc,
+__device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitView& orbit, long long index, const Sc& dc,
                             int& iteration, int& ref, const Sc& delta_in, Sc& derivative,
                             const Nrm& initial_norm, StatSink<Stats>& st, unsigned& ticks,
                             unsigned long long deadline_ns, float& out_value, std::uint32_t& out_count, bool& deadline,
-                            bool& unresolved, const PlaneOut& planes) {
+                            bool& unresolved, const PlaneOut& planes, double& exit_mag2,
+                            Sc& exit_total, Nrm& exit_previous) {
     const int kMaxTailRebases = 64;
     const int kMaxTailSteps = 65536;
     const double dc_re = sc_re_d(dc);
     const double dc_im = scale2(dc.im, dc.e);
     const double escape2 = escape_r2_d(p.escape_mode);
-    const double safe_escape2 = escape2 + 1.0e-7;
-    double dr = sc_re_d(delta_in);
-    double di = scale2(delta_in.im, delta_in.e);
+    Tail<Planes> t{};
+    t.dr = sc_re_d(delta_in);
+    t.di = scale2(delta_in.im, delta_in.e);
+    t.ref = ref;
+    t.derivative = derivative;
     out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
     out_count = static_cast<std::uint32_t>(p.max_iter);
     double tort_re = 0.0, tort_im = 0.0;
-    int power = 1, length = 0, tail_steps = 0, tail_iterations = 0, tail_rebases = 0;
+    int power = 1, length = 0, tail_iterations = 0;
     Nrm previous = initial_norm;
-    bool ready = false;
     const bool strict = p.strict != 0;
-    while (iteration < p.max_iter && ref >= 0 && ref + 1 < p.orbit_size) {
-        if (deadline_ns && ((ticks++ & 255U) == 0U) && global_ns() >= deadline_ns) {
+    Exit exit = kExitNone;
+    bool ended = false;
+    while (iteration < p.max_iter && t.ref >= 0 && t.ref + 1 < p.orbit_size) {
+        if (deadline_ns && (ticks & 255U) == 0U && global_ns() >= deadline_ns) {
             out_value = nan_f();
             out_count = 0;
             deadline = true;
             unresolved = true;
             st.add(kDeadlineAborts);
             st.add(kUnresolvedPixels);
-            return false;
+            ended = true;
+            break;
         }
-        const double zr = orbit.zd_re(ref);
-        const double zi = orbit.zd_im(ref);
-        if constexpr (Planes) {
-            Sc prior = sc_make(zr + dr, zi + di, 0);
-            sc_normalize(prior);
-            derivative = sc_add(sc_twice(sc_mul(prior, derivative)), sc_one());
+        int room = imin(p.max_iter - iteration, kMaxTailSteps - tail_iterations);
+        if (deadline_ns) room = imin(room, 256 - static_cast<int>(ticks & 255U));
+        bool open = false;
+        const int moved = t.rebases;
+        const int made = tail_run<Planes>(p, dc_re, dc_im, room, t, open);
+        st.add(kTailRebases, static_cast<unsigned long long>(t.rebases - moved));
+        if (made > 0) {
+            ticks += static_cast<unsigned>(made);
+            iteration += made;
+            tail_iterations += made;
+            st.add(kLogical, static_cast<unsigned long long>(made));
+            st.add(kExactSteps, static_cast<unsigned long long>(made));
+            if constexpr (Planes) {
+                if (!open) {
+                    const double re = orbit.zd_re(t.ref) + t.dr, im = orbit.zd_im(t.ref) + t.di;
+                    previous = nrm_from_d(re * re + im * im);
+                } else if (made > 1) {
+                    previous = nrm_from_d(t.prior_re * t.prior_re + t.prior_im * t.prior_im);
+                }
+            }
+            if (!open) continue;
+        } else {
+            ++ticks;
+            const double dr = t.dr, di = t.di;
+            const double zr = orbit.zd_re(t.ref);
+            const double zi = orbit.zd_im(t.ref);
+            if constexpr (Planes) {
+                Sc prior = sc_make(zr + dr, zi + di, 0);
+                sc_normalize(prior);
+                t.derivative = sc_add(sc_twice(sc_mul(prior, t.derivative)), sc_one());
+            }
+            const double lin_re = 2.0 * (zr * dr - zi * di);
+            const double lin_im = 2.0 * (zr * di + zi * dr);
+            const double sq_re = dr * dr - di * di;
+            const double sq_im = 2.0 * dr * di;
+            t.dr = lin_re + sq_re + dc_re;
+            t.di = lin_im + sq_im + dc_im;
+            ++t.ref;
+            ++iteration;
+            if (++tail_iterations > kMaxTailSteps) {
+                st.add(kTailRebaseFallbacks);
+                st.add(kUnresolvedPixels);
+                unresolved = true;
+                out_value = strict ? nan_f() : encode(static_cast<double>(iteration), p.output_bias);
+                out_count = strict ? 0u : static_cast<std::uint32_t>(iteration);
+                ended = true;
+                break;
+            }
+            st.add(kLogical);
+            st.add(kExactSteps);
         }
-        const double lin_re = 2.0 * (zr * dr - zi * di);
-        const double lin_im = 2.0 * (zr * di + zi * dr);
-        const double sq_re = dr * dr - di * di;
-        const double sq_im = 2.0 * dr * di;
-        dr = lin_re + sq_re + dc_re;
-        di = lin_im + sq_im + dc_im;
-        ++ref;
-        ++iteration;
-        if (++tail_iterations > kMaxTailSteps) {
-            st.add(kTailRebaseFallbacks);
-            st.add(kUnresolvedPixels);
-            unresolved = true;
-            out_value = strict ? nan_f() : encode(static_cast<double>(iteration), p.output_bias);
-            out_count = strict ? 0u : static_cast<std::uint32_t>(iteration);
-            return true;
-        }
-        st.add(kLogical);
-        st.add(kExactSteps);
-        const double tr = orbit.zd_re(ref) + dr;
-        const double ti = orbit.zd_im(ref) + di;
+        // The tests of the step just taken, exactly.
+        const double tr = orbit.zd_re(t.ref) + t.dr;
+        const double ti = orbit.zd_im(t.ref) + t.di;
         const double mag2 = tr * tr + ti * ti;
         if (!is_finite(mag2)) {
             unresolved = true;
@@ -442,32 +658,31 @@ __device__ __noinline__ bool double_tail(const PlainParams& p, const OrbitView& 
             st.add(kUnresolvedPixels);
             out_value = strict ? nan_f() : encode(static_cast<double>(iteration), p.output_bias);
             out_count = strict ? 0u : static_cast<std::uint32_t>(iteration);
-            return false;
+            ended = true;
+            break;
         }
-        if (mag2 > escape2) {
-            const double magnitude = sqrt(dmax(mag2, safe_escape2));
-            out_value = static_cast<float>(
-                (static_cast<double>(iteration) - log(log(magnitude)) / kLogTwo) - p.output_bias);
+        if (below(escape2, mag2)) {
             out_count = static_cast<std::uint32_t>(iteration);
+            exit = kExitTail;
+            exit_mag2 = mag2;
             if constexpr (Planes) {
-                Sc escaped = sc_make(tr, ti, 0);
-                sc_normalize(escaped);
-                planes.escape(index, kalles_raw(iteration), escaped, nrm_from_d(mag2), previous, derivative,
-                              p.pixel_spacing);
+                exit_total = sc_make(tr, ti, 0);
+                exit_previous = previous;
             }
-            return false;
+            ended = true;
+            break;
         }
-        previous = nrm_from_d(mag2);
-        const double dmag2 = dr * dr + di * di;
-        ++tail_steps;
+        if constexpr (Planes) previous = nrm_from_d(mag2);
+        const double dmag2 = t.dr * t.dr + t.di * t.di;
+        ++t.steps;
         if (p.cycle) {
-            if (tail_steps >= 64 && (tail_steps & 31) == 0) {
-                if (!ready) {
+            if (t.steps >= 64 && (t.steps & 31) == 0) {
+                if (!t.ready) {
                     tort_re = tr;
                     tort_im = ti;
                     power = 1;
                     length = 0;
-                    ready = true;
+                    t.ready = true;
                 } else {
                     const double cr = tr - tort_re;
                     const double ci = ti - tort_im;
@@ -476,7 +691,8 @@ __device__ __noinline__ bool double_tail(const PlainParams& p, const OrbitView& 
                     const double tol = p.strict_cycle ? 1.0e-24 : 1.0e-18;
                     if (iteration >= cycle_min && mag2 < 3.0 && dist2 <= tol * dmax(1.0, mag2)) {
                         if constexpr (Planes) planes.clear(index, p.max_iter);
-                        return false;
+                        ended = true;
+                        break;
                     }
                     if (++length >= power) {
                         tort_re = tr;
@@ -487,34 +703,42 @@ __device__ __noinline__ bool double_tail(const PlainParams& p, const OrbitView& 
                 }
             }
         }
-        if (mag2 < dmag2) {
-            dr = tr;
-            di = ti;
-            ref = 0;
-            tail_steps = 0;
-            ready = false;
+        if (below(mag2, dmag2)) {
+            t.dr = tr;
+            t.di = ti;
+            t.ref = 0;
+            t.steps = 0;
+            t.ready = false;
             st.add(kTailRebases);
-            if (++tail_rebases > kMaxTailRebases) {
+            if (++t.rebases > kMaxTailRebases) {
                 st.add(kTailRebaseFallbacks);
                 st.add(kUnresolvedPixels);
                 unresolved = true;
                 out_value = strict ? nan_f() : encode(static_cast<double>(iteration), p.output_bias);
                 out_count = strict ? 0u : static_cast<std::uint32_t>(iteration);
                 if constexpr (Planes) planes.clear(index, p.max_iter);
-                return true;
+                ended = true;
+                break;
             }
         }
     }
-    if (iteration < p.max_iter) {
+    derivative = t.derivative;
+    if (!ended && iteration < p.max_iter) {
         unresolved = true;
         st.add(kUnresolvedPixels);
         out_value = strict ? nan_f() : encode(static_cast<double>(iteration), p.output_bias);
         out_count = strict ? 0u : static_cast<std::uint32_t>(iteration);
         if constexpr (Planes) planes.clear(index, p.max_iter);
     }
-    return false;
+    return exit;
 }
 
+// The FP64 pipe bounds it, with the integer instructions beside it issuing in
+// 40 % of the cycles.  640x360 at 1e30: 202 us (0.92 ms with products in FP64,
+// every test exact and the logarithms at each lane's own escape), 247 us where
+// pixels repeat a rebase (1.73 ms).  Blocks of 64 threads and the larger
+// operations out of line were 2 to 8 % slower, integer products in the general
+// operations too 7 %.
 template <bool Planes, bool Stats>
 __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams p) {
     const long long total_pixels = static_cast<long long>(p.width) * p.height;
@@ -531,8 +755,8 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
     // Pixel offsets (renderer.cpp:12764-12783): the view span times the
     // signed pixel-centre fraction, both in FloatExp.
     // A point render takes dc from its list (renderer.cpp:12838-12842).
-    const double x_fraction = pixel_offset(px, p.width, p.coordinate_mode) / static_cast<double>(p.width);
-    const double y_fraction = -pixel_offset(py, p.height, p.coordinate_mode) / static_cast<double>(p.height);
+    const double x_fraction = pixel_fraction(px, p.width, p.coordinate_mode);
+    const double y_fraction = neg_(pixel_fraction(py, p.height, p.coordinate_mode));
     const Sc dc = p.points ? sc_make(p.points[index].re, p.points[index].im, p.points[index].e)
                            : sc_from_fe(fe_mul(p.view_width, x_fraction), fe_mul(p.view_height, y_fraction));
     const unsigned long long deadline_ns = p.deadline_base ? *p.deadline_base + p.budget_ns : 0ull;
@@ -542,14 +766,9 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
     int ref = 1;
     int iteration = 1;
     if (p.series_on && nrm_cmp(sc_norm2(dc), p.series_r2) <= 0) {
-        // Horner evaluation of the image series (renderer.cpp:8594-8639).
-        Sc value = ld_sc(&p.series[p.series_terms - 1]);
-        Sc poly_derivative = sc_zero();
-        for (int k = p.series_terms - 1; k > 1; --k) {
-            if constexpr (Planes) poly_derivative = sc_add(sc_mul(poly_derivative, dc), value);
-            value = sc_add(sc_mul(value, dc), ld_sc(&p.series[k - 1]));
-        }
-        if constexpr (Planes) derivative = sc_add(sc_mul(poly_derivative, dc), value);
+        Sc value, poly;
+        series_sum<Planes>([&](int k) { return ld_sc(&p.series[k]); }, p.series_terms, dc, value, poly);
+        if constexpr (Planes) derivative = sc_add(sc_mul(poly, dc), value);
         delta = sc_mul(value, dc);
         ref = p.series_iteration;
         iteration = p.series_iteration;
@@ -575,6 +794,11 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
     bool unresolved = false;
     const int cycle_min = p.strict_cycle ? 2048 : 512;
     const int cycle_margin = p.strict_cycle ? 78 : 60;
+    bool beyond = false;  // left the reference: exact steps finish the pixel
+    Exit exit = kExitNone;
+    double exit_mag2 = 0.0;
+    Sc exit_total = sc_zero();
+    Nrm exit_norm = nrm_make(0.0, 0), exit_previous = nrm_make(0.0, 0);
 
     while (iteration < p.max_iter) {
         if (deadline_ns && ((ticks++ & 255U) == 0U) && global_ns() >= deadline_ns) {
@@ -589,8 +813,10 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
         if (ref < 0 || ref >= p.orbit_size) {
             out_value = encode(static_cast<double>(iteration), p.output_bias);
             out_count = static_cast<std::uint32_t>(iteration);
-            if constexpr (Planes) planes.escape(index, kalles_raw(iteration), total, total_norm, prev_total_norm,
-                                                derivative, p.pixel_spacing);
+            exit = kExitRecord;
+            exit_total = total;
+            exit_norm = total_norm;
+            exit_previous = prev_total_norm;
             escaped = true;
             break;
         }
@@ -626,15 +852,17 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
             break;
         }
         if (nrm_outside(total_norm, p.escape_mode) || fe_positive(margin)) {
-            out_value = smooth_escape(iteration, total_norm, p.output_bias);
             out_count = static_cast<std::uint32_t>(iteration);
-            if constexpr (Planes) planes.escape(index, kalles_raw(iteration), total, total_norm, prev_total_norm,
-                                                derivative, p.pixel_spacing);
+            exit = kExitNorm;
+            exit_total = total;
+            exit_norm = total_norm;
+            exit_previous = prev_total_norm;
             escaped = true;
             break;
         }
-        if (p.cycle) {
-            if (iteration >= cycle_min && (iteration & 31) == 0 && nrm_cmp(total_norm, nrm_make(0.75, 2)) < 0) {
+        const bool cycle_turn = p.cycle && iteration >= cycle_min && (iteration & 31) == 0;
+        if (cycle_turn) {
+            if (nrm_cmp(total_norm, nrm_make(0.75, 2)) < 0) {
                 if (!ready) {
                     tortoise = total;
                     power = 1;
@@ -661,12 +889,13 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
         // Rebase when |Z + d| < |d| (renderer.cpp:13047-13153).
         const Nrm delta_norm = sc_norm2(delta);
         if (nrm_cmp(total_norm, delta_norm) < 0) {
-            if (++rebases > 64) {
-                exact_continuation<Planes, Stats>(p, orbit, index, dc, total, total_norm, derivative,
-                                                         iteration, st, ticks, deadline_ns, out_value,
-                                                         out_count, timed_out, planes);
-                if (timed_out) unresolved = true;
-                escaped = !timed_out;
+            // At index 0 the total is the delta: where the two norms, rounded
+            // differently, compare less there, the same turn repeats to the
+            // limit.  64 turns of 23 FP64 instructions doubled a field's time
+            // when one pixel in ten met them.
+            const bool repeats = ref == 0 && same(delta, total) && deadline_ns == 0 && !cycle_turn;
+            if (++rebases > 64 || repeats) {
+                beyond = true;
                 break;
             }
             delta = total;
@@ -674,11 +903,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
             continue;
         }
         if (p.map_end > 1 && ref >= p.map_end) {
-            exact_continuation<Planes, Stats>(p, orbit, index, dc, total, total_norm, derivative,
-                                                     iteration, st, ticks, deadline_ns, out_value, out_count,
-                                                     timed_out, planes);
-            if (timed_out) unresolved = true;
-            escaped = !timed_out;
+            beyond = true;
             break;
         }
         const Fe dn = fe_make(delta_norm.m, delta_norm.e);
@@ -699,22 +924,13 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
         if (bla_allowed && (map_length <= 0 || ref + map_length > p.max_iter) && delta_norm.e > -90) {
             st.add(kDoubleTailPixels);
             const int tail_start = iteration;
-            const bool pathological = double_tail<Planes, Stats>(
-                p, orbit, index, dc, iteration, ref, delta, derivative, total_norm, st, ticks, deadline_ns,
-                out_value, out_count, timed_out, unresolved, planes);
+            exit = double_tail<Planes, Stats>(p, orbit, index, dc, iteration, ref, delta, derivative, total_norm, st,
+                                              ticks, deadline_ns, out_value, out_count, timed_out, unresolved,
+                                              planes, exit_mag2, exit_total, exit_previous);
             if (timed_out || unresolved) break;
             const unsigned long long steps = iteration > tail_start ? iteration - tail_start : 0;
             st.add(kTailSteps, steps);
             st.max(kMaxTailSteps, steps);
-            if (pathological) {
-                delta = dc;
-                if constexpr (Planes) derivative = sc_one();
-                ref = 1;
-                iteration = 1;
-                have_total = false;
-                pixel_disable_bla = true;
-                continue;
-            }
             escaped = true;
             break;
         }
@@ -777,7 +993,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
                         const Sc prior = sc_add(z, delta);
                         derivative = sc_add(sc_twice(sc_mul(prior, derivative)), sc_one());
                     }
-                    delta = sc_add(sc_twice(sc_mul(z, delta)), sc_add(sc_mul(delta, delta), dc));
+                    delta = sc_add(sc_twice(sc_mul(z, delta)), sc_add(sc_sqr(delta), dc));
                     ++ref;
                     ++iteration;
                     st.add(kReplaySteps);
@@ -790,10 +1006,11 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
                         break;
                     }
                     if (nrm_outside(replay_norm, p.escape_mode) || fe_positive(replay_margin)) {
-                        out_value = smooth_escape(iteration, replay_norm, p.output_bias);
                         out_count = static_cast<std::uint32_t>(iteration);
-                        if constexpr (Planes) planes.escape(index, kalles_raw(iteration), replay_total, replay_norm,
-                                                            total_norm, derivative, p.pixel_spacing);
+                        exit = kExitNorm;
+                        exit_total = replay_total;
+                        exit_norm = replay_norm;
+                        exit_previous = total_norm;
                         escaped = true;
                         break;
                     }
@@ -832,12 +1049,34 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
             const Sc prior = sc_add(z, delta);
             derivative = sc_add(sc_twice(sc_mul(prior, derivative)), sc_one());
         }
-        delta = sc_add(sc_twice(sc_mul(z, delta)), sc_add(sc_mul(delta, delta), dc));
+        delta = sc_add(sc_twice(sc_mul(z, delta)), sc_add(sc_sqr(delta), dc));
         ++ref;
         ++iteration;
         prev_total_norm = prior_norm;
         st.add(kLogical);
         st.add(kExactSteps);
+    }
+    if (beyond) {
+        exit = exact_continuation<Planes, Stats>(p, orbit, dc, total, total_norm, exit_previous, derivative, iteration,
+                                                 st, ticks, deadline_ns, out_value, out_count, timed_out);
+        exit_total = total;
+        exit_norm = total_norm;
+        if (timed_out) unresolved = true;
+        escaped = !timed_out;
+    }
+    if (exit == kExitNorm) out_value = smooth_escape(iteration, exit_norm, p.output_bias);
+    if (exit == kExitTail) {
+        const double magnitude = sqrt(dmax(exit_mag2, escape_r2_d(p.escape_mode) + 1.0e-7));
+        out_value = static_cast<float>((static_cast<double>(iteration) - log(log(magnitude)) / kLogTwo)
+                                       - p.output_bias);
+        if constexpr (Planes) {
+            sc_normalize(exit_total);
+            exit_norm = nrm_from_d(exit_mag2);
+        }
+    }
+    if constexpr (Planes) {
+        if (exit != kExitNone) planes.escape(index, kalles_raw(iteration), exit_total, exit_norm, exit_previous,
+                                             derivative, p.pixel_spacing);
     }
     if (!escaped && !timed_out && !unresolved) {
         out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
