@@ -323,7 +323,13 @@ struct alignas(8) FxSeriesScaled {
     int terms;
     int shift;
     int scale;
-    int pad;
+    // Set where every pixel is within the series' radius and the factors
+    // below are normal floats: the pixel code then goes from the series to
+    // the plain-float tail without floatexp steps.
+    int whole;
+    float step_x, step_y;  // 2^(view exponent - scale)
+    float grow;            // 2^shift
+    float block_r2;        // no block starts there for a delta whose square exceeds this
 };
 
 struct FxParams {

@@ -15,12 +15,11 @@ namespace fgb {
 namespace {
 
 __global__ void __launch_bounds__(128, 8) floatexp_kernel(const FxParams p) {
-    const long long pixels = static_cast<long long>(p.width) * p.height;
-    const long long index = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (index >= pixels) return;
-    const int py = static_cast<int>(index / p.width);
-    const int px = static_cast<int>(index - static_cast<long long>(py) * p.width);
-    fxk::render_pixel(p, px, py);
+    // At most kMaxPixels, below 2^31.
+    const unsigned index = blockIdx.x * 128u + threadIdx.x;
+    if (index >= static_cast<unsigned>(p.width) * static_cast<unsigned>(p.height)) return;
+    const unsigned py = index / static_cast<unsigned>(p.width);
+    fxk::render_pixel(p, static_cast<int>(index - py * static_cast<unsigned>(p.width)), static_cast<int>(py));
 }
 
 // Batched persistent form: every warp claims chunks of pixels from one
@@ -52,43 +51,72 @@ __global__ void __launch_bounds__(128, 8) floatexp_queue_kernel(const __grid_con
     }
 }
 
-// Series prologue: one thread per field rescales the F2e coefficients to
-// the field's view (see FxSeriesScaled).
+// Largest squared radius of the blocks that start at reference index `start`
+// (aligned levels, whatever their length): above it no lookup finds one.
+template <typename Step>
+__device__ float start_radius2(const Step* table, const LevelIndex* index, int start) {
+    const int levels = __ldg(&index->levels);
+    if (levels == 0 || start > __ldg(&index->count[0])) return 0.0f;
+    float most = 0.0f;
+    const int offset = start - 1;
+    for (int level = 1; level < levels && (offset & ((1 << level) - 1)) == 0; ++level) {
+        if ((offset >> level) >= __ldg(&index->count[level])) continue;
+        f32x::N1e r2;
+        int len;
+        fxk::block_head(table + __ldg(&index->offset[level]) + (offset >> level), r2, len);
+        most = fmaxf(most, r2.e >= 100 ? 3.0e38f : f32x::ldexpf_fast(r2.m, r2.e));
+    }
+    return most;
+}
+
+// Series prologue: one warp per field rescales the F2e coefficients to the
+// field's view (see FxSeriesScaled), a term per lane.
 __global__ void series_prologue_kernel(const __grid_constant__ FxBatch b) {
-    const int f = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (f >= b.count) return;
-    const FxParams& p = b.field[f];
+    constexpr unsigned kFull = 0xffffffffu;
+    const FxParams& p = b.field[blockIdx.x];
     FxSeriesScaled* out = p.series_scaled;
     if (!out || !p.series_on) return;
+    static_assert(kMaxSeriesTerms <= 33, "a lane per term");
     const int scale = p.view_width.e > p.view_height.e ? p.view_width.e : p.view_height.e;
     const int terms = p.series_terms < kMaxSeriesTerms ? p.series_terms : kMaxSeriesTerms;
-    int shift = -0x3fffffff;
-    for (int k = 1; k < terms; ++k) {
-        const f32x::F2e c = p.series[k];
-        if (c.x == 0.0f && c.y == 0.0f) continue;
-        const int e = c.e + k * scale;
-        shift = e > shift ? e : shift;
-    }
+    const int k = static_cast<int>(threadIdx.x) + 1;
+    const bool has = k < terms;
+    const f32x::F2e c = has ? p.series[k] : f32x::zero();
+    const bool zero = c.x == 0.0f && c.y == 0.0f;
+    int shift = __reduce_max_sync(kFull, zero ? -0x3fffffff : c.e + k * scale);
     if (shift == -0x3fffffff) shift = 0;
-    out->b[0][0] = 0.0f;
-    out->b[0][1] = 0.0f;
     // Trailing terms below 2^-48 of the largest are dropped from the pixels'
     // Horner loop: with |u| <= 1 each is smaller than that largest term
     // times u^k by more than float rounding can see.  (Terms inside the kept
     // range stay, however small: a small low-order coefficient still
     // dominates near the view's centre.)
-    int used = 2;
-    for (int k = 1; k < terms; ++k) {
-        const f32x::F2e c = p.series[k];
-        const long long d = static_cast<long long>(c.e) + static_cast<long long>(k) * scale - shift;
-        const bool keep = d > -200 && !(c.x == 0.0f && c.y == 0.0f);
+    const long long d = static_cast<long long>(c.e) + static_cast<long long>(k) * scale - shift;
+    const bool keep = has && d > -200 && !zero;
+    if (has) {
         out->b[k][0] = keep ? f32x::ldexpf_fast(c.x, static_cast<int>(d)) : 0.0f;
         out->b[k][1] = keep ? f32x::ldexpf_fast(c.y, static_cast<int>(d)) : 0.0f;
-        if (keep && d > -48 && k + 1 > used) used = k + 1;
     }
+    const int used = __reduce_max_sync(kFull, keep && d > -48 ? k + 1 : 2);
+    if (k != 1) return;
+    out->b[0][0] = 0.0f;
+    out->b[0][1] = 0.0f;
     out->terms = used < terms ? used : terms;
     out->shift = shift;
     out->scale = scale;
+    const int sx = p.view_width.e - scale, sy = p.view_height.e - scale;
+    const f32x::N1e corner = f32x::norm2(f32x::add(f32x::make(p.view_width.x, 0.0f, p.view_width.e - 1),
+                                                   f32x::make(0.0f, p.view_height.x, p.view_height.e - 1)));
+    const int at = p.series_iteration;
+    const bool whole = p.formula == kFormulaMandelbrot && !p.shallow && !p.disable_bla && sx >= -60 && sy >= -60
+        && shift >= -60 && shift <= 30 && f32x::n_cmp(f32x::n_norm(corner.m * 1.001f, corner.e), p.series_r2) < 0
+        && at > 0 && at < p.max_iter && at + 1 < p.orbit_size && !(p.map_end > 1 && at >= p.map_end);
+    out->whole = whole ? 1 : 0;
+    if (!whole) return;
+    out->step_x = f32x::pow2f(sx);
+    out->step_y = f32x::pow2f(sy);
+    out->grow = f32x::pow2f(shift);
+    out->block_r2 = p.approx_order <= 1 ? start_radius2(p.linear, p.linear_index, at)
+                                        : start_radius2(p.cubic, p.cubic_index, at);
 }
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -267,7 +295,7 @@ int resident_grid(const void* kernel, int blocks_per_sm, long long needed_blocks
 cudaError_t launch_series_prologue(const FxParams* fields, int count, cudaStream_t stream) {
     if (count < 1 || count > kMaxFxFields) return cudaErrorInvalidValue;
     const FxBatch b = make_batch(fields, nullptr, count);
-    series_prologue_kernel<<<(count + 63) / 64, 64, 0, stream>>>(b);
+    series_prologue_kernel<<<count, 32, 0, stream>>>(b);
     return cudaGetLastError();
 }
 

@@ -240,10 +240,8 @@ __device__ __noinline__ F2e apply_cubic_derivative(const FxCubic* s, const F2e& 
 // the deep pixels' hot loop, so it is inlined into the pixel function: as a
 // call it cost a stack frame's worth of register saves per pixel.
 template <bool Planes>
-__device__ __forceinline__ PixelOut float_tail(const FxParams& p, int iteration, int ref, const F2e& delta, const F2e& dc,
-                               F2e derivative) {
-    const float dcr = to_float_x(dc), dci = to_float_y(dc);
-    float dr = to_float_x(delta), di = to_float_y(delta);
+__device__ __forceinline__ PixelOut float_tail(const FxParams& p, int iteration, int ref, float dr, float di, float dcr,
+                               float dci, F2e derivative) {
     const float escape2 = p.escape_mode == 1 ? 1.0e8f : 4.0f;
     const float safe2 = escape2 + 1.0e-7f;
     int steps = 0, rebases = 0;
@@ -426,6 +424,52 @@ __device__ __noinline__ PixelOut shallow_pixel(const FxParams& p, int px, int py
     return inside;
 }
 
+// The pixel's offset from the reference.
+__device__ __forceinline__ F2e pixel_offset(const FxParams& p, float wx, float wy) {
+    const F2e dx = norm(wx, 0.0f, p.view_width.e);
+    const F2e dy = norm(wy, 0.0f, p.view_height.e);
+    return add(make(dx.x, 0.0f, dx.e), make(0.0f, dy.x, dy.e));
+}
+
+// Its parts as plain floats, scaled as the pair above is: a shared exponent
+// first, then one multiplication by a power of two.
+__device__ __forceinline__ void pixel_offset_floats(const FxParams& p, float wx, float wy, float& x, float& y) {
+    const int bx = (f_bits(wx) >> 23) & 0xff, by = (f_bits(wy) >> 23) & 0xff;  // 0: a zero offset
+    const int ex = bx ? p.view_width.e + bx - 126 : -0x20000000, ey = by ? p.view_height.e + by - 126 : -0x20000000;
+    const int e = ex > ey ? ex : ey;
+    const float fx = wx * pow2f(max(ex - e, -41) + 126 - bx), fy = wy * pow2f(max(ey - e, -41) + 126 - by);
+    x = ldexpf_fast(ex - e < -40 ? 0.0f : fx, e);
+    y = ldexpf_fast(ey - e < -40 ? 0.0f : fy, e);
+}
+
+// The turn after the series in plain float: true where it certainly goes to
+// the tail, from there (dr, di) or, after a rebase, from the total at index
+// 0.  Its tests compare squares that the general turn rounds elsewhere, so
+// each needs 2^-10 of room (the reference's quantised norm included, |total|^2
+// > 2^-12); components are normal floats or the general turn decides.  No
+// value of the tail depends on which turn was taken: delta and total are the
+// same floats, scaled.
+__device__ __forceinline__ bool turn_to_tail(const FxParams& p, const FxSeriesScaled* sc, int& ref, float& dr,
+                                             float& di) {
+    constexpr float kRoom = 1.0f + 0x1p-10f;
+    const float2 z = orbit_float(p.orbit, ref);
+    const float tr = z.x + dr, ti = z.y + di;
+    const float m = tr * tr + ti * ti, dm = dr * dr + di * di;
+    const float limit = p.escape_mode == 1 ? 1.0e8f : 4.0f;
+    const bool clear = fminf(fabsf(dr), fabsf(di)) >= 0x1p-60f && dm > 0x1p-80f && m > 0x1p-12f
+        && m * kRoom < limit && m > 1.1e-7f * (z.x * z.x + z.y * z.y);
+    if (!clear) return false;
+    if (m > dm * kRoom) return dm > __ldg(&sc->block_r2) * kRoom;
+    if (m * kRoom < dm && m > 0.25f && fminf(fabsf(tr), fabsf(ti)) >= 0x1p-60f) {
+        // Rebased: at index 0 the total is the delta, and no block starts.
+        dr = tr;
+        di = ti;
+        ref = 0;
+        return true;
+    }
+    return false;
+}
+
 // One Mandelbrot pixel of the floatexp form; shared by the per-field kernel
 // and the batched persistent queues.
 template <bool Planes>
@@ -433,23 +477,31 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
     if (p.shallow) return shallow_pixel<Planes>(p, px, py);
     const float xf = axis_offset(px, p.width, p.coordinate_mode) / static_cast<float>(p.width);
     const float yf = -axis_offset(py, p.height, p.coordinate_mode) / static_cast<float>(p.height);
-    const F2e dx = norm(p.view_width.x * xf, 0.0f, p.view_width.e);
-    const F2e dy = norm(p.view_height.x * yf, 0.0f, p.view_height.e);
-    const F2e dc = add(make(dx.x, 0.0f, dx.e), make(0.0f, dy.x, dy.e));
-
+    const float wx = p.view_width.x * xf, wy = p.view_height.x * yf;
+    const FxSeriesScaled* sc = p.series_on ? p.series_scaled : nullptr;
+    const bool whole = sc != nullptr && __ldg(&sc->whole) != 0;
+    F2e dc = zero();
+    bool series = whole;
+    if (!whole) {
+        dc = pixel_offset(p, wx, wy);
+        series = p.series_on && n_cmp(norm2(dc), p.series_r2) <= 0;
+    }
     F2e delta = dc;
     F2e derivative = one_f2e();
     int ref = 1;
     int iteration = 1;
-    if (p.series_on && n_cmp(norm2(dc), p.series_r2) <= 0) {
-        if (p.series_scaled) {
+    bool tail = false;  // straight to the plain-float tail
+    float tail_dr = 0.0f, tail_di = 0.0f, dcr = 0.0f, dci = 0.0f;
+    if (series) {
+        ref = p.series_iteration;
+        iteration = p.series_iteration;
+        if (sc != nullptr) {
             // Plain-float Horner on u = dc 2^-scale with the field's
             // prescaled coefficients (|u| <= 1), rescaled once at the end;
             // with planes the derivative sum_k k b_k u^(k-1) alongside.
-            const FxSeriesScaled* sc = p.series_scaled;
             const int scale = __ldg(&sc->scale);
-            const float ur = ldexpf_fast(p.view_width.x * xf, p.view_width.e - scale);
-            const float ui = ldexpf_fast(p.view_height.x * yf, p.view_height.e - scale);
+            const float ur = whole ? wx * __ldg(&sc->step_x) : ldexpf_fast(wx, p.view_width.e - scale);
+            const float ui = whole ? wy * __ldg(&sc->step_y) : ldexpf_fast(wy, p.view_height.e - scale);
             const int terms = __ldg(&sc->terms);
             // Coefficient pairs in one 8-byte load each (the struct's pairs
             // are 8-byte aligned).
@@ -473,11 +525,23 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
                 vi = ni;
             }
             const int shift = __ldg(&sc->shift);
-            delta = norm(vr * ur - vi * ui, vr * ui + vi * ur, shift);
+            const float x = vr * ur - vi * ui, y = vr * ui + vi * ur;
             if constexpr (Planes) {
                 // d/dc [v(u) u] 2^shift = (v + u v'(u)) 2^(shift - scale)
                 derivative = norm(vr + (wr * ur - wi * ui), vi + (wr * ui + wi * ur), shift - scale);
             }
+            if (whole) {
+                const float grow = __ldg(&sc->grow);
+                tail_dr = x * grow;
+                tail_di = y * grow;
+                tail = turn_to_tail(p, sc, ref, tail_dr, tail_di);
+                if (tail) {
+                    pixel_offset_floats(p, wx, wy, dcr, dci);
+                } else {
+                    dc = pixel_offset(p, wx, wy);
+                }
+            }
+            if (!tail) delta = norm(x, y, shift);
         } else {
             F2e value = ld_f2e(&p.series[p.series_terms - 1]);
             F2e poly = zero();
@@ -488,8 +552,6 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
             if constexpr (Planes) derivative = add(mul(poly, dc), value);
             delta = mul(value, dc);
         }
-        ref = p.series_iteration;
-        iteration = p.series_iteration;
     }
     const N1e limit = bailout(p.escape_mode);
     const N1e three = N1e{0.75f, 2};
@@ -499,7 +561,7 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
     N1e total_norm = n_norm(0.0f, 0);
     bool no_pixel_bla = false;
     int rebases = 0;
-    while (iteration < p.max_iter) {
+    while (!tail && iteration < p.max_iter) {
         if (ref < 0 || ref >= p.orbit_size) {
             result = out_of(static_cast<float>(iteration) - p.output_bias, static_cast<std::uint32_t>(iteration));
             break;
@@ -558,7 +620,11 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
         }
         const int length = lin ? __ldg(&lin->len) : (cub ? __ldg(&cub->len) : 0);
         if (bla && (length <= 0 || ref + length > p.max_iter) && dn.e > -90) {
-            result = float_tail<Planes>(p, iteration, ref, delta, dc, derivative);
+            tail_dr = to_float_x(delta);
+            tail_di = to_float_y(delta);
+            dcr = to_float_x(dc);
+            dci = to_float_y(dc);
+            tail = true;
             break;
         }
         if (length > 0 && ref + length <= p.max_iter) {
@@ -616,6 +682,9 @@ __device__ __noinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int p
         delta = add(twice(mul(z, delta)), add(mul(delta, delta), dc));
         ++ref;
         ++iteration;
+    }
+    if (tail) {
+        result = float_tail<Planes>(p, iteration, ref, tail_dr, tail_di, dcr, dci, derivative);
     }
     return result;
 }
