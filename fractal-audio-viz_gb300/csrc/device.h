@@ -318,8 +318,8 @@ constexpr int kStatsSlots = 39;
 // (k >= 1) with u = dc * 2^-scale, |u| <= 1 over the view, so every pixel
 // evaluates it in plain float (kernel-side prologue, render_fe.cu).
 constexpr int kMaxSeriesTerms = 33;
-struct alignas(8) FxSeriesScaled {
-    float b[kMaxSeriesTerms][2];
+struct alignas(16) FxSeriesScaled {
+    float b[kMaxSeriesTerms + 1][2];  // the last pair only fills the 16 bytes
     int terms;
     int shift;
     int scale;
@@ -328,6 +328,7 @@ struct alignas(8) FxSeriesScaled {
     // the plain-float tail without floatexp steps.
     int whole;
     float step_x, step_y;  // 2^(view exponent - scale)
+    float per_x, per_y;    // 1 / width, 1 / height
     float grow;            // 2^shift
     float block_r2;        // no block starts there for a delta whose square exceeds this
 };

@@ -43,10 +43,9 @@ __global__ void __launch_bounds__(128, 8) floatexp_queue_kernel(const __grid_con
         for (long long g = static_cast<long long>(base) + lane; g < end; g += 32) {
             while (g >= b.first[f + 1]) ++f;
             const FxParams& p = b.field[f];
-            const int local = static_cast<int>(g - b.first[f]);
-            const int py = local / p.width;
-            const int px = local - py * p.width;
-            fxk::render_pixel(p, px, py);
+            const unsigned local = static_cast<unsigned>(g - b.first[f]);
+            const unsigned py = local / static_cast<unsigned>(p.width);
+            fxk::render_pixel(p, static_cast<int>(local - py * static_cast<unsigned>(p.width)), static_cast<int>(py));
         }
     }
 }
@@ -109,11 +108,14 @@ __global__ void series_prologue_kernel(const __grid_constant__ FxBatch b) {
     const int at = p.series_iteration;
     const bool whole = p.formula == kFormulaMandelbrot && !p.shallow && !p.disable_bla && sx >= -60 && sy >= -60
         && shift >= -60 && shift <= 30 && f32x::n_cmp(f32x::n_norm(corner.m * 1.001f, corner.e), p.series_r2) < 0
+        && p.width <= 32768 && p.height <= 32768
         && at > 0 && at < p.max_iter && at + 1 < p.orbit_size && !(p.map_end > 1 && at >= p.map_end);
     out->whole = whole ? 1 : 0;
     if (!whole) return;
     out->step_x = f32x::pow2f(sx);
     out->step_y = f32x::pow2f(sy);
+    out->per_x = 1.0f / static_cast<float>(p.width);
+    out->per_y = 1.0f / static_cast<float>(p.height);
     out->grow = f32x::pow2f(shift);
     out->block_r2 = p.approx_order <= 1 ? start_radius2(p.linear, p.linear_index, at)
                                         : start_radius2(p.cubic, p.cubic_index, at);

@@ -302,10 +302,14 @@ __device__ __noinline__ PixelOut alt_pixel(const FxParams& p, int px, int py) {
     return out_of(static_cast<float>(p.max_iter) - p.output_bias, static_cast<std::uint32_t>(p.max_iter));
 }
 
+__device__ __noinline__ PixelOut floatexp_pixel_planes(const FxParams& p, int px, int py) {
+    return floatexp_pixel<true>(p, px, py);
+}
+
 // Every field kind of the floatexp form: Mandelbrot (deep or shallow mode)
 // or another formula, with or without derivative planes.
 __device__ __forceinline__ PixelOut field_pixel(const FxParams& p, int px, int py) {
-    if (p.formula == kFormulaMandelbrot) return p.de_x ? floatexp_pixel<true>(p, px, py) : floatexp_pixel<false>(p, px, py);
+    if (p.formula == kFormulaMandelbrot) return p.de_x ? floatexp_pixel_planes(p, px, py) : floatexp_pixel<false>(p, px, py);
     return p.de_x ? alt_pixel<true>(p, px, py) : alt_pixel<false>(p, px, py);
 }
 
