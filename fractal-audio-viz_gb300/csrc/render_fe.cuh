@@ -462,7 +462,9 @@ __device__ __forceinline__ bool turn_to_tail(const FxParams& p, const FxSeriesSc
         && m * kRoom < limit && m > 1.1e-7f * (z.x * z.x + z.y * z.y);
     if (!clear) return false;
     if (m > dm * kRoom) return dm > __ldg(&sc->block_r2) * kRoom;
-    if (m * kRoom < dm && m > 0.25f && fminf(fabsf(tr), fabsf(ti)) >= 0x1p-60f) {
+    // (With the high bailout the quantised norm of a small total may compare
+    // below the delta's again at index 0.)
+    if (m * kRoom < dm && (p.escape_mode != 1 || m > 0.25f) && fminf(fabsf(tr), fabsf(ti)) >= 0x1p-60f) {
         // Rebased: at index 0 the total is the delta, and no block starts.
         dr = tr;
         di = ti;
@@ -684,9 +686,8 @@ __device__ __noinline__ PixelOut floatexp_general(const FxParams& p, int px, int
 // pixels whose turn that leaves open take general turns.  Of a
 // field at 1e100 1,375 instructions per pixel were 170 of series, 7 tail steps
 // of 20 and about 1,000 of floatexp offsets, norms and tests around them:
-// 3840x2160 in 348 us, and 243 us without those, in calls; inlined, with
-// offsets divided by Markstein's rule, the 112-level 1920x1080 ladder took
-// 12.5 ms before and 11.4 ms after.
+// 3840x2160 in 348 us, the 112-level 1920x1080 ladder in 16.3 ms, and 11.1 ms
+// this way (12.5 ms while it was a call with IEEE divisions).
 template <bool Planes>
 __device__ __forceinline__ PixelOut floatexp_pixel(const FxParams& p, int px, int py) {
     if (p.shallow) return shallow_pixel<Planes>(p, px, py);
