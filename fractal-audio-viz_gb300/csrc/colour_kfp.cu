@@ -65,8 +65,7 @@ struct KfpDevice {
 // differences of raw float field values, which FP32 forms exactly for
 // neighbouring values; only the special cases (interior, glitch, clamps) are
 // shifted into the same frame.
-__device__ __forceinline__ float sample(const float* __restrict__ field, const KfpDevice& k, int x, int y) {
-    const float v = __ldg(field + static_cast<long long>(y) * k.width + x);
+__device__ __forceinline__ float sample_of(const KfpDevice& k, float v) {
     // Common case without FP64: a finite value in [0, max_iter - bias) with a
     // non-negative bias and offset passes through unchanged (v >= 0 makes both
     // shifted values non-negative; v < sample_hi is the double comparison
@@ -85,6 +84,10 @@ __device__ __forceinline__ float sample(const float* __restrict__ field, const K
     return v;
 }
 
+__device__ __forceinline__ float sample(const float* __restrict__ field, const KfpDevice& k, int x, int y) {
+    return sample_of(k, __ldg(field + static_cast<long long>(y) * k.width + x));
+}
+
 // x / d for a constant divisor d with r = RN(1 / d), by Markstein's
 // correction of the rounded product (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
@@ -99,6 +102,14 @@ __device__ __forceinline__ float div_const(float x, float d, float r) {
     const float q0 = __fmul_rn(x, r);
     const float e = __fmaf_rn(-q0, d, x);
     return __fmaf_rn(e, r, q0);
+}
+
+// v / 255 for a palette share v in [0, 256): a share below 2^-100, where the
+// corrected product may miss the quotient, moves no byte.
+__device__ __forceinline__ float byte_share(float v) {
+    constexpr float r = 1.0f / 255.0f;
+    const float q0 = __fmul_rn(v, r);
+    return __fmaf_rn(__fmaf_rn(-q0, 255.0f, v), r, q0);
 }
 
 constexpr float kHalfPiF = kPiF / 2.0f;
@@ -462,7 +473,13 @@ __device__ __forceinline__ void kfp_pixel(const float* __restrict__ field, const
         return reflected(field, k, x, y, dx, dy, centre);
     };
     float l = centre, r = centre, u = centre, d = centre, tl = centre, tr = centre, bl = centre, br = centre;
-    if (needs_difference || needs_slopes || texture) {
+    if (Kalles && !Planes && x > 0 && y > 0) {
+        // Its three neighbours, all in the frame.
+        const float* const at = field + index;
+        l = sample_of(k, __ldg(at - 1));
+        u = sample_of(k, __ldg(at - k.width));
+        tl = sample_of(k, __ldg(at - k.width - 1));
+    } else if (needs_difference || needs_slopes || texture) {
         l = neighbour(-1, 0);
         u = neighbour(0, -1);
         if (needs_difference) {
@@ -587,11 +604,9 @@ __device__ __forceinline__ void kfp_pixel(const float* __restrict__ field, const
             if (inverse_transition) f = 1.0f - f;
             const int upper = lower + 1 < k.lut_size ? lower + 1 : 0;  // (lower + 1) mod size, lower in [0, size)
             const float g = 1.0f - f;
-            o_r = FGB_DIV(static_cast<float>(lut[lower * 3]) * g + static_cast<float>(lut[upper * 3]) * f, 255.0f);
-            o_g = FGB_DIV(static_cast<float>(lut[lower * 3 + 1]) * g + static_cast<float>(lut[upper * 3 + 1]) * f,
-                          255.0f);
-            o_b = FGB_DIV(static_cast<float>(lut[lower * 3 + 2]) * g + static_cast<float>(lut[upper * 3 + 2]) * f,
-                          255.0f);
+            o_r = byte_share(static_cast<float>(lut[lower * 3]) * g + static_cast<float>(lut[upper * 3]) * f);
+            o_g = byte_share(static_cast<float>(lut[lower * 3 + 1]) * g + static_cast<float>(lut[upper * 3 + 1]) * f);
+            o_b = byte_share(static_cast<float>(lut[lower * 3 + 2]) * g + static_cast<float>(lut[upper * 3 + 2]) * f);
         } else {
             o_r = FGB_DIV(static_cast<float>(lut[lower * 3]), 255.0f);
             o_g = FGB_DIV(static_cast<float>(lut[lower * 3 + 1]), 255.0f);

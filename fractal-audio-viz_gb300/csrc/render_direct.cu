@@ -856,7 +856,7 @@ __device__ __forceinline__ double unit(double v) { return v < 0.0 ? 0.0 : (1.0 <
 // reference's double operations in its order (this translation unit has no
 // FMA contraction), so its bytes are the reference's.  A music-driven frame
 // has new controls each time: on the host the 65,536 entries took 1.2 ms of
-// such a frame, here 8 us of FP64, and nothing waits for an upload.
+// such a frame, here 13 us of FP64, and nothing waits for an upload.
 __global__ void __launch_bounds__(128) aurora_lut_kernel(const float2* __restrict__ waves, int size,
                                                          const __grid_constant__ AuroraPalette p,
                                                          std::uint8_t* __restrict__ lut) {
