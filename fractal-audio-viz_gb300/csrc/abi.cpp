@@ -24,6 +24,7 @@
 #include "device.h"
 #include "mlp.h"
 #include "fractal_gb300.h"
+#include "host_pages.h"
 #include "reference.h"
 #include "runtime.h"
 
@@ -122,6 +123,13 @@ void* scratch(ThreadRuntime& rt, ScratchSlot slot, std::size_t bytes) {
         rt.capacity[slot] = bytes;
     }
     return rt.scratch[slot];
+}
+
+// A result into the caller's memory, whose pages are mapped while the render
+// before it runs.
+void copy_to_caller(void* to, const void* from, std::size_t bytes, cudaStream_t stream, const char* what) {
+    map_pages(to, bytes);
+    check_cuda(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, stream), what);
 }
 
 void wait_scratch(ThreadRuntime& rt, cudaStream_t stream) {
@@ -688,21 +696,23 @@ void render_to_host(float* output, FractalRenderPlanes* planes, int width, int h
     check_cuda(cudaEventRecord(rt.start, rt.stream), "cudaEventRecord");
     launch(out, collect, rt, rt.stream);
     check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-    check_cuda(cudaMemcpyAsync(output, out.field, pixels * sizeof(float), cudaMemcpyDeviceToHost, rt.stream),
-               "copy field to host");
     if (planes) {
-        check_cuda(cudaMemcpyAsync(planes->orbit_iteration, out.p_iter, pixels * sizeof(std::int64_t),
-                                   cudaMemcpyDeviceToHost, rt.stream), "copy planes");
-        check_cuda(cudaMemcpyAsync(planes->phase, out.p_phase, pixels * sizeof(double), cudaMemcpyDeviceToHost,
-                                   rt.stream), "copy planes");
-        check_cuda(cudaMemcpyAsync(planes->de_x, out.p_dex, pixels * sizeof(double), cudaMemcpyDeviceToHost,
-                                   rt.stream), "copy planes");
-        check_cuda(cudaMemcpyAsync(planes->de_y, out.p_dey, pixels * sizeof(double), cudaMemcpyDeviceToHost,
-                                   rt.stream), "copy planes");
-        check_cuda(cudaMemcpyAsync(planes->test1, out.p_t1, pixels * sizeof(double), cudaMemcpyDeviceToHost,
-                                   rt.stream), "copy planes");
-        check_cuda(cudaMemcpyAsync(planes->test2, out.p_t2, pixels * sizeof(double), cudaMemcpyDeviceToHost,
-                                   rt.stream), "copy planes");
+        // All of them now: a copy to pageable memory holds this thread.
+        map_pages(output, pixels * sizeof(float));
+        for (void* plane : {static_cast<void*>(planes->orbit_iteration), static_cast<void*>(planes->phase),
+                            static_cast<void*>(planes->de_x), static_cast<void*>(planes->de_y),
+                            static_cast<void*>(planes->test1), static_cast<void*>(planes->test2)}) {
+            map_pages(plane, pixels * sizeof(double));
+        }
+    }
+    copy_to_caller(output, out.field, pixels * sizeof(float), rt.stream, "copy field to host");
+    if (planes) {
+        copy_to_caller(planes->orbit_iteration, out.p_iter, pixels * sizeof(std::int64_t), rt.stream, "copy planes");
+        copy_to_caller(planes->phase, out.p_phase, pixels * sizeof(double), rt.stream, "copy planes");
+        copy_to_caller(planes->de_x, out.p_dex, pixels * sizeof(double), rt.stream, "copy planes");
+        copy_to_caller(planes->de_y, out.p_dey, pixels * sizeof(double), rt.stream, "copy planes");
+        copy_to_caller(planes->test1, out.p_t1, pixels * sizeof(double), rt.stream, "copy planes");
+        copy_to_caller(planes->test2, out.p_t2, pixels * sizeof(double), rt.stream, "copy planes");
     }
     std::array<unsigned long long, kStatsSlots> stats{};
     if (collect) {
@@ -1099,7 +1109,7 @@ int kfp_host(const float* field, uint8_t* output, int width, int height, int max
         check_cuda(cudaEventRecord(rt.start, rt.stream), "cudaEventRecord");
         kfp_colour(d_field, d_rgb, width, height, max_iter, *options, in, lut_size, rt, rt.stream);
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream), "copy RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "KFP colour");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -1249,7 +1259,7 @@ int kfp_planes_host(const float* field, uint8_t* output, int width, int height, 
         }
         kfp_colour(d_field, d_rgb, width, height, max_iter, o, in, lut_size, rt, rt.stream, &pl, samples, flags);
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream), "copy RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "KFP plane colour");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -1434,8 +1444,7 @@ void atlas_from_host(ThreadRuntime& rt, AtlasLaunch& a, const void* parent, cons
     check_cuda(cudaEventRecord(rt.start, rt.stream), "cudaEventRecord");
     check_cuda(run_atlas(rt, a, tables, rt.stream), "atlas kernel launch");
     check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-    check_cuda(cudaMemcpyAsync(output, device_out, out_bytes, cudaMemcpyDeviceToHost, rt.stream),
-               "copy atlas frame to host");
+    copy_to_caller(output, device_out, out_bytes, rt.stream, "copy atlas frame to host");
     check_cuda(cudaStreamSynchronize(rt.stream), "atlas frame");
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -2534,7 +2543,7 @@ int colourise_field(const float* field, uint8_t* output, int width, int height, 
         check_cuda(launch_aurora(d_field, d_rgb, static_cast<long long>(pixels), lut, lut_size, scale, max_iter,
                                  rt.stream, interior), "aurora kernel launch");
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream), "copy RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "aurora colour");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -3108,8 +3117,7 @@ int fractal_atlas_colourise_kfp_raw(const float* parent, int parent_width, int p
         check_cuda(run_atlas(rt, a, tables, rt.stream), "atlas surface launch");
         kfp_colour(a.field_out, d_rgb, output_width, output_height, max_iter, *options, in, lut_size, rt, rt.stream);
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream),
-                   "copy atlas RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy atlas RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "raw KFP atlas");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -3180,8 +3188,7 @@ int fractal_atlas_colourise_kfp(const float* parent, int parent_width, int paren
         }
         check_cuda(launch_kfp_atlas(at, d_rgb, k, in.lut, in.period, in.type, rt.stream), "KFP atlas launch");
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream),
-                   "copy atlas RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy atlas RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "KFP atlas");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -3344,8 +3351,7 @@ int fractal_atlas_colourise_kfp_planes(const float* parent, int parent_width, in
         kfp_colour(a.field_out, d_rgb, output_width, output_height, target_max_iter, o, in, lut_size, rt, rt.stream,
                    &pl, samples, flags);
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream),
-                   "copy atlas RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy atlas RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "plane-aware KFP atlas");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;
@@ -3613,8 +3619,7 @@ int crop_colourise_kfp_common(const float* source, int source_width, int source_
         check_cuda(run_atlas(rt, a, tables, rt.stream), "crop surface launch");
         kfp_colour(a.field_out, d_rgb, output_width, output_height, max_iter, *options, in, lut_size, rt, rt.stream);
         check_cuda(cudaEventRecord(rt.stop, rt.stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(output, d_rgb, pixels * 3, cudaMemcpyDeviceToHost, rt.stream),
-                   "copy crop RGB to host");
+        copy_to_caller(output, d_rgb, pixels * 3, rt.stream, "copy crop RGB to host");
         check_cuda(cudaStreamSynchronize(rt.stream), "KFP crop");
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, rt.start, rt.stop) == cudaSuccess) rt.last_kernel_ms = ms;

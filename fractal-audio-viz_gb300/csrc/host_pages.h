@@ -1,0 +1,41 @@
+// Pages of a caller's buffer, mapped before the GPU copies into it.
+//
+// A fresh allocation has no pages yet.  On this machine the copy to host then
+// faults them in one by one from the GPU's side: six planes of 960x540 into
+// new arrays took 20 ms against 1.1 ms into mapped ones.  Asking the kernel
+// for the whole range takes 0.3 to 1.3 ms, on the calling thread while the
+// render runs: the same render took 20 ms before and takes 1.6 ms now.
+// Contents do not change; a range that cannot be mapped
+// for writing, or a kernel without the request, leaves the copy as it was.
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+
+#ifdef __linux__
+#include <sys/mman.h>
+#include <unistd.h>
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23  // Linux 5.14
+#endif
+#endif
+
+namespace fgb {
+
+// Below this the copy is staged by the driver and faults nothing.
+constexpr std::size_t kMapFrom = 64 * 1024;
+
+inline void map_pages(void* at, std::size_t bytes) {
+#ifdef __linux__
+    if (at == nullptr || bytes < kMapFrom) return;
+    static const std::uintptr_t page = static_cast<std::uintptr_t>(sysconf(_SC_PAGESIZE));
+    const std::uintptr_t first = reinterpret_cast<std::uintptr_t>(at) & ~(page - 1);
+    const std::uintptr_t end = (reinterpret_cast<std::uintptr_t>(at) + bytes + page - 1) & ~(page - 1);
+    (void)madvise(reinterpret_cast<void*>(first), end - first, MADV_POPULATE_WRITE);
+#else
+    (void)at;
+    (void)bytes;
+#endif
+}
+
+}  // namespace fgb
