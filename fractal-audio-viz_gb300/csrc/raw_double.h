@@ -68,6 +68,15 @@ FX_HD Sc add_cut(const Sc& a, const Sc& b) {
     return sc_make(diff > 60 ? a.re : choose(diff < -60, b.re, re), diff > 60 ? a.im : choose(diff < -60, b.im, im), 0);
 }
 
+// Whether a part z + d of a raw z lies on the other side of zero than z, zero
+// counting with the positive side: a positive z that d cancels exactly stays,
+// a negative one crosses (a row of pixels on the real axis meets both).
+FX_HD bool folds(double z, double d) {
+    const std::uint64_t magnitude = 0x7fffffffffffffffull;
+    return (hi_of(z) ^ hi_of(d)) < 0
+        && (bits_of(d) & magnitude) >= (bits_of(z) & magnitude) + (hi_of(z) >= 0 ? 1u : 0u);
+}
+
 FX_HD double flip(double v, bool negate) {
     return from_hilo(hi_of(v) ^ (negate ? static_cast<int>(0x80000000u) : 0), lo_of(v));
 }

@@ -361,11 +361,6 @@ __device__ __forceinline__ Sc alt_step_raw(const double2& z, const Sc& d, const 
     return add_cut(sc_make(lr, li, 0), sc_make(sr, si, 0));
 }
 
-// A part of Z + d has crossed zero, or reached it.
-__device__ __forceinline__ bool folds(double z, double d) {
-    return (hi_of(z) ^ hi_of(d)) < 0 && (bits_of(d) & 0x7fffffffffffffffull) >= (bits_of(z) & 0x7fffffffffffffffull);
-}
-
 // AlternateLinearBlaLevels::lookup (renderer.cpp:8536-8567).
 // The delta's squared norm is formed only where the exponents leave its
 // order against the two-step block's radius open.
