@@ -118,8 +118,10 @@ void* scratch(ThreadRuntime& rt, ScratchSlot slot, std::size_t bytes) {
         rt.capacity[slot] = 0;
         check_cuda(cudaMalloc(&rt.scratch[slot], bytes), "cudaMalloc (scratch)");
         // Zeroed once: the direct queue's spill entries carry a generation
-        // mark that must not match by accident.
-        check_cuda(cudaMemset(rt.scratch[slot], 0, bytes), "cudaMemset (scratch)");
+        // mark that must not match by accident.  Complete before it is handed
+        // out: no stream of the library's, nor a caller's, waits for another.
+        check_cuda(cudaMemsetAsync(rt.scratch[slot], 0, bytes, rt.stream), "cudaMemset (scratch)");
+        check_cuda(cudaStreamSynchronize(rt.stream), "cudaMemset (scratch)");
         rt.capacity[slot] = bytes;
     }
     return rt.scratch[slot];
