@@ -203,6 +203,12 @@ bool reserve(CostNet* n, int rows, std::string& why) {
         free_workspace(n);
         return false;
     }
+    // The callers' streams do not wait for the clears.
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        why = "cost network: CUDA error while clearing the workspace";
+        free_workspace(n);
+        return false;
+    }
     n->capacity = rows;
     return true;
 }

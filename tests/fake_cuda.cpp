@@ -5,7 +5,8 @@
 // Streams are numbered handles; work on them is only counted.  What is
 // watched:
 //   * fake_hazards: launches made while the clear of a new allocation may
-//     still run (cleared as a whole, on a stream nobody has waited for since);
+//     still run (cleared as a whole, on another stream than the launch's that
+//     nobody has waited for since);
 //   * fake_launches, fake_allocated, fake_uploaded: totals.
 #include <cuda_runtime_api.h>
 #include <sys/mman.h>
@@ -139,9 +140,11 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
     *n = 4;
     return cudaSuccess;
 }
-cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long, cudaDriverEntryPointQueryResult*) {
-    *f = nullptr;
-    return cudaErrorNotSupported;
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* result) {
+    *f = reinterpret_cast<void*>(+[]() -> int { return 0; });  // a driver call that succeeds, whatever its arguments
+    *result = cudaDriverEntryPointSuccess;
+    return cudaSuccess;
 }
 
 void** __cudaRegisterFatBinary(void*) { static void* at = nullptr; return &at; }
@@ -164,9 +167,14 @@ cudaError_t __cudaGetKernel(void** kernel, const void* function) {
     *kernel = const_cast<void*>(function);
     return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(void*, dim3, dim3, void**, std::size_t, cudaStream_t) {
+cudaError_t __cudaLaunchKernel(void*, dim3, dim3, void**, std::size_t, cudaStream_t stream) {
     ++launches;
-    if (!clearing.empty()) ++hazards;
+    for (cudaStream_t other : clearing) {
+        if (other != stream) {
+            ++hazards;
+            break;
+        }
+    }
     return cudaSuccess;
 }
 }

@@ -47,3 +47,22 @@ def test_no_launch_while_a_new_buffer_is_cleared(library, formula, flags):
     launches, hazards = map(int, fake_cuda.run(library, CODE.format(direct=ids[formula], flags=flags, formula=formula)).split())
     assert launches > 0
     assert hazards == 0
+
+
+def test_the_cost_network_workspace_is_clear_before_its_first_layer(library):
+    launches, hazards = map(int, fake_cuda.run(library, """
+        lib.fractal_gb300_costnet_create.restype = ctypes.c_void_p
+        lib.fractal_gb300_costnet_predict.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p,
+                                                      ctypes.c_void_p]
+        net = lib.fractal_gb300_costnet_create(7)
+        assert net, native.last_error(lib)
+        stream = lib.fake_stream()
+        rows = (ctypes.c_uint16 * (1024 * 320 + 8))()
+        x = (ctypes.addressof(rows) + 15) // 16 * 16
+        out = (ctypes.c_float * 1024)()
+        for count in (128, 1024):
+            check(lib.fractal_gb300_costnet_predict(net, x, count, ctypes.addressof(out), stream))
+        print(lib.fake_launches(), lib.fake_hazards())
+        """).split())
+    assert launches > 0
+    assert hazards == 0
