@@ -1066,8 +1066,18 @@ __global__ void __launch_bounds__(128, Formula == kFormulaJulia ? 3 : 4) alt_que
                     AltOutcome started = kAltDone;
                     if (base + lane < items) {
                         started = alt_begin<WithPlanes, Formula>(p, static_cast<long long>(base + lane), t);
-                        while (started == kAltContinue && !p.disable_bla && p.alt_index.levels > 1
-                               && !no_block(p, t.ref - p.alt_start, t.delta)) {
+                        while (started == kAltContinue) {
+                            // The first turn and every 16th look at the clock:
+                            // blocks alone may take a pixel to the cap.
+                            if (deadline && (t.ticks++ & 15u) == 0u && t.it < p.max_iter && global_ns() >= deadline) {
+                                alt_store(p, t.index, nan_f(), 0u);
+                                started = kAltDone;
+                                break;
+                            }
+                            if (p.disable_bla || p.alt_index.levels <= 1
+                                || no_block(p, t.ref - p.alt_start, t.delta)) {
+                                break;
+                            }
                             started = alt_general<WithPlanes, Formula>(p, t, max_block);
                         }
                     }
