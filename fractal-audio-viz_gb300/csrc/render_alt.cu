@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "cycle_turn.h"
 #include "device.h"
 #include "int_mul.h"
 
@@ -937,7 +938,7 @@ __device__ __noinline__ AltOutcome alt_general(const AltParams& p, AltLane<WithP
         s.pending = false;
         if (alt_escaped<WithPlanes>(p, s)) return kAltEscaped;
     }
-    if (p.cycle && s.it >= 2048 && (s.it & 31) == 0 && alt_cycle<WithPlanes>(p, s)) {
+    if (cycle_turn(p.cycle != 0, s.it) && alt_cycle<WithPlanes>(p, s)) {
         return alt_interior<WithPlanes>(p, s.index);
     }
     return kAltContinue;
@@ -1074,7 +1075,7 @@ __global__ void __launch_bounds__(128, Formula == kFormulaJulia ? 3 : 4) alt_que
                                 started = kAltDone;
                                 break;
                             }
-                            if (p.disable_bla || p.alt_index.levels <= 1
+                            if (p.disable_bla || p.alt_index.levels <= 1 || !turn_before_listing(p.cycle != 0, t.it)
                                 || no_block(p, t.ref - p.alt_start, t.delta)) {
                                 break;
                             }
