@@ -787,27 +787,19 @@ void* create_handle(const char* x, const char* y, const char* zoom, int max_iter
 }  // namespace
 
 // ---------------------------------------------------------- aurora palette
-// aurora_palette_for / colour_basis_for (renderer.cpp:4788-4923), built on
-// the host exactly as the reference does and cached per thread.
+// aurora_palette_for / colour_basis_for (renderer.cpp:4788-4923): the waves'
+// table on the host, the entries on the device with the reference's operations.
 namespace {
-
-// The aurora waves' cosine / sine table (the part of aurora_palette_for that
-// depends on the iteration cap alone, renderer.cpp:4841-4860) of the calling
-// thread's last cap, on the device.
-struct AuroraWaves {
-    int max_iter = -1;
-    int device = -1;
-    const void* at = nullptr;
-};
 
 // The device palette for the parameters, made on `stream`, which waits for
 // earlier users of the scratch buffers first.
 const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_iter, double phase, double vocal,
                                double pitch, int& size, const std::uint8_t* accents = nullptr) {
-    thread_local AuroraWaves cache;
     size = std::min(65536, std::max(4096, max_iter * 4));
-    auto* waves = static_cast<float2*>(scratch(rt, kScratchWaves, static_cast<std::size_t>(size) * sizeof(float2)));
-    if (cache.max_iter != max_iter || cache.device != rt.device || cache.at != waves) {
+    const std::size_t wave_bytes = static_cast<std::size_t>(size) * sizeof(float2);
+    if (rt.capacity[kScratchWaves] < wave_bytes) rt.waves_iter = -1;  // a new buffer, even where making it fails
+    auto* waves = static_cast<float2*>(scratch(rt, kScratchWaves, wave_bytes));
+    if (rt.waves_iter != max_iter) {
         std::vector<float2> table(static_cast<std::size_t>(size));
         const double denominator = std::max(1, size - 1);
         for (int i = 0; i < size; ++i) {
@@ -815,13 +807,13 @@ const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_i
             table[static_cast<std::size_t>(i)].x = static_cast<float>(std::cos(angle));
             table[static_cast<std::size_t>(i)].y = static_cast<float>(std::sin(angle));
         }
-        cache.max_iter = -1;
+        rt.waves_iter = -1;
         // Earlier frames may still read the previous table.
         wait_scratch(rt, rt.stream);
         check_cuda(cudaMemcpyAsync(waves, table.data(), table.size() * sizeof(float2), cudaMemcpyHostToDevice,
                                    rt.stream), "upload aurora waves");
         check_cuda(cudaStreamSynchronize(rt.stream), "upload aurora waves");
-        cache = AuroraWaves{max_iter, rt.device, waves};
+        rt.waves_iter = max_iter;
     }
     AuroraPalette p{};
     const double mix = std::clamp(vocal, 0.0, 1.0);

@@ -81,6 +81,10 @@ struct ThreadRuntime {
     cudaEvent_t lane_join[kPlainLanes] = {};
     int last_shapes[4] = {};
     int pinned_shapes[4] = {};  // set by fractal_gb300_set_queue_shapes
+    // Cap of the aurora waves' cosine / sine table in kScratchWaves (the part of
+    // aurora_palette_for that depends on it alone, renderer.cpp:4841-4860), or -1.
+    // It lives and dies with the scratch.
+    int waves_iter = -1;
     void* costnet = nullptr;    // attached tile-cost network (not owned)
     cudaStream_t tile_stream = nullptr;  // stream of the last tile-scheduled batch
     cudaStream_t batch_stream = nullptr; // stream of the last keyframe batch
