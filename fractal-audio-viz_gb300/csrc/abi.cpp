@@ -791,6 +791,13 @@ void* create_handle(const char* x, const char* y, const char* zoom, int max_iter
 // table on the host, the entries on the device with the reference's operations.
 namespace {
 
+// Whether calls on `stream` are being recorded into a caller's graph.
+bool recording(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(stream, &status), "cudaStreamIsCapturing");
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // The device palette for the parameters, made on `stream`, which waits for
 // earlier users of the scratch buffers first.
 const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_iter, double phase, double vocal,
@@ -2717,12 +2724,17 @@ int fractal_gb300_colourise_device(const float* field, uint8_t* rgb, int width, 
         }
         ThreadRuntime& rt = thread_runtime();
         cudaStream_t stream = stream_handle ? static_cast<cudaStream_t>(stream_handle) : rt.stream;
+        // A call recorded into a graph makes its palette at once, on the
+        // thread's own stream: an event of work outside the graph cannot be
+        // waited for inside it, and one recorded inside it by no later call.
+        const bool recorded = recording(stream);
         int lut_size = 0;
-        const std::uint8_t* lut = aurora_lut(rt, stream, max_iter, phase, vocal, pitch, lut_size);
+        const std::uint8_t* lut = aurora_lut(rt, recorded ? rt.stream : stream, max_iter, phase, vocal, pitch, lut_size);
+        if (recorded) check_cuda(cudaStreamSynchronize(rt.stream), "aurora palette");
         const float scale = static_cast<float>(lut_size - 1) / static_cast<float>(max_iter);
         check_cuda(launch_aurora(field, rgb, static_cast<long long>(width) * height, lut, lut_size, scale, max_iter,
                                  stream), "aurora kernel launch");
-        release_scratch(rt, stream);
+        if (!recorded) release_scratch(rt, stream);
     });
 }
 
