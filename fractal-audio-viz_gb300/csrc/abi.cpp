@@ -799,10 +799,18 @@ bool recording(cudaStream_t stream) {
 }
 
 // The device palette for the parameters, made on `stream`, which waits for
-// earlier users of the scratch buffers first.
+// earlier users of the scratch buffers first.  The last one is kept: a frame
+// whose controls did not change pays neither the launch nor its 7 us.
 const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_iter, double phase, double vocal,
                                double pitch, int& size, const std::uint8_t* accents = nullptr) {
     size = std::min(65536, std::max(4096, max_iter * 4));
+    PaletteKey key{max_iter, phase, vocal, pitch, accents != nullptr, {}};
+    if (accents != nullptr) std::copy(accents, accents + 9, key.accents.begin());
+    if (rt.palette == key) {
+        wait_scratch(rt, stream);
+        return static_cast<const std::uint8_t*>(rt.scratch[kScratchLut]);
+    }
+    rt.palette = PaletteKey{};
     const std::size_t wave_bytes = static_cast<std::size_t>(size) * sizeof(float2);
     if (rt.capacity[kScratchWaves] < wave_bytes) rt.waves_iter = -1;  // a new buffer, even where making it fails
     auto* waves = static_cast<float2*>(scratch(rt, kScratchWaves, wave_bytes));
@@ -842,6 +850,9 @@ const std::uint8_t* aurora_lut(ThreadRuntime& rt, cudaStream_t stream, int max_i
     auto* lut = static_cast<std::uint8_t*>(scratch(rt, kScratchLut, static_cast<std::size_t>(size) * 3));
     wait_scratch(rt, stream);
     check_cuda(launch_aurora_lut(waves, size, p, lut, stream), "aurora palette launch");
+    // A later call with the same controls may come on another stream.
+    release_scratch(rt, stream);
+    rt.palette = key;
     return lut;
 }
 

@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstddef>
 #include <cstdint>
 #include <map>
@@ -51,6 +52,18 @@ enum ScratchSlot {
     kScratchCount
 };
 
+// What an aurora palette's entries depend on.
+struct PaletteKey {
+    int max_iter = -1;  // -1: none
+    double phase = 0, vocal = 0, pitch = 0;
+    bool accented = false;
+    std::array<std::uint8_t, 9> accents{};
+    bool operator==(const PaletteKey& o) const {
+        return max_iter == o.max_iter && phase == o.phase && vocal == o.vocal && pitch == o.pitch
+            && accented == o.accented && accents == o.accents;
+    }
+};
+
 struct ThreadRuntime {
     int device = -1;
     cudaStream_t stream = nullptr;
@@ -85,6 +98,7 @@ struct ThreadRuntime {
     // aurora_palette_for that depends on it alone, renderer.cpp:4841-4860), or -1.
     // It lives and dies with the scratch.
     int waves_iter = -1;
+    PaletteKey palette;  // of the entries in kScratchLut
     void* costnet = nullptr;    // attached tile-cost network (not owned)
     cudaStream_t tile_stream = nullptr;  // stream of the last tile-scheduled batch
     cudaStream_t batch_stream = nullptr; // stream of the last keyframe batch
