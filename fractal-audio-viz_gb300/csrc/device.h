@@ -495,7 +495,7 @@ enum DirectCounter {
     kSpillTaken = kSpillMade + 4,   // per launch: and by consumers
     kGeneration = kSpillTaken + 4,  // batch generation (not reset; bumped per batch)
 };
-constexpr int kDirectLaunches = 4;  // one for fresh pixels, three for spilled ones
+constexpr int kDirectLaunches = 4;  // at most: one for fresh pixels, three for spilled ones
 struct DirectBatch {
     DirectParams field[kMaxDirectFields];
     long long first[kMaxDirectFields + 1];  // pixel prefix over the batch
@@ -508,6 +508,7 @@ struct DirectBatch {
     // A fresh pixel still running after `budget` steps is spilled (when the
     // list has room); the launches that follow take the list 32 to a warp.
     int budget;
+    int launches;                           // 1 to kDirectLaunches
     int steps;                              // steps between refills (fresh pixels)
     int long_steps;                         // steps between refills (spilled pixels)
     int fast_smooth;                        // smooth value in FP32 (floatexp form's direct levels)

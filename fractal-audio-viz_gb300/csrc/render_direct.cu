@@ -530,6 +530,7 @@ constexpr int kRefill = 8;                // idle lanes before a resuming warp t
 constexpr int kLeave = 20;                // active lanes below which it gives its pixels back ...
 constexpr int kPatience = 16;             // ... after so many rounds,
 constexpr int kShortList = 32 * 4 * 152;  // unless the list gives a warp to each sub-partition at most
+constexpr long long kOneResume = 65536;   // pixels of a batch up to which one launch resumes
 constexpr int kResumeBlocks = 2;          // per SM: two warps for each sub-partition
 
 template <int Formula, bool Planes, bool Resume, bool Integer>
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const
         }
         const unsigned long long rank = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
         if (rank >= (items + 31) / 32) return;
-        leave = launch + 1 < kDirectLaunches && items > kShortList ? kLeave : 0;
+        leave = launch + 1 < b.launches && items > kShortList ? kLeave : 0;
     }
     WarpQueue q{0, 0, 0, 0, 0, false};
     bool active = false;
@@ -830,11 +831,7 @@ cudaError_t launch_queue(const DirectBatch& b, int sms, int blocks_per_sm, cudaS
     if (grid < 1) grid = 1;
     direct_queue_kernel<Formula, Planes, false, Integer><<<static_cast<unsigned>(grid), 128, 0, s>>>(b, 0);
     const long long resume = std::min<long long>(static_cast<long long>(sms) * kResumeBlocks, needed);
-    // No lane leaves a list of at most kShortList, so a small batch's second
-    // and third resuming launches would find nothing: 160x90 at 1e3 took 66 us
-    // with them.
-    const int launches = b.spill_capacity <= 0 ? 1 : (pixels > kShortList ? kDirectLaunches : 2);
-    for (int launch = 1; launch < launches; ++launch) {
+    for (int launch = 1; launch < b.launches; ++launch) {
         direct_queue_kernel<Formula, Planes, true, Integer><<<static_cast<unsigned>(resume), 128, 0, s>>>(b, launch);
     }
     return cudaGetLastError();
@@ -1008,6 +1005,20 @@ static bool view_meets_interior(const DirectParams& p) {
     return cardioid || bulb;
 }
 
+// Launches of a batch: one for fresh pixels and up to three for spilled ones.
+// None of those finds anything where no cap exceeds the budget, and each costs
+// 2 to 4 us: 256x144 at 1e3, where nothing spills, took 64 us with three, 55
+// with one.  One also does for small batches whose pixels do spill: it keeps
+// every lane and refills from the list, and up to kOneResume pixels that is
+// within two refills of its 38,912 lanes.
+static int direct_launches(const DirectBatch& b, long long pixels) {
+    if (b.spill_capacity <= 0) return 1;
+    int longest = 0;
+    for (int f = 0; f < b.count; ++f) longest = std::max(longest, b.field[f].max_iter);
+    if (longest <= b.budget) return 1;
+    return pixels > kOneResume ? kDirectLaunches : 2;
+}
+
 namespace {
 constexpr int kDefaultSpinLimit = 1 << 22;
 thread_local int fault_spin_limit = kDefaultSpinLimit;
@@ -1049,6 +1060,7 @@ cudaError_t launch_direct_batch(const DirectParams* fields, int count, void* scr
         b.spill_capacity = spill_entries;
         b.budget = 256;
     }
+    b.launches = direct_launches(b, pixels);
     b.steps = shape.steps > 0 ? shape.steps : 2;
     b.long_steps = 16;
     int device = 0, sms = 152;
