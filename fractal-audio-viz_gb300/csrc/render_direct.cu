@@ -212,6 +212,40 @@ __device__ __forceinline__ int budget_stop(const DirectBatch& b, int max_iter) {
     return b.budget < max_iter ? b.budget : max_iter;
 }
 
+// direct_run for an orbit on the real axis (a row of every view centred there
+// with an odd height, the period-2 point of a Julia set with a real constant):
+// one square and one sum a step.  The imaginary part stays a zero, negative
+// where the cross term and the parameter's zero both are.  As general steps,
+// one a round, these pixels held up a 400x225 whole-set view: 6.5 ms, 3.0 ms
+// here.
+template <int Formula>
+__device__ __forceinline__ int direct_run_real(Lane& l, int room, unsigned saved, unsigned mark) {
+    const unsigned long long r2 = dbits(l.escape2);
+    const int added = hi_of(l.pi);
+    double zr = l.zr, rs = l.rs;
+    int sign = hi_of(l.zi);
+    int k = 0;
+#pragma unroll 1
+    for (; k < room; ++k) {
+        const double nr = rs + l.pr;
+        const int hr = hi_of(nr) & 0x7fffffff;
+        const double nrs = int_mul_even(factor_a(nr), factor_b(nr));
+        if (hr < (523 << 20) || hr >= (1523 << 20) || lo_of(nr) == saved || lo_of(nr) == mark || dbits(nrs) > r2) break;
+        int cross = sign ^ hi_of(zr);
+        if constexpr (Formula == kFormulaBurningShip) cross = 0;
+        if constexpr (Formula == kFormulaTricorn) cross = ~cross;
+        sign = cross & added;
+        zr = nr;
+        rs = nrs;
+    }
+    l.zr = zr;
+    l.zi = from_hilo(sign & static_cast<int>(0x80000000u), 0);
+    l.rs = rs;
+    l.is = 0.0;
+    l.it += k;
+    return k;
+}
+
 // Up to `limit` steps of a spilled pixel on the integer and FP64 pipes, each
 // with its tests on single words: it stops before a step that escapes, may
 // close a cycle or moves the cycle marks (multiples of 64; spilled pixels are
@@ -222,10 +256,12 @@ __device__ __forceinline__ int budget_stop(const DirectBatch& b, int max_iter) {
 template <int Formula>
 __device__ __forceinline__ int direct_run(Lane& l, int limit) {
     const int room = min(min(limit, l.max_iter - 1 - l.it), 63 - (l.it & 63));
-    if (room <= 0 || !product_range(l.zr) || !product_range(l.zi)) return 0;
-    const int bound = hi_of(l.escape2) - (1 << 20);  // both squares below R^2 / 2 cannot escape
+    if (room <= 0 || !product_range(l.zr)) return 0;
     const unsigned saved = lo_of(__longlong_as_double(static_cast<long long>(l.saved_r)));
     const unsigned mark = lo_of(__longlong_as_double(static_cast<long long>(l.mark_r)));
+    if (is_zero(l.zi) && is_zero(l.pi)) return direct_run_real<Formula>(l, room, saved, mark);
+    if (!product_range(l.zi)) return 0;
+    const int bound = hi_of(l.escape2) - (1 << 20);  // both squares below R^2 / 2 cannot escape
     double zr = l.zr, zi = l.zi, rs = l.rs, is = l.is;
     FactorA fr = factor_a(zr);
     FactorB gi = factor_b(zi);
