@@ -315,6 +315,7 @@ void launch_deep_mandelbrot(ReferenceContext& ctx, DeviceTables& dev, const Outp
     p.allow_recovery = o.allow_recovery;
     p.strict_cycle = o.strict_cycle;
     p.cycle = cycle ? 1 : 0;
+    p.axis = dev.axis;
     p.escape_mode = o.escape_radius_mode;
     p.max_bla_len = std::clamp(std::min(series_block, static_cast<int>(o.max_bla_length)), 2, kMaxSafeBlaLength);
     p.max_lin_len = std::clamp(std::min(series_block, static_cast<int>(o.max_linear_bla_length)), 2,

@@ -81,6 +81,7 @@ struct DeviceTables {
     AltStep* alt = nullptr;
     LevelIndex alt_index;
     int block_top = 0;  // see AltParams
+    int axis = 0;       // Z_1, the centre, has one part zero (kRawZero)
     fx::Sc* series = nullptr;
     int series_terms = 0;
     // floatexp mirrors (built on the first floatexp render)
@@ -123,6 +124,7 @@ struct PlainParams {
     int allow_recovery;
     int strict_cycle;
     int cycle;  // Brent cycle detection (non-strict or strict_cycle renders)
+    int axis;   // the reference lies on an axis (DeviceTables)
     int escape_mode;
     int max_bla_len;
     int max_lin_len;

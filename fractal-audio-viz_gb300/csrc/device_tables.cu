@@ -195,6 +195,7 @@ std::shared_ptr<DeviceTables> device_tables(ReferenceContext& ctx) {
         const std::vector<OrbitRec> records = make_orbit_records(ctx);
         t.orbit = upload(records);
         t.orbit_size = static_cast<int>(records.size());
+        t.axis = records.size() > 1 && (records[1].raw & kRawZero) != 0 ? 1 : 0;
         // A 2x2 block's radius is at most that of its first step, the
         // tolerance times max(|Z|, 1) (or less): merging only shrinks it.
         int top = 0;

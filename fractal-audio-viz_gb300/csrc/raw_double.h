@@ -77,6 +77,8 @@ FX_HD bool folds(double z, double d) {
         && (bits_of(d) & magnitude) >= (bits_of(z) & magnitude) + (hi_of(z) >= 0 ? 1u : 0u);
 }
 
+FX_HD double twice_raw(double v) { return is_zero(v) ? v : add_exp(v, 1); }
+
 FX_HD double flip(double v, bool negate) {
     return from_hilo(hi_of(v) ^ (negate ? static_cast<int>(0x80000000u) : 0), lo_of(v));
 }

@@ -928,9 +928,10 @@ std::vector<OrbitRec> make_orbit_records(const ReferenceContext& ctx) {
         r.zd_im = orbit.im_d[i];
         r.zf_re = static_cast<float>(fx::sc_re_d(r.z));
         r.zf_im = static_cast<float>(fx::sc_im_d(r.z));
-        const bool raw = fx::raw_value(fx::sc_make(fx::sc_re_d(r.z), fx::sc_im_d(r.z), 0))
-            && r.zd_re == fx::sc_re_d(r.z) && r.zd_im == fx::sc_im_d(r.z);
-        r.raw = raw ? kRawOrbit : 0;
+        const double z[2] = {fx::sc_re_d(r.z), fx::sc_im_d(r.z)};
+        const auto fits_part = [](double v) { return fx::raw_part(v) || fx::bits_of(v) == 0; };
+        const bool raw = r.zd_re == z[0] && r.zd_im == z[1] && fits_part(z[0]) && fits_part(z[1]);
+        r.raw = !raw ? 0 : (fx::raw_part(z[0]) && fx::raw_part(z[1]) ? kRawOrbit : kRawZero);
         r.top = fx::imax(fx::bexp(r.zd_re), fx::bexp(r.zd_im));
         r.parts = fx::sc_to_fec(orbit.scaled[i]);
         // Mandelbrot rebuilds the escape margin from the compact orbit

@@ -61,7 +61,7 @@ struct alignas(128) OrbitRec {
     double zd_im;
     float zf_re;       // Z_i rounded to float: the estimates that settle a
     float zf_im;       // test far from its bound without FP64
-    int raw;           // kRawOrbit, kRawFold (raw_double.h)
+    int raw;           // kRawOrbit, kRawZero, kRawFold (raw_double.h)
     int top;           // biased exponent of the larger part of Z_i
     fx::Sc z;          // compact orbit value Z_i
     fx::Fec parts;     // Z_i components as FloatExp (escape margin input)
@@ -72,7 +72,8 @@ struct alignas(128) OrbitRec {
     };
 };
 constexpr int kRawOrbit = 1;  // both parts of Z_i in the raw range
-constexpr int kRawFold = 2;   // and of the fold constant, or zero
+constexpr int kRawZero = 4;   // each in the raw range or +0, but not both in it
+constexpr int kRawFold = 2;   // either, and the parts of the fold constant in the range or zero
 static_assert(sizeof(OrbitRec) == 128, "one record per cache line");
 
 struct OrbitData {

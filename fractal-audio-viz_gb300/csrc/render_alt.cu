@@ -291,8 +291,6 @@ __device__ __forceinline__ bool jac_part(double v) {
     return static_cast<unsigned>(bexp(v) - kRawLow) <= kJacSpan || is_zero(v);
 }
 
-__device__ __forceinline__ double twice_raw(double v) { return is_zero(v) ? v : add_exp(v, 1); }
-
 // jac_step on the values themselves: total raw (a part may have cancelled to
 // zero), entries on one exponent k.  The parameter plane's +1 is 2^-k in the
 // entries' unit; below 2^-600 of it, it cannot move a sum that is above
@@ -342,7 +340,7 @@ __device__ __forceinline__ bool jac_step_raw(const Sc& total, RawJac& j) {
 template <int Formula>
 __device__ __forceinline__ Sc alt_step_raw(const double2& z, const Sc& d, const Sc& pd, bool fold, const Sc& total,
                                            const double2& constant) {
-    const double z2r = add_exp(z.x, 1), z2i = add_exp(z.y, 1);
+    const double z2r = twice_raw(z.x), z2i = twice_raw(z.y);
     double lr = z2r * d.re - z2i * d.im;
     double li = z2r * d.im + z2i * d.re;
     if constexpr (Formula == kFormulaBurningShip) {
@@ -612,7 +610,8 @@ __device__ __forceinline__ int high(double v) { return hi_of(v) & 0x7fffffff; }
 // test on high words: nonzero parts in range, no block as large as the
 // delta, and exponents near enough that no shared-exponent sum drops an
 // operand (2 Z d and d^2 differ by the exponents of 2 Z and d, to within 4).
-// The other steps on raw values take the longer form.
+// The other steps on raw values take the longer form, among them every step
+// of a reference on an axis, whose orbit has zero parts.
 template <bool WithPlanes, int Formula>
 __device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlanes>& s, int limit) {
     const Sc pd = s.pd;
@@ -643,10 +642,10 @@ __device__ __forceinline__ int alt_raw_run(const AltParams& p, AltLane<WithPlane
 #pragma unroll 1
     while (k < room) {
         const int flags = head.z;
-        if (!(flags & kRawOrbit)) break;
+        if (!(flags & (kRawOrbit | kRawZero))) break;
         const int dr = high(d.re), di = high(d.im);
         const int most = imax(dr, di), top = most >> 20;
-        bool plain = imin(dr, di) >= kHighLow && most <= kHighTop && 2 * (top - 1023) >= block_top
+        bool plain = (flags & kRawOrbit) && imin(dr, di) >= kHighLow && most <= kHighTop && 2 * (top - 1023) >= block_top
             && static_cast<unsigned>(head.w + 1 - top + 55) <= 110u;
         if constexpr (WithPlanes) {
             const int a = high(j.xa), b = high(j.xb), c = high(j.ya), e = high(j.yb);

@@ -466,7 +466,12 @@ struct Tail {
 // from FP32 to 2^-17 of the larger: R^2 is passed only above (1 - 2^-14) R^2
 // or with |d| > 4 R, and one is the smaller for certain when the estimates
 // differ by 2^-8 (the larger not below 2^-100).
-template <bool Planes>
+//
+// `Axis`: the reference lies on an axis and its orbit has zero parts, which
+// the integer products do not take; its products with Z run in FP64.  A kernel
+// of its own: a branch in the usual loop cost it 1 %, a second loop beside it
+// 1 to 3 %.
+template <bool Planes, bool Axis>
 __device__ __forceinline__ int tail_run(const PlainParams& p, double dc_re, double dc_im, int room, Tail<Planes>& t,
                                         bool& open) {
     constexpr int kMaxRebases = 64;
@@ -484,7 +489,7 @@ __device__ __forceinline__ int tail_run(const PlainParams& p, double dc_re, doub
     }
     while (made < room && at + 1 < p.orbit_size) {
         const bool origin = is_zero(z.x) && is_zero(z.y);  // after a rebase
-        if (!origin && !(head.z & kRawOrbit)) break;
+        if (!origin && !(head.z & (Axis ? kRawOrbit | kRawZero : kRawOrbit))) break;
         const int hr = high(dr), hi = high(di);
         if (imin(hr, hi) < kHighLow || imax(hr, hi) > kHighTop) break;
         const OrbitRec* const next = p.orbit + at + 1;
@@ -495,13 +500,22 @@ __device__ __forceinline__ int tail_run(const PlainParams& p, double dc_re, doub
             if (!derivative_run(total_re, total_im, t.derivative, derivative)) break;
         }
         const FactorA fr = factor_a(dr), fi = factor_a(di);
-        const FactorB zr = factor_b(add_exp(z.x, 1)), zi = factor_b(add_exp(z.y, 1));
-        const double rr = int_mul_even(fr, zr), ii = int_mul_even(fi, zi);
-        const double ri = int_mul_even(fi, zr), ir = int_mul_even(fr, zi);
+        double lr, li;
+        if constexpr (Axis) {
+            const double z2r = twice_raw(z.x), z2i = twice_raw(z.y);
+            lr = z2r * dr - z2i * di;
+            li = z2r * di + z2i * dr;
+        } else {
+            const FactorB zr = factor_b(add_exp(z.x, 1)), zi = factor_b(add_exp(z.y, 1));
+            const double rr = int_mul_even(fr, zr), ii = int_mul_even(fi, zi);
+            const double ri = int_mul_even(fi, zr), ir = int_mul_even(fr, zi);
+            lr = rr - ii;
+            li = ri + ir;
+        }
         const FactorB gr = factor_b(dr), gi = factor_b(di);
         const double uu = int_mul_even(fr, gr), vv = int_mul_even(fi, gi), uv = int_mul_even(fr, gi);
         const double sr = uu - vv, si = add_exp(uv, 1);
-        double xr = (rr - ii) + sr, xi = (ri + ir) + si;
+        double xr = lr + sr, xi = li + si;
         xr = choose(origin, sr, xr);
         xi = choose(origin, si, xi);
         // dc does not move a sum 60 binades above it.
@@ -561,7 +575,7 @@ __device__ __forceinline__ int tail_run(const PlainParams& p, double dc_re, doub
 
 // render_scaled_double_tail (renderer.cpp:12451-12669). Returns kExitTail,
 // with |Z + d|^2 in `exit_mag2`, for a value that the caller finishes.
-template <bool Planes, bool Stats>
+template <bool Planes, bool Stats, bool Axis>
 __device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitView& orbit, long long index, const Sc& dc,
                             int& iteration, int& ref, const Sc& delta_in, Sc& derivative,
                             const Nrm& initial_norm, StatSink<Stats>& st, unsigned& ticks,
@@ -601,7 +615,7 @@ __device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitVie
         if (deadline_ns) room = imin(room, 256 - static_cast<int>(ticks & 255U));
         bool open = false;
         const int moved = t.rebases;
-        const int made = tail_run<Planes>(p, dc_re, dc_im, room, t, open);
+        const int made = tail_run<Planes, Axis>(p, dc_re, dc_im, room, t, open);
         st.add(kTailRebases, static_cast<unsigned long long>(t.rebases - moved));
         if (made > 0) {
             ticks += static_cast<unsigned>(made);
@@ -739,7 +753,7 @@ __device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitVie
 // pixels repeat a rebase (1.73 ms).  Blocks of 64 threads and the larger
 // operations out of line were 2 to 8 % slower, integer products in the general
 // operations too 7 %.
-template <bool Planes, bool Stats>
+template <bool Planes, bool Stats, bool Axis>
 __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams p) {
     const long long total_pixels = static_cast<long long>(p.width) * p.height;
     const long long index = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -924,7 +938,7 @@ __global__ void __launch_bounds__(128) plain_mandelbrot_kernel(const PlainParams
         if (bla_allowed && (map_length <= 0 || ref + map_length > p.max_iter) && delta_norm.e > -90) {
             st.add(kDoubleTailPixels);
             const int tail_start = iteration;
-            exit = double_tail<Planes, Stats>(p, orbit, index, dc, iteration, ref, delta, derivative, total_norm, st,
+            exit = double_tail<Planes, Stats, Axis>(p, orbit, index, dc, iteration, ref, delta, derivative, total_norm, st,
                                               ticks, deadline_ns, out_value, out_count, timed_out, unresolved,
                                               planes, exit_mag2, exit_total, exit_previous);
             if (timed_out || unresolved) break;
@@ -1096,7 +1110,11 @@ cudaError_t launch_plain_variant(const PlainParams& p, cudaStream_t stream) {
     const long long pixels = static_cast<long long>(p.width) * p.height;
     const dim3 block(128);
     const dim3 grid(static_cast<unsigned>((pixels + 127) / 128));
-    plain::plain_mandelbrot_kernel<Planes, Stats><<<grid, block, 0, stream>>>(p);
+    if (p.axis) {
+        plain::plain_mandelbrot_kernel<Planes, Stats, true><<<grid, block, 0, stream>>>(p);
+    } else {
+        plain::plain_mandelbrot_kernel<Planes, Stats, false><<<grid, block, 0, stream>>>(p);
+    }
     return cudaGetLastError();
 }
 
