@@ -980,7 +980,7 @@ constexpr int kAltLeave = 20;
 constexpr int kAltPatience = 24;  // rounds: 384 steps
 constexpr int kAltShort = 32 * 4 * 152;      // pixels: one full warp per SM sub-partition
 constexpr int kAltBusyWarps = 8 * 152;       // warps that keep the FP64 pipe busy
-constexpr long long kAltPhasePixels = 16384; // smaller fields run in one launch
+constexpr long long kAltPhasePixels = 131072; // smaller fields run in one launch (alt_launch)
 
 // Registers: the parameter-plane formulas, whose general turns wait for
 // instructions, gain from four blocks (1280x720 with planes: 10.0 against
@@ -1157,6 +1157,13 @@ int alt_queue_blocks() {
 
 // The launches of one field: `queue.counters` holds the claim counters and
 // spill counts (kAltQueueCounters words), `queue.spill` two lists.
+//
+// Up to kAltPhasePixels one launch does everything.  The later ones cost 4 us
+// each, which a field of short orbits does not get back (400x225 at 1e12: 95
+// us with eight, 66 with one, 84 as one thread per pixel), and a field of long
+// ones has little to regroup while the first launch's lanes (77,824) hold most
+// of its pixels: 320x180 at 1e24 took 3.6 ms with eight and 2.3 with one for
+// one Julia set, with planes 2.9 and 3.9 for another.
 template <bool WithPlanes, int Formula>
 cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t stream) {
     const long long pixels = static_cast<long long>(p.width) * p.height;

@@ -3,7 +3,7 @@
 On the CPU: a pixel that runs ahead of its lane (csrc/cycle_turn.h) never
 makes a step that a cycle test follows, whatever mixture of blocks and single
 steps it takes, since the list it waits on keeps no cycle state.  On the GPU:
-fields above one launch's 16,384 pixels, with interior regions and caps well
+fields above one launch's 131,072 pixels, with interior regions and caps well
 above the first cycle test, equal the same fields without cycle tests (an
 interior pixel is at the cap either way, and no view here has an orbit that
 stays within the test's 2^-39 and escapes later).
@@ -65,7 +65,7 @@ def test_no_cycle_state_begins_before_a_pixel_is_listed(tmp_path):
     ("tricorn", "-0.1", "0.05", b"1e6", ("0", "0")), ("julia", "0.1", "0.1", b"1e6", ("-0.12", "0.74"))])
 def test_cycle_tests_change_no_value(package, product, formula, x, y, zoom, julia, planes):
     native = package.native
-    width, height, cap = 200, 112, 6000
+    width, height, cap = 512, 260, 6000
     fields = []
     for off in (0, 1):
         options = native.RenderOptions(strict=0, disable_cycle=off)
