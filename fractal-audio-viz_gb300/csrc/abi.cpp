@@ -344,9 +344,11 @@ void launch_deep_mandelbrot(ReferenceContext& ctx, DeviceTables& dev, const Outp
                "plain Mandelbrot kernel launch");
 }
 
-// Counters and spill lists of the alternate-formula queue: one slot per lane
-// stream of a batch, and one (the last) for single renders.  A list holds up
-// to 262,144 pixels of 128 bytes: more than the lanes of a launch.
+// Counters and lists of the alternate-formula queue: counters for each lane
+// stream of a batch and (the last) for single renders, lists for each lane
+// that carries such fields.  A slot's lists take 87 MB for a field above
+// 262,144 pixels (two spill lists of 2^18 entries of 128 bytes, and 64 entries
+// for each warp of the launch), the warps' entries alone up to 131,072 pixels.
 constexpr int kAltQueueSlots = ThreadRuntime::kPlainLanes + 1;
 constexpr std::size_t kAltQueueStride = 256;
 static_assert(kAltQueueCounters * sizeof(unsigned long long) <= kAltQueueStride, "one slot");
@@ -362,8 +364,8 @@ struct AltQueues {
 AltQueues alt_queues(ThreadRuntime& rt, long long pixels, int slots) {
     AltQueues q;
     q.counters = static_cast<char*>(scratch(rt, kScratchAltQueue, kAltQueueSlots * kAltQueueStride));
-    q.capacity = std::min<long long>(pixels, 1ll << 18);
-    q.slot_bytes = 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes() + alt_ready_bytes();
+    q.capacity = alt_spill_capacity(pixels);
+    q.slot_bytes = 2 * static_cast<std::size_t>(q.capacity) * alt_spill_entry_bytes() + alt_ready_bytes(pixels);
     q.slot_bytes = (q.slot_bytes + 255) / 256 * 256;
     q.spill = static_cast<char*>(scratch(rt, kScratchAltSpill, slots * q.slot_bytes));
     return q;
@@ -1542,7 +1544,8 @@ struct BatchPlan {
     // Plain-form launches: (stream, the alternate queue's claim counter for
     // that stream).
     std::vector<std::function<void(cudaStream_t, const AltQueue&)>> plain;
-    long long alternate_pixels = 0;  // of the largest alternate-formula field among them
+    std::vector<char> alternate;     // whether each is an alternate-formula field
+    long long alternate_pixels = 0;  // of the largest of those
     // A time budget stamps its origin per launch in one per-thread word, so
     // budgeted plain launches stay one after another on one stream.
     bool serial_plain = false;
@@ -1593,6 +1596,18 @@ TileBuffers tile_buffers(char* base, int tiles, int rows) {
 int plain_lanes(const BatchPlan& plan) {
     return plan.plain.size() > 1 && !plan.serial_plain
         ? static_cast<int>(std::min<std::size_t>(ThreadRuntime::kPlainLanes, plan.plain.size())) : 0;
+}
+
+// Lists for alternate-formula fields: one for each lane that carries any.
+int alternate_slots(const BatchPlan& plan, std::array<int, ThreadRuntime::kPlainLanes>& list) {
+    const int lanes = std::max(1, plain_lanes(plan));
+    int slots = 0;
+    list.fill(-1);
+    for (std::size_t i = 0; i < plan.plain.size(); ++i) {
+        int& mine = list[i % static_cast<std::size_t>(lanes)];
+        if (plan.alternate[i] && mine < 0) mine = slots++;
+    }
+    return slots;
 }
 
 void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRuntime& rt, cudaStream_t main,
@@ -1662,16 +1677,20 @@ void enqueue_batch(const BatchPlan& plan, const BatchShapes& shapes, ThreadRunti
         }
     }
     if (lanes > 0) {
+        std::array<int, ThreadRuntime::kPlainLanes> list;
+        alternate_slots(plan, list);
         for (std::size_t i = 0; i < plan.plain.size(); ++i) {
             const int lane = static_cast<int>(i % lanes);
-            plan.plain[i](rt.lanes[lane], alt_queue_slot(alternates, lane, lane));
+            plan.plain[i](rt.lanes[lane], plan.alternate[i] ? alt_queue_slot(alternates, lane, list[lane]) : AltQueue{});
         }
         for (int l = 0; l < lanes; ++l) {
             check_cuda(cudaEventRecord(rt.lane_join[l], rt.lanes[l]), "cudaEventRecord (lane join)");
             check_cuda(cudaStreamWaitEvent(main, rt.lane_join[l], 0), "cudaStreamWaitEvent (lane join)");
         }
     } else {
-        for (const auto& launch : plan.plain) launch(plain_stream, alt_queue_slot(alternates, 0, 0));
+        for (std::size_t i = 0; i < plan.plain.size(); ++i) {
+            plan.plain[i](plain_stream, plan.alternate[i] ? alt_queue_slot(alternates, 0, 0) : AltQueue{});
+        }
     }
     if (fork) {
         check_cuda(cudaEventRecord(rt.join, rt.side), "cudaEventRecord (join)");
@@ -1684,7 +1703,10 @@ void launch_plan(const BatchPlan& plan, const BatchShapes& shapes, ThreadRuntime
     void* direct_scratch = plan.direct.empty() ? nullptr : scratch(rt, kScratchDirect, plan.direct_bytes);
     auto* counter = static_cast<unsigned long long*>(scratch(rt, kScratchQueue, 256));
     AltQueues alternates;
-    if (plan.alternate_pixels > 0) alternates = alt_queues(rt, plan.alternate_pixels, std::max(1, plain_lanes(plan)));
+    if (plan.alternate_pixels > 0) {
+        std::array<int, ThreadRuntime::kPlainLanes> list;
+        alternates = alt_queues(rt, plan.alternate_pixels, alternate_slots(plan, list));
+    }
     if (!graph) {
         enqueue_batch(plan, shapes, rt, stream, direct_scratch, counter, alternates);
         return;
@@ -1999,6 +2021,7 @@ void render_field_batch(const std::vector<FieldRequest>& fields, const char* x_c
                                        series_block, o, false, rt, s);
             }
         });
+        plan.alternate.push_back(raw->formula != kFormulaMandelbrot);
         if (raw->formula != kFormulaMandelbrot) {
             plan.alternate_pixels = std::max(plan.alternate_pixels, static_cast<long long>(width) * height);
         }

@@ -464,8 +464,8 @@ void render_floatexp_from_reference(ReferenceContext& ctx, const Outputs& out, i
 cudaError_t launch_plain_mandelbrot(const PlainParams& params, bool planes, bool stats, cudaStream_t stream);
 // Device memory of one alternate-formula render, which no other launch uses
 // at the same time: kAltQueueCounters words, two spill lists of `capacity`
-// entries each (alt_spill_entry_bytes) and the warps' lists of started pixels
-// (alt_ready_bytes).
+// entries each (alt_spill_capacity, alt_spill_entry_bytes) and the warps' lists
+// of started pixels (alt_ready_bytes), for a field of up to so many pixels.
 constexpr int kAltQueueCounters = 16;
 struct AltQueue {
     unsigned long long* counters;
@@ -473,7 +473,8 @@ struct AltQueue {
     long long capacity;
     void* ready;
 };
-std::size_t alt_ready_bytes();
+long long alt_spill_capacity(long long pixels);
+std::size_t alt_ready_bytes(long long pixels);
 std::size_t alt_spill_entry_bytes();
 cudaError_t launch_plain_alternate(const AltParams& params, bool planes, const AltQueue& queue, cudaStream_t stream);
 // A batch of direct fields (one kernel over all of them); the batch struct

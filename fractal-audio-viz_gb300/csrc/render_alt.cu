@@ -1191,13 +1191,18 @@ cudaError_t alt_launch(const AltParams& p, const AltQueue& queue, cudaStream_t s
 
 std::size_t alt_spill_entry_bytes() { return sizeof(AltSaved); }
 
-// One list of kAltPark pixels per warp of the largest grid.
-std::size_t alt_ready_bytes() {
-    const int blocks = std::max({alt_queue_blocks<true, kFormulaJulia>(), alt_queue_blocks<false, kFormulaJulia>(),
+// More entries than the lanes of a launch; none where one launch does.
+long long alt_spill_capacity(long long pixels) {
+    return pixels > kAltPhasePixels ? std::min<long long>(pixels, 1ll << 18) : 0;
+}
+
+// One list of kAltPark pixels per warp of the largest grid for the field.
+std::size_t alt_ready_bytes(long long pixels) {
+    const long long blocks = std::max({alt_queue_blocks<true, kFormulaJulia>(), alt_queue_blocks<false, kFormulaJulia>(),
                                  alt_queue_blocks<true, kFormulaBurningShip>(),
                                  alt_queue_blocks<false, kFormulaBurningShip>(),
                                  alt_queue_blocks<true, kFormulaTricorn>(), alt_queue_blocks<false, kFormulaTricorn>()});
-    return static_cast<std::size_t>(blocks) * 4 * kAltPark * sizeof(AltSaved);
+    return static_cast<std::size_t>(std::min(blocks, (pixels + 127) / 128)) * 4 * kAltPark * sizeof(AltSaved);
 }
 
 cudaError_t launch_plain_alternate(const AltParams& p, bool planes, const AltQueue& queue, cudaStream_t stream) {
