@@ -481,8 +481,8 @@ cudaError_t launch_plain_alternate(const AltParams& params, bool planes, const A
 // travels as a __grid_constant__ kernel parameter.
 constexpr int kMaxDirectFields = 64;
 // A pixel that ran past its iteration budget, parked with its whole state
-// so that the next launch resumes it bit for bit; `ready` carries the batch's
-// generation once the entry is written.
+// so that the next launch resumes it bit for bit; `ready` carries the mark of
+// the batch and launch (spill_mark) once the entry is written.
 struct alignas(128) DirectSpill {
     double zr, zi, dr, di, test1, test2;
     unsigned long long saved_r, saved_i, mark_r, mark_i;
@@ -499,6 +499,10 @@ enum DirectCounter {
     kGeneration = kSpillTaken + 4,  // batch generation (not reset; bumped per batch)
 };
 constexpr int kDirectLaunches = 4;  // at most: one for fresh pixels, three for spilled ones
+// Differs for every launch of every batch: launches 0 and 2 write one list.
+FX_HD unsigned long long spill_mark(unsigned long long generation, int launch) {
+    return generation * kDirectLaunches + static_cast<unsigned long long>(launch);
+}
 struct DirectBatch {
     DirectParams field[kMaxDirectFields];
     long long first[kMaxDirectFields + 1];  // pixel prefix over the batch
@@ -517,7 +521,7 @@ struct DirectBatch {
     int fast_smooth;                        // smooth value in FP32 (floatexp form's direct levels)
     DirectSpill* spill;                     // two lists of spill_capacity entries
     long long spill_capacity;
-    // Bound on a consumer's wait for a spilled entry's generation mark (then
+    // Bound on a consumer's wait for a spilled entry's mark (then
     // kQueueError is set and the entry is dropped), and a fault-injection
     // switch for tests: spilled entries are written but never published.
     int spin_limit;

@@ -623,12 +623,13 @@ __global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const
                 }
                 base = __shfl_sync(kFull, base, 0);
                 if (!active && base + rank < items) {
-                    // Written by an earlier launch; the wait for the entry's
-                    // generation mark is bounded.
+                    // Written by the launch before, whose mark it must carry;
+                    // the wait for it is bounded.
                     const DirectSpill& e = list[base + rank];
                     bool ready = false;
                     for (int spin = 0; spin < b.spin_limit; ++spin) {
-                        if (*reinterpret_cast<const volatile unsigned long long*>(&e.ready) == generation) {
+                        if (*reinterpret_cast<const volatile unsigned long long*>(&e.ready)
+                            == spill_mark(generation, launch - 1)) {
                             ready = true;
                             break;
                         }
@@ -757,7 +758,7 @@ __global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const
         const unsigned spilling = __ballot_sync(kFull, spill);
         if (spilling != 0u) {
             // Hand the lanes to the spill list (one reservation per warp, the
-            // entry's generation mark written last); a full list lets them
+            // entry's mark written last); a full list lets them
             // run on here.
             const int leader = __ffs(spilling) - 1;
             unsigned long long base = 0;
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const
                     e.field = l.field;
                     e.local = l.local;
                     __threadfence();
-                    if (!b.withhold_publish) *reinterpret_cast<volatile unsigned long long*>(&e.ready) = generation;
+                    if (!b.withhold_publish) *reinterpret_cast<volatile unsigned long long*>(&e.ready) = spill_mark(generation, launch);
                     active = false;
                 } else {
                     l.stop_at = Resume ? l.max_iter + 1 : l.max_iter;  // (never offered again)
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(128, Resume ? 4 : 8) direct_queue_kernel(const
 __global__ void direct_coords_kernel(const __grid_constant__ DirectBatch b) {
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < kGeneration) b.counter[i] = 0ull;
-    if (i == kGeneration) b.counter[i] += 1ull;  // a new mark for this batch's spill entries
+    if (i == kGeneration) b.counter[i] += 1ull;  // new marks for this batch's spill entries
     for (int f = 0; f < b.count; ++f) {
         const DirectParams& p = b.field[f];
         const long long span = static_cast<long long>(p.width) + p.height;

@@ -25,13 +25,17 @@ def check(status):
 """
 
 
+def cuda_include() -> str:
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    return os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+
+
 def link(package, directory) -> str:
     """The library's objects with the stand-in runtime; returns the path."""
     built = os.path.dirname(package.build())
     sources = sorted(os.listdir(os.path.join(PACKAGE_DIR, "csrc")))
     objects = [os.path.join(built, name + ".o") for name in sources if name.endswith((".cu", ".cpp"))]
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    include = cuda_include()
     path = os.path.join(str(directory), "libfake.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I" + include,
                     os.path.join(ROOT, "tests", "fake_cuda.cpp"), *objects, "-o", path, "-ldl", "-lpthread"], check=True)

@@ -11,10 +11,13 @@ launch.
 from __future__ import annotations
 
 import ctypes
+import os
+import subprocess
 
 import pytest
 
 from . import fake_cuda
+from .conftest import ROOT
 
 
 def test_resuming_launches(package, tmp_path):
@@ -32,6 +35,29 @@ print(*counts)
 """)
     # The coordinate tables, the fresh pixels, and the resuming launches.
     assert list(map(int, out.split())) == [2, 3, 2, 3, 2, 5, 2, 5]
+
+
+def test_marks_tell_launches_apart(tmp_path):
+    """A list is written by every other launch: an entry that one of them left
+    out must not pass for its own with the mark of the one before."""
+    source, binary = tmp_path / "driver.cpp", tmp_path / "driver"
+    source.write_text("""
+#include "device.h"
+#include <set>
+int main() {
+    std::set<unsigned long long> marks{0ull};  // 0: a cleared entry
+    for (unsigned long long generation = 1; generation <= 1000; ++generation) {
+        for (int launch = 0; launch < fgb::kDirectLaunches; ++launch) {
+            if (!marks.insert(fgb::spill_mark(generation, launch)).second) return 1;
+        }
+    }
+    return 0;
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(fake_cuda.PACKAGE_DIR, "csrc"),
+                    "-I" + os.path.join(ROOT, "include"), "-I" + fake_cuda.cuda_include(), str(source), "-o", str(binary)],
+                   check=True)
+    subprocess.run([str(binary)], check=True)
 
 
 _ARGS = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_char_p, ctypes.c_char_p,
