@@ -591,7 +591,12 @@ __device__ __noinline__ PixelOut floatexp_general(const FxParams& p, int px, int
         }
         const N1e dn = norm2(delta);
         if (n_cmp(total_norm, dn) < 0) {
-            if (++rebases > 64) {
+            // At index 0 the total is the delta: where its quantised norm
+            // compares below the other there, which the high bailout's does,
+            // the same turn repeats to the limit.
+            const bool repeats = ref == 0 && f_bits(total.x) == f_bits(delta.x) && f_bits(total.y) == f_bits(delta.y)
+                && total.e == delta.e;
+            if (++rebases > 64 || repeats) {
                 result = continue_direct<Planes>(p, total, iteration, dc, derivative);
                 break;
             }
