@@ -21,6 +21,7 @@
 
 #include <cstdint>
 
+#include "corrected_quotient.h"
 #include "device.h"
 
 namespace fgb {
@@ -102,14 +103,6 @@ __device__ __forceinline__ float div_const(float x, float d, float r) {
     const float q0 = __fmul_rn(x, r);
     const float e = __fmaf_rn(-q0, d, x);
     return __fmaf_rn(e, r, q0);
-}
-
-// v / 255 for a palette share v in [0, 256): a share below 2^-100, where the
-// corrected product may miss the quotient, moves no byte.
-__device__ __forceinline__ float byte_share(float v) {
-    constexpr float r = 1.0f / 255.0f;
-    const float q0 = __fmul_rn(v, r);
-    return __fmaf_rn(__fmaf_rn(-q0, 255.0f, v), r, q0);
 }
 
 constexpr float kHalfPiF = kPiF / 2.0f;
@@ -606,9 +599,9 @@ __device__ __forceinline__ void kfp_pixel(const float* __restrict__ field, const
             if (inverse_transition) f = 1.0f - f;
             const int upper = lower + 1 < k.lut_size ? lower + 1 : 0;  // (lower + 1) mod size, lower in [0, size)
             const float g = 1.0f - f;
-            o_r = byte_share(static_cast<float>(lut[lower * 3]) * g + static_cast<float>(lut[upper * 3]) * f);
-            o_g = byte_share(static_cast<float>(lut[lower * 3 + 1]) * g + static_cast<float>(lut[upper * 3 + 1]) * f);
-            o_b = byte_share(static_cast<float>(lut[lower * 3 + 2]) * g + static_cast<float>(lut[upper * 3 + 2]) * f);
+            o_r = fx::byte_share(static_cast<float>(lut[lower * 3]) * g + static_cast<float>(lut[upper * 3]) * f);
+            o_g = fx::byte_share(static_cast<float>(lut[lower * 3 + 1]) * g + static_cast<float>(lut[upper * 3 + 1]) * f);
+            o_b = fx::byte_share(static_cast<float>(lut[lower * 3 + 2]) * g + static_cast<float>(lut[upper * 3 + 2]) * f);
         } else {
             o_r = FGB_DIV(static_cast<float>(lut[lower * 3]), 255.0f);
             o_g = FGB_DIV(static_cast<float>(lut[lower * 3 + 1]), 255.0f);

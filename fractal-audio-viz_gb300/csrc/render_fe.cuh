@@ -16,6 +16,7 @@
 
 #include <cstdint>
 
+#include "corrected_quotient.h"
 #include "device.h"
 
 namespace fgb {
@@ -424,14 +425,6 @@ __device__ __noinline__ PixelOut shallow_pixel(const FxParams& p, int px, int py
     return inside;
 }
 
-// offset / dimension given 1 / dimension: Markstein's correction of the rounded
-// product (colour_kfp.cu) is the IEEE quotient for every half-integer offset
-// of a dimension up to 32768 (all of them compared on a host).
-__device__ __forceinline__ float offset_quotient(float offset, float dimension, float per) {
-    const float q = __fmul_rn(offset, per);
-    return __fmaf_rn(__fmaf_rn(-q, dimension, offset), per, q);
-}
-
 // The pixel's offset from the reference as plain floats, scaled as the
 // floatexp pair is: a shared exponent first, then one multiplication by a
 // power of two.
@@ -701,9 +694,9 @@ __device__ __forceinline__ PixelOut floatexp_pixel(const FxParams& p, int px, in
     float x = 0.0f, y = 0.0f;
     F2e derivative = one_f2e();
     if (whole) {
-        const float wx = p.view_width.x * offset_quotient(axis_offset(px, p.width, p.coordinate_mode),
+        const float wx = p.view_width.x * fx::offset_quotient(axis_offset(px, p.width, p.coordinate_mode),
                                                           static_cast<float>(p.width), __ldg(&sc->per_x));
-        const float wy = p.view_height.x * offset_quotient(-axis_offset(py, p.height, p.coordinate_mode),
+        const float wy = p.view_height.x * fx::offset_quotient(-axis_offset(py, p.height, p.coordinate_mode),
                                                            static_cast<float>(p.height), __ldg(&sc->per_y));
         series_horner<Planes>(sc, wx * __ldg(&sc->step_x), wy * __ldg(&sc->step_y), x, y, derivative);
         const float grow = __ldg(&sc->grow);
