@@ -14,8 +14,9 @@
 // top bit, so its lowest 32-bit word is zero: int_mul reports that word, and
 // where it is zero the caller takes int_mul_even, which rounds ties to even.
 // That happens for operands with 20 trailing zero bits between them: one
-// product in 50,000 of full mantissas, but every one that follows a deep
-// cancellation.  Operands and result must be normal.
+// product in 95,000 of independent full mantissas, one square in 1,024 (10
+// bits suffice), and every one that follows a deep cancellation.  Operands and
+// result must be normal.
 #pragma once
 
 #include "scaled.h"

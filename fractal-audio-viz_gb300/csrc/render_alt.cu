@@ -965,15 +965,16 @@ __device__ __forceinline__ unsigned long long alt_deadline(const AltParams& p) {
 // of ready pixels.  Run by the lanes just refilled, the starts and blocks
 // took 80 % of the instructions.
 //
-// Once no pixel is left to take, a warp that has run kAltPatience rounds with
-// fewer than kAltLeave active lanes leaves: it spills them to a list that the next launch takes as
-// its input, so the few long orbits (10 % of a Julia view past 500 steps, 1 %
-// to the cap) run 32 to a warp instead of one in each.  Lifetimes are
-// close to exponential whatever their scale, so a rule on lanes suits every
-// view where a budget of steps suits one; the patience lets pixels that all
-// end soon end where they are (a burning-ship view's, 8.4 ms without it and
-// 5.8 ms with it).  A list short enough to give every
-// SM sub-partition one warp gains nothing from another launch and runs to its end.
+// In a field of several launches (alt_launch), once no pixel is left to take, a
+// warp that has run kAltPatience rounds with fewer than kAltLeave active lanes
+// leaves: it spills them to a list that the next launch takes as its input, so
+// the few long orbits (10 % of a Julia view past 500 steps, 1 % to the cap) run
+// 32 to a warp instead of one in each.  Lifetimes are close to exponential
+// whatever their scale, so a rule on lanes suits every view where a budget of
+// steps suits one; the patience lets pixels that all end soon end where they
+// are (a burning-ship view's, 8.4 ms without it and 5.8 ms with it).  A list
+// short enough to give every SM sub-partition one warp gains nothing from
+// another launch and runs to its end.
 constexpr int kAltRefill = 8;
 constexpr int kAltPhases = 8;
 constexpr int kAltLeave = 20;

@@ -110,7 +110,7 @@ __device__ const Step* find_block(const Step* table, const LevelIndex* index, in
     // `start` is aligned to a level's blocks from its trailing zeros down.
     // The index words of the first level are loaded together: a pixel alone
     // in its warp waits for them once.  The 112-level 1920x1080 ladder took
-    // 16.7 ms with every level tested in turn and 16.3 ms this way.
+    // 17.2 ms with every level tested in turn and 16.3 ms this way.
     const int offset = start - 1;
     const int longest = 31 - __clz(max_length);
     int level = min(min(longest, kMaxLevels - 1), offset ? __ffs(offset) - 1 : kMaxLevels - 1);

@@ -23,8 +23,8 @@
 // operands those rules do not cover (subnormal, infinite, NaN) go to
 // out-of-line general paths.  A complex product with its normalisation then
 // takes 6 FP64 instructions where the comparisons and halvings made it 18.
-// Measured: a 640x360 plain field at 1e30 in 3.10 ms before and 0.98 ms now,
-// an 853x480 burning-ship field with planes at 1e40 in 106 and 39 ms.
+// These rules alone took a 640x360 plain field at 1e30 from 3.10 to 0.98 ms and
+// an 853x480 burning-ship field with planes at 1e40 from 106 to 39 ms.
 #pragma once
 
 #include <cstdint>
