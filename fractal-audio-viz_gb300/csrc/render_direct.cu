@@ -566,7 +566,7 @@ constexpr int kRefill = 8;                // idle lanes before a resuming warp t
 constexpr int kLeave = 20;                // active lanes below which it gives its pixels back ...
 constexpr int kPatience = 16;             // ... after so many rounds,
 constexpr int kShortList = 32 * 4 * 152;  // unless the list gives a warp to each sub-partition at most
-constexpr long long kOneResume = 65536;   // pixels of a batch up to which one launch resumes
+constexpr long long kOneResume = 262144;  // pixels of a batch up to which one launch resumes
 constexpr int kResumeBlocks = 2;          // per SM: two warps for each sub-partition
 
 template <int Formula, bool Planes, bool Resume, bool Integer>
@@ -1050,10 +1050,10 @@ static bool view_meets_interior(const DirectParams& p) {
 
 // Launches of a batch: one for fresh pixels and up to three for spilled ones.
 // None of those finds anything where no cap exceeds the budget, and each costs
-// 2 to 4 us: 256x144 at 1e3, where nothing spills, took 64 us with three, 55
-// with one.  One also does for small batches whose pixels do spill: it keeps
-// every lane and refills from the list, and up to kOneResume pixels that is
-// within two refills of its 38,912 lanes.
+// 3 us and twice that of the calling thread: 257x256 around nothing that
+// spills took 61 us with three, 55 with one.  One also serves the batches of
+// up to kOneResume pixels that do spill better: it keeps its 38,912 lanes full
+// from the list (640x360 at 1e5.7: 4.1 ms, with three 6.5 ms).
 static int direct_launches(const DirectBatch& b, long long pixels) {
     if (b.spill_capacity <= 0) return 1;
     int longest = 0;

@@ -25,8 +25,8 @@ def test_resuming_launches(package, tmp_path):
 options = native.RenderOptions()
 field = (ctypes.c_float * (512 * 512))()
 counts = []
-for width, height, cap in ((64, 36, 256), (64, 36, 257), (256, 256, 256), (256, 256, 257), (257, 256, 256),
-                           (257, 256, 257), (512, 512, 100), (512, 512, 5000)):
+for width, height, cap in ((64, 36, 256), (64, 36, 257), (512, 512, 256), (512, 512, 257), (513, 512, 256),
+                           (513, 512, 257), (900, 800, 100), (900, 800, 5000)):
     before = lib.fake_launches()
     check(lib.fractal_gb300_render_direct_device(field, None, width, height, b"1", b"-0.5", b"0.0", cap, 0, 0.0, 0.0,
                                                  ctypes.byref(options), None))
@@ -64,10 +64,10 @@ _ARGS = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_
          ctypes.c_char_p, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_void_p,
          ctypes.c_void_p]
 SEA = (b"4.5e5", b"-0.743643887037151", b"0.13182590420533", (0.0, 0.0))
-VIEWS = [("mandelbrot", SEA, 256, 256, 3000), ("mandelbrot", SEA, 257, 256, 3000), ("mandelbrot", SEA, 200, 112, 256),
+VIEWS = [("mandelbrot", SEA, 512, 512, 3000), ("mandelbrot", SEA, 513, 512, 3000), ("mandelbrot", SEA, 200, 112, 256),
          ("burning-ship", (b"20", b"-1.76", b"-0.03", (0.0, 0.0)), 257, 255, 4000),
          ("julia", (b"1", b"0.0", b"0.0", (-0.7269, 0.1889)), 1101, 619, 4000),
-         ("tricorn", (b"30", b"-1.4", b"0.01", (0.0, 0.0)), 640, 360, 4000),
+         ("tricorn", (b"30", b"-1.4", b"0.01", (0.0, 0.0)), 801, 401, 4000),
          # 646,000 pixels past the budget, of 524,288 entries.
          ("burning-ship", (b"1", b"-0.5", b"-0.3", (0.0, 0.0)), 3840, 2160, 600)]
 
