@@ -365,6 +365,20 @@ __device__ __forceinline__ int exact_run(const PlainParams& p, const Sc& paramet
     return made;
 }
 
+// How many general steps follow before a run that took none is tried again:
+// none after its first failure, then one, two, up to 32.  A pixel exactly on an
+// axis has a zero part at every step, and entering the run in vain each time
+// lengthened them all: a 200x113 field around -1.62 at 1e12, one row of it on
+// the axis, took 6.0 ms (9.2 with thread-per-pixel FP64 tests) and 4.8 this way.
+struct Rest {
+    int left = 0, next = 0;
+    __device__ bool over() { return left == 0 || left-- == 0; }
+    __device__ void tell(int made) {
+        left = made == 0 ? next : 0;
+        next = made == 0 ? imin(imax(2 * next, 1), 32) : 0;
+    }
+};
+
 // Exact scaled recurrence from the reconstructed total once the pixel has
 // left the compact reference (renderer.cpp:13053-13146 and 13155-13250).
 // kExitNorm with the last total, its norm and the one before for a value that
@@ -384,6 +398,7 @@ __device__ __forceinline__ Exit exact_continuation(const PlainParams& p, const O
     const int cycle_margin = p.strict_cycle ? 78 : 60;
     out_value = encode(static_cast<double>(p.max_iter), p.output_bias);
     out_count = static_cast<std::uint32_t>(p.max_iter);
+    Rest rest;
     while (iteration < p.max_iter) {
         if (deadline_ns && (ticks & 255U) == 0U && global_ns() >= deadline_ns) {
             out_value = nan_f();
@@ -396,16 +411,19 @@ __device__ __forceinline__ Exit exact_continuation(const PlainParams& p, const O
         prior = total_norm;
         int made = 0;
         bool open = false;
-        total = to_raw(total);
-        if (plain && total.e == 0) {
+        if (plain && rest.over()) {
+            total = to_raw(total);
             Sc before = sc_zero();
             const int room = imin(p.max_iter - iteration, deadline_ns ? 256 - static_cast<int>(ticks & 255U) : INT_MAX);
-            made = exact_run<Planes>(p, plain_parameter, iteration, room, cycle_min, total, before, derivative, open);
+            if (total.e == 0) {
+                made = exact_run<Planes>(p, plain_parameter, iteration, room, cycle_min, total, before, derivative, open);
+            }
             if constexpr (Planes) {
                 if (made > 1) prior = sc_norm2(normal_form(before));
             }
+            total = normal_form(total);
+            rest.tell(made);
         }
-        total = normal_form(total);
         if (made == 0) {
             if constexpr (Planes) derivative = sc_add(sc_twice(sc_mul(total, derivative)), sc_one());
             total = sc_add(sc_sqr(total), parameter);
@@ -600,6 +618,7 @@ __device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitVie
     const bool strict = p.strict != 0;
     Exit exit = kExitNone;
     bool ended = false;
+    Rest rest;
     while (iteration < p.max_iter && t.ref >= 0 && t.ref + 1 < p.orbit_size) {
         if (deadline_ns && (ticks & 255U) == 0U && global_ns() >= deadline_ns) {
             out_value = nan_f();
@@ -615,7 +634,11 @@ __device__ __forceinline__ Exit double_tail(const PlainParams& p, const OrbitVie
         if (deadline_ns) room = imin(room, 256 - static_cast<int>(ticks & 255U));
         bool open = false;
         const int moved = t.rebases;
-        const int made = tail_run<Planes, Axis>(p, dc_re, dc_im, room, t, open);
+        int made = 0;
+        if (rest.over()) {
+            made = tail_run<Planes, Axis>(p, dc_re, dc_im, room, t, open);
+            rest.tell(made);
+        }
         st.add(kTailRebases, static_cast<unsigned long long>(t.rebases - moved));
         if (made > 0) {
             ticks += static_cast<unsigned>(made);
