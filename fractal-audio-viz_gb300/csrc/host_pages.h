@@ -5,9 +5,10 @@
 // new arrays took 20 ms against 1.1 ms into mapped ones.  Asking the kernel
 // for the whole range takes 0.3 to 1.3 ms, on the calling thread while the
 // render runs: the same render took 20 ms without it and 1.6 ms with it.  For
-// pages that are there already the request costs 2 us.  Contents do not change;
-// a range that cannot be mapped for writing, or a kernel without the request,
-// leaves the copy as it was.
+// pages that are there already the request costs 3 to 10 us, so the callers
+// leave small results alone.  Contents do not change; a range that cannot be
+// mapped for writing, or a kernel without the request, leaves the copy as it
+// was.
 #pragma once
 
 #include <cstddef>

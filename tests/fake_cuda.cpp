@@ -7,7 +7,8 @@
 //   * fake_hazards: launches made while the clear of a new allocation may
 //     still run (cleared as a whole, on another stream than the launch's that
 //     nobody has waited for since);
-//   * fake_launches, fake_allocated, fake_uploaded: totals.
+//   * fake_launches, fake_allocated, fake_uploaded: totals;
+//   * fake_mapped: bytes of the caller's memory whose pages were asked for.
 #include <cuda_runtime_api.h>
 #include <sys/mman.h>
 
@@ -25,7 +26,7 @@ thread_local Call pushed;
 thread_local int device = 0;
 int devices = 1;
 long long launches = 0, hazards = 0;
-std::size_t allocated = 0, uploaded = 0;
+std::size_t allocated = 0, uploaded = 0, mapped = 0;
 std::map<char*, std::size_t> memory;
 std::multimap<std::size_t, char*> given_back;  // reused for an equal size, as the allocator does
 std::set<cudaStream_t> clearing;               // streams with the clear of an allocation in flight
@@ -50,7 +51,14 @@ long long fake_launches() { return launches; }
 long long fake_hazards() { return hazards; }
 std::size_t fake_allocated() { return allocated; }
 std::size_t fake_uploaded() { return uploaded; }
+std::size_t fake_mapped() { return mapped; }
 void* fake_stream() { return handle(); }
+
+// The library's requests for pages come here; they change nothing.
+int madvise(void*, std::size_t bytes, int) noexcept {
+    mapped += bytes;
+    return 0;
+}
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = devices; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* n) { *n = device; return cudaSuccess; }

@@ -18,7 +18,7 @@ package = load_package()
 native = package.native
 lib = native.load({path!r}, gb300=True)
 lib.fake_stream.restype = ctypes.c_void_p
-for name in ("fake_launches", "fake_hazards", "fake_allocated", "fake_uploaded"):
+for name in ("fake_launches", "fake_hazards", "fake_allocated", "fake_uploaded", "fake_mapped"):
     getattr(lib, name).restype = ctypes.c_longlong
 def check(status):
     assert status == 0, native.last_error(lib)
